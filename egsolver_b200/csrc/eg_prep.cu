@@ -436,12 +436,13 @@ void launch_task_reset(int bits, int heavy_begin, int n_pad, const int *toff, Cl
     else k_task_reset<int64_t><<<(unsigned)g, 256, 0, st>>>(heavy_begin, n_pad, toff, ct, (int64_t *)hacc, hrem);
 }
 
-/* Credits back in original vertex order (and width). */
+/* Credits back in original vertex order (iperm; null: already there) and in
+ * the width asked for. */
 template <class T, class O>
 __global__ void k_gather_out(int n, const int *iperm, const T *F, O *out)
 {
     for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
-        const T x = F[iperm[v]];
+        const T x = F[iperm ? iperm[v] : (int)v];
         out[v] = (x == credit_traits<T>::top) ? credit_traits<O>::top : (O)x;
     }
 }
@@ -457,6 +458,14 @@ __global__ void k_count_top(int n_pad, const T *F, unsigned long long *out)
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
 }
 
+/* Credits in original vertex order back into the renumbered array. */
+template <class T>
+__global__ void k_resume_credits(int n, const int *iperm, const T *credits, T *F)
+{
+    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x)
+        F[iperm[v]] = credits[v];
+}
+
 static unsigned grid_cap(long long items, int block)
 {
     long long g = (items + block - 1) / block;
@@ -467,6 +476,12 @@ void launch_init_credits(int bits, int n_alloc, void *F, int topv, cudaStream_t 
 {
     if (bits == 32) k_init_credits<int32_t><<<grid_cap(n_alloc, 256), 256, 0, st>>>(n_alloc, (int32_t *)F, topv);
     else k_init_credits<int64_t><<<grid_cap(n_alloc, 256), 256, 0, st>>>(n_alloc, (int64_t *)F, topv);
+}
+
+void launch_resume_credits(int bits, int n, const int *iperm, const void *credits, void *F, cudaStream_t st)
+{
+    if (bits == 32) k_resume_credits<int32_t><<<grid_cap(n, 256), 256, 0, st>>>(n, iperm, (const int32_t *)credits, (int32_t *)F);
+    else k_resume_credits<int64_t><<<grid_cap(n, 256), 256, 0, st>>>(n, iperm, (const int64_t *)credits, (int64_t *)F);
 }
 
 void launch_count_top(int bits, int n_pad, const void *F, unsigned long long *out, cudaStream_t st)

@@ -1,0 +1,112 @@
+"""GPU tests of the sweep solver (eg_sweep.cu): exact credits where its
+layout changes -- one CTA or the grid, values in shared or global memory,
+edges staged or not, cut vertices -- and the hand-over to frontier rounds."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import egsolver_b200 as eg
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def hub_game(degrees, n=900, seed=5, wmax=40):
+    """Vertices of out-degree 1..3 and one of each given out-degree, owners alternating."""
+    rng = np.random.default_rng(seed)
+    deg = rng.integers(1, 4, n)
+    deg[rng.choice(n, len(degrees), replace=False)] = degrees
+    rp = np.concatenate([[0], np.cumsum(deg)])
+    m = int(rp[-1])
+    return eg.Game(row_ptr=rp, succ=rng.integers(0, n, m), weight=rng.integers(-wmax, wmax + 1, m),
+                   owner=rng.integers(0, 2, n).astype(np.uint8))
+
+
+def want(game):
+    """The oracle's credits (it takes owner-sorted games)."""
+    own = game.owners()
+    order = np.argsort(own, kind="stable")
+    inv = np.empty_like(order)
+    inv[order] = np.arange(order.size)
+    deg = np.diff(game.row_ptr)[order]
+    idx = np.concatenate([np.arange(game.row_ptr[v], game.row_ptr[v + 1]) for v in order])
+    g = eg.Game(row_ptr=np.concatenate([[0], np.cumsum(deg)]), succ=inv[game.succ[idx]], weight=game.weight[idx],
+                num_nodes0=int((own == 0).sum()))
+    f, st = O.eg_solve(g, bits=64, max_loop_=1 << 60)
+    assert st["finished"]
+    return f[inv]
+
+
+# 3,590 vertices of out-degree 4 fill the shared memory of one CTA
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 1025, 3500, 3700])
+def test_one_cta_and_grid_sizes(n):
+    g = eg.generate(1, n, min(4, n), 9, 77 + n) if n > 4 else eg.Game(
+        row_ptr=np.arange(n + 1), succ=np.arange(n)[::-1].copy(), weight=np.arange(n) - 1, num_nodes0=n // 2)
+    f, st = eg.solve(g)
+    np.testing.assert_array_equal(f, want(g))
+    assert st.num_top == int((f == eg.EG_TOP64).sum())
+    assert (st.grid == 1) == (n <= 3500)
+
+
+@pytest.mark.parametrize("n,degrees", [(900, [255, 256, 257]), (900, [511, 513, 800]), (6000, [256, 4097, 5000]),
+                                       (6000, [33] * 700)])
+def test_cut_vertices(n, degrees):
+    g = hub_game(degrees, n)
+    ref = want(g)
+    f, _ = eg.solve(g)
+    np.testing.assert_array_equal(f, ref)
+    f32, st = eg.solve(g, narrow=True)
+    assert st.credit_bits == 32
+    np.testing.assert_array_equal(f32, ref)
+
+
+@pytest.fixture(scope="module")
+def power_20k():
+    g = eg.generate(2, 20000, 4096, 50, 11)
+    return g, want(g)
+
+
+# few CTAs: their values (28 B per vertex), then only their edges, leave shared memory
+@pytest.mark.parametrize("ctas", [1, 3, 5, 147])
+def test_values_and_edges_outside_shared_memory(power_20k, ctas):
+    g, ref = power_20k
+    f, st = eg.solve(g, grid_ctas=ctas)
+    assert st.grid == ctas
+    np.testing.assert_array_equal(f, ref)
+
+
+@pytest.mark.parametrize("lanes_degree", [1, 2, 16, 40])
+def test_lanes_per_vertex(lanes_degree):
+    g = eg.generate(1, 6000, lanes_degree, 30, 3)
+    f, _ = eg.solve(g)
+    np.testing.assert_array_equal(f, want(g))
+
+
+def test_round_cap_on_the_grid_gives_a_lower_bound():
+    g = eg.generate(4, 9000, 16, 100, 21, param=2)
+    ref = want(g)
+    with eg.ResidentGame(g) as r:
+        status, st = r.solve(raise_on_error=False, max_rounds=1)
+        assert eg._ffi.STATUS_NAMES[status] == "EG_ERR_LOOPCAP" and st.rounds == 1
+        part = r.credits()
+        assert np.all(part <= ref) and np.any(part < ref)
+        r.solve()
+        np.testing.assert_array_equal(r.credits(), ref)
+
+
+def test_hand_over_to_frontier_rounds():
+    """Chains of 4,096 vertices along which one credit moves back a vertex
+    per sweep: few raises in each of thousands of sweeps."""
+    length, chains = 4096, 1100
+    n = length * chains
+    succ = np.arange(1, n + 1, dtype=np.int32)
+    succ[length - 1::length] = np.arange(length - 1, n, length)
+    weight = np.zeros(n, np.int32)
+    weight[length - 2::length] = -5
+    g = eg.Game(row_ptr=np.arange(n + 1), succ=succ, weight=weight, num_nodes0=n // 2)
+    f, st = eg.solve(g)
+    ref = np.full(n, 5)
+    ref[length - 1::length] = 0
+    np.testing.assert_array_equal(f, ref)
+    assert st.rounds > 512 and st.num_top == 0
