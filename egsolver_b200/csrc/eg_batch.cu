@@ -67,12 +67,14 @@ template <typename CT> struct Lim;
 template <> struct Lim<int> {
     static constexpr int top = 1 << 30;
     static constexpr int low = -(1 << 30);
+    static constexpr int dual_max = 1 << 29; /* potentials above count as out */
     static constexpr int lo_acc = INT32_MIN;
     static constexpr int hi_acc = INT32_MAX;
 };
 template <> struct Lim<long long> {
     static constexpr long long top = 1LL << 62;
     static constexpr long long low = -(1LL << 62);
+    static constexpr long long dual_max = 1LL << 61;
     static constexpr long long lo_acc = INT64_MIN;
     static constexpr long long hi_acc = INT64_MAX;
 };
@@ -110,7 +112,18 @@ struct Shared {
     unsigned raise[3];    /* per-sweep OR of raised thresholds (rotating)     */
     int unit;
     long long p[8], mg[8];
+    long long dual[8];    /* 1 - 2^nshift p: what a dual sweep adds per vertex */
 };
+
+/* What a unit's sweep computes: lifts of the credits; lifts of a potential;
+ * or the removal of vertices whose potential is not one.  See run_unit. */
+enum { UNIT_PRIMAL, UNIT_DUAL, UNIT_KILL };
+constexpr int kUnitFirstPrimal = 4, kUnitSecondPrimal = 16, kUnitFirstDual = 8, kUnitMaxDual = 128;
+constexpr long long kUnitMaxPrimal = 1 << 20;
+/* Units below this many sweeps do not park: all but 1 in 500 of the
+ * thresholds of random games at uniform thresholds end within it, and the
+ * tail runs no certificates. */
+constexpr long long kParkSweeps = 512;
 
 template <int KG> struct Log2 {
     static constexpr int v = KG == 1 ? 0 : KG == 2 ? 1 : KG == 4 ? 2 : 3;
@@ -171,9 +184,47 @@ __device__ __forceinline__ void column_walk(const void *E, int i0, int W, const 
     }
 }
 
+/* log2 of the factor by which a unit's potentials count the weights w d - p:
+ * the largest (at most 2^20) that leaves room for 512 (32-bit credits: 2^29 /
+ * 2^20) or more times the largest weight below Lim::dual_max; -1 where even 1
+ * does not, and the unit runs without certificates.  From the device's
+ * thresholds, so that a captured launch serves any. */
+template <int KG, typename CT>
+__device__ __forceinline__ int potential_shift(const UnitDesc &u)
+{
+    long long big = 0;
+    for (int k = 0; k < KG; k++) big = max(big, (long long)abs((long long)u.p[u.k0 + k]));
+    big += (long long)u.wpad * u.d;
+    const long long limit = sizeof(CT) == 8 ? 1LL << 50 : 1LL << 20;
+    int s = -1;
+    while (s < 20 && (big << (s + 1)) <= limit) s++;
+    return s;
+}
+
 /* Solves one unit (KG thresholds, credit type CT, slot width WIDE, credits
  * in shared memory or, with GF (a hybrid unit, KG = 1), rows from u.srows on
- * in the unit's global scratch). */
+ * in the unit's global scratch).
+ *
+ * The sweeps that raise credits are cut short by certificates, as in
+ * eg_sweep.cu: after a few primal sweeps the buffer that held the open
+ * thresholds' credits takes potentials of the game with the players
+ * exchanged and weights -(2^nshift (w d - p) + 1) (dual sweeps, from 0),
+ * then kill sweeps put every vertex out (TOP) whose potential is not one,
+ * until none goes.  The vertices left are TOP of the game itself; the others
+ * start again from credit 0, for four times as many sweeps, and so on.
+ * Nothing of the credits but the TOPs is kept over an attempt: a second
+ * buffer would halve the thresholds of a group, and the sweeps run again
+ * are at most a third of the last phase.  A vertex at TOP before an attempt
+ * holds LOW in it.  The column walk is the same for all: a dual sweep takes
+ * the max where a primal one takes the min, with -2^nshift d for d, and the
+ * two sentinel rows hold each other's values, so that a pad decides
+ * nothing.
+ *
+ * A sweep is bound by shared-memory gathers and issue; the certificates cut
+ * the number of sweeps.  Measured, device time of a solve: 32 games of 1,024
+ * to 16,384 vertices at 8 thresholds 350 ms -> 1.0 ms (40 sweeps at most);
+ * 64 games of 1,024 to 65,536 vertices at 8 thresholds 34 to 59 s -> 93 ms
+ * (310 sweeps at most). */
 template <int KG, typename CT, bool WIDE, bool GF>
 __device__ __forceinline__ void run_unit(const UnitDesc &u, int uglobal, unsigned char *smem, Shared &sh,
                                          const UnitParams &P, unsigned long long t0, unsigned long long &lifts,
@@ -200,22 +251,28 @@ __device__ __forceinline__ void run_unit(const UnitDesc &u, int uglobal, unsigne
         sh.p[tid] = u.p[u.k0 + tid];
         sh.mg[tid] = u.mg[u.k0 + tid];
     }
+    const int nshift = potential_shift<KG, CT>(u);
+    if (tid < KG) sh.dual[tid] = 1 - ((long long)u.p[u.k0 + tid] << max(nshift, 0));
     if (tid == 0) sh.raise[0] = sh.raise[1] = sh.raise[2] = 0;
     __syncthreads();
     const CT d = (CT)u.d;
     const unsigned full = (1u << KG) - 1u;
     unsigned amask = full;
-    long long r = 0;
+    long long r = 0; /* primal sweeps */
     int st = EG_OK;
-    for (;;) {
+    int mode = UNIT_PRIMAL, dual_len = kUnitFirstDual;
+    long long left = nshift < 0 ? INT64_MAX : kUnitFirstPrimal, primal_len = kUnitSecondPrimal;
+    for (int it = 0;; it = it == 2 ? 0 : it + 1) {
         unsigned raised = 0;
+        const bool dual = mode != UNIT_PRIMAL;
+        const CT mul = dual ? (CT)-(CT)(d << max(nshift, 0)) : d;
         for (int s = warp; s < ns; s += nwarps) {
             const int b = __ldg(u.slice_off + s);
             const int W = (__ldg(u.slice_off + s + 1) - b) >> 5;
             const bool own1 = s >= s0;
             CT acc[KG];
-            if (own1) column_walk<KG, CT, WIDE, true, UNR, GF>(u.E, b + lane, W, F, d, acc);
-            else column_walk<KG, CT, WIDE, false, UNR, GF>(u.E, b + lane, W, F, d, acc);
+            if (own1 != dual) column_walk<KG, CT, WIDE, true, UNR, GF>(u.E, b + lane, W, F, mul, acc);
+            else column_walk<KG, CT, WIDE, false, UNR, GF>(u.E, b + lane, W, F, mul, acc);
             const int v = 32 * s + lane;
             const bool real = own1 ? (v - 32 * s0 < u.n1) : (v < u.n0);
             if (real) {
@@ -225,10 +282,11 @@ __device__ __forceinline__ void run_unit(const UnitDesc &u, int uglobal, unsigne
                 for (int k = 0; k < KG; k++) {
                     if (amask >> k & 1u) {
                         /* threshold and MG from shared memory: used once per vertex */
-                        const CT val = acc[k] + (CT)sh.p[k];
-                        const CT nv = val > (CT)sh.mg[k] ? TOPI : (val > 0 ? val : (CT)0);
-                        if (nv > old.v[k]) {
-                            mine[k] = nv;
+                        const CT val = acc[k] + (CT)(dual ? sh.dual[k] : sh.p[k]);
+                        const CT cap = dual ? Lim<CT>::dual_max : (CT)sh.mg[k];
+                        const CT nv = val > cap ? TOPI : (val > 0 ? val : (CT)0);
+                        if (nv > old.v[k] && !(dual && old.v[k] == LOWI)) {
+                            mine[k] = mode == UNIT_KILL ? TOPI : nv;
                             raised |= 1u << k;
                         }
                     }
@@ -236,21 +294,40 @@ __device__ __forceinline__ void run_unit(const UnitDesc &u, int uglobal, unsigne
             }
         }
         raised = __reduce_or_sync(0xffffffffu, raised);
-        const int slot = (int)(r % 3);
-        if (lane == 0 && raised) atomicOr(&sh.raise[slot], raised);
-        if (tid == 0) {
-            if (P.timeout_ns && globaltimer_ns() - t0 > P.timeout_ns) atomicOr(&sh.raise[slot], 1u << 16);
-            /* park: this variant's queue is empty and half of all phase-1
+        if (lane == 0 && raised) atomicOr(&sh.raise[it], raised);
+        if (tid == 0 && !dual) {
+            if (P.timeout_ns && globaltimer_ns() - t0 > P.timeout_ns) atomicOr(&sh.raise[it], 1u << 16);
+            /* park: this variant's queue is empty and a share of all phase-1
              * CTAs have nothing left, so the GPU is running the tail; the
              * unit's open thresholds continue on clusters */
-            if (P.tails && (r & 15) == 15 && ld_volatile(&P.ctrl->next) >= P.num_units &&
+            if (P.tails && (r & 15) == 15 && r >= kParkSweeps && ld_volatile(&P.ctrl->next) >= P.num_units &&
                 100 * ld_volatile(P.idle) >= P.park_percent * P.park_total)
-                atomicOr(&sh.raise[slot], 1u << 17);
+                atomicOr(&sh.raise[it], 1u << 17);
         }
         __syncthreads();
-        const unsigned word = sh.raise[slot];
+        const unsigned word = sh.raise[it];
+        if (tid == 0) sh.raise[it == 0 ? 2 : it - 1] = 0;
+        if (mode == UNIT_DUAL) {
+            if (--left == 0 || !(word & full)) mode = UNIT_KILL;
+            continue;
+        }
+        if (mode == UNIT_KILL) {
+            if (word & full) continue;
+            /* what is left is certified: TOP; the others start again from 0 */
+            for (int i = tid; i < rows * KG; i += blockDim.x) {
+                const int row = i >> LK, k = i & (KG - 1);
+                if (amask >> k & 1u) {
+                    CT *x = F.at(row) + k;
+                    *x = row >= npad ? (row == npad ? TOPI : LOWI) : (*x == TOPI ? (CT)0 : TOPI);
+                }
+            }
+            mode = UNIT_PRIMAL;
+            left = primal_len;
+            primal_len = min(4 * primal_len, kUnitMaxPrimal);
+            __syncthreads();
+            continue;
+        }
         if (tid == 0) {
-            sh.raise[(r + 2) % 3] = 0;
             lifts += (unsigned long long)(u.n0 + u.n1) * (unsigned)__popc(amask);
             edges += (unsigned long long)u.m * (unsigned)__popc(amask);
         }
@@ -268,6 +345,20 @@ __device__ __forceinline__ void run_unit(const UnitDesc &u, int uglobal, unsigne
         if (P.max_rounds >= 0 && r >= P.max_rounds) {
             st = EG_ERR_LOOPCAP;
             break;
+        }
+        if (--left == 0) {
+            /* the buffer turns into potentials, the sentinel rows change places */
+            for (int i = tid; i < rows * KG; i += blockDim.x) {
+                const int row = i >> LK, k = i & (KG - 1);
+                if (amask >> k & 1u) {
+                    CT *x = F.at(row) + k;
+                    *x = row >= npad ? (row == npad ? LOWI : TOPI) : (*x == TOPI ? LOWI : (CT)0);
+                }
+            }
+            mode = UNIT_DUAL;
+            left = dual_len;
+            dual_len = min(4 * dual_len, kUnitMaxDual);
+            __syncthreads();
         }
     }
     __syncthreads();
@@ -297,6 +388,7 @@ __device__ __forceinline__ void run_unit(const UnitDesc &u, int uglobal, unsigne
             e.resume = 1;
             e.pad = 0;
             tl->e[at] = e;
+            atomicAdd(P.parked, 1);
         } else {
             atomicExch(&sh.unit, 1); /* cannot happen: lists hold every threshold */
         }
@@ -934,6 +1026,7 @@ eg_status make_units(const HostPacked &h, const PackedDev &pd, int K, int d, con
         u.ns = h.ns;
         u.s0 = h.s0;
         u.d = d;
+        u.wpad = h.wpad;
         u.k0 = 0;
         u.pad = K; /* thresholds to list */
         u.variant = kUnitTail | (c64 ? kUnitCredit64 : 0) | (h.wide ? kUnitWide : 0);
@@ -958,6 +1051,7 @@ eg_status make_units(const HostPacked &h, const PackedDev &pd, int K, int d, con
         u.ns = h.ns;
         u.s0 = h.s0;
         u.d = d;
+        u.wpad = h.wpad;
         u.k0 = gr.first;
         const int kg = 1 << gr.second;
         const size_t need = (size_t)h.rows() * kg * (c64 ? 8 : 4);
@@ -1197,21 +1291,22 @@ static int tail_clusters(int cls, int csize, int block, int smem)
     return n;
 }
 
-eg_status launch_unit_set(UnitLauncher &L, cudaStream_t main, const UnitSet &S, const UnitDesc *units_dev,
-                          TailList *tails, void *tail_scratch, LaunchCtrl *ctrl, int block, int num_sms,
-                          long long max_rounds, unsigned long long timeout_ns, int *grid_total, int park_percent,
-                          int tail_sweeps, int tail_cluster)
+eg_status launch_units(UnitLauncher &L, cudaStream_t main, const UnitSet &S, const UnitDesc *units_dev, TailList *tails,
+                       LaunchCtrl *ctrl, int block, int num_sms, long long max_rounds, unsigned long long timeout_ns,
+                       int *grid_total, int park_percent)
 {
     cudaError_t e = cudaMemsetAsync(ctrl, 0, sizeof(LaunchCtrl), main);
     if (e != cudaSuccess) return eg_set_error(EG_ERR_CUDA, "launch set-up failed: %s", cudaGetErrorString(e));
     k_tail_rewind<<<1, 256, 0, main>>>(tails, units_dev);
-    e = cudaEventRecord(L.fork, main);
-    if (e != cudaSuccess) return eg_set_error(EG_ERR_CUDA, "launch set-up failed: %s", cudaGetErrorString(e));
-    /* phase 1: the variant holding the heaviest unit is launched first */
+    /* the variant holding the heaviest unit is launched first */
     std::vector<int> vs;
     for (int v = 0; v < kNumVariants; v++)
         if (S.off[v + 1] > S.off[v]) vs.push_back(v);
     std::stable_sort(vs.begin(), vs.end(), [&](int a, int c) { return S.top_cost[a] > S.top_cost[c]; });
+    /* one variant runs on `main` itself; several side by side on forked streams */
+    const bool fork = vs.size() > 1;
+    if (fork) e = cudaEventRecord(L.fork, main);
+    if (e != cudaSuccess) return eg_set_error(EG_ERR_CUDA, "launch set-up failed: %s", cudaGetErrorString(e));
     std::vector<int> grids(vs.size());
     int total = 0;
     for (size_t i = 0; i < vs.size(); i++) {
@@ -1233,6 +1328,7 @@ eg_status launch_unit_set(UnitLauncher &L, cudaStream_t main, const UnitSet &S, 
         p.ctrl = &ctrl->c[v];
         p.tails = tails;
         p.idle = &ctrl->idle;
+        p.parked = &ctrl->parked;
         p.num_units = S.off[v + 1] - S.off[v];
         p.unit_base = S.off[v];
         p.park_total = total;
@@ -1242,18 +1338,33 @@ eg_status launch_unit_set(UnitLauncher &L, cudaStream_t main, const UnitSet &S, 
         p.max_rounds = max_rounds;
         p.timeout_ns = timeout_ns;
         void *args[] = {(void *)&p};
-        e = cudaStreamWaitEvent(L.aux[v], L.fork, 0);
+        cudaStream_t st = fork ? L.aux[v] : main;
+        if (fork) e = cudaStreamWaitEvent(st, L.fork, 0);
         if (e == cudaSuccess)
-            e = cudaLaunchKernel((const void *)kernel_of(v), dim3(grids[i]), dim3(block), args, (size_t)S.smem[v], L.aux[v]);
-        if (e == cudaSuccess) e = cudaEventRecord(L.join[v], L.aux[v]);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(main, L.join[v], 0);
+            e = cudaLaunchKernel((const void *)kernel_of(v), dim3(grids[i]), dim3(block), args, (size_t)S.smem[v], st);
+        if (fork && e == cudaSuccess) e = cudaEventRecord(L.join[v], st);
+        if (fork && e == cudaSuccess) e = cudaStreamWaitEvent(main, L.join[v], 0);
         if (e != cudaSuccess) return eg_set_error(EG_ERR_CUDA, "unit kernel launch failed: %s", cudaGetErrorString(e));
     }
-    /* phase 2: the tail lists on clusters, heaviest entries first, one
-     * kernel per class that can hold entries (those with no entries at run
-     * time exit at once) */
+    if (grid_total) *grid_total = total;
+    return EG_OK;
+}
+
+int tail_entries(const UnitSet &S, const LaunchCtrl &after)
+{
+    size_t n = (size_t)after.parked;
+    for (int c = 0; c < kTailClasses; c++) n += S.tail_init[c].size();
+    return (int)n;
+}
+
+eg_status launch_tail(UnitLauncher &L, cudaStream_t main, const UnitSet &S, const UnitDesc *units_dev, TailList *tails,
+                      void *tail_scratch, LaunchCtrl *ctrl, int num_sms, long long max_rounds,
+                      unsigned long long timeout_ns, int tail_sweeps, int tail_cluster)
+{
+    /* heaviest entries first, one kernel per class that can hold entries
+     * (those with no entries at run time exit at once) */
     k_tail_order<<<kTailClasses, 1024, 0, main>>>(tails, units_dev);
-    e = cudaEventRecord(L.fork2, main);
+    cudaError_t e = cudaEventRecord(L.fork2, main);
     if (e != cudaSuccess) return eg_set_error(EG_ERR_CUDA, "launch set-up failed: %s", cudaGetErrorString(e));
     char *gs = (char *)tail_scratch;
     int dev = 0;
@@ -1330,7 +1441,6 @@ eg_status launch_unit_set(UnitLauncher &L, cudaStream_t main, const UnitSet &S, 
         if (e == cudaSuccess) e = cudaStreamWaitEvent(main, L.join[slot], 0);
         if (e != cudaSuccess) return eg_set_error(EG_ERR_CUDA, "tail kernel launch failed: %s", cudaGetErrorString(e));
     }
-    if (grid_total) *grid_total = total;
     return EG_OK;
 }
 
@@ -1694,8 +1804,8 @@ extern "C" eg_status eg_batch_set_thresholds(eg_batch *b, const int32_t *p)
 static eg_status batch_enqueue(eg_batch *b, cudaStream_t st, int *grid)
 {
     const unsigned long long tns = b->timeout_ms > 0 ? (unsigned long long)(b->timeout_ms * 1e6) : 0ull;
-    return launch_unit_set(b->launcher, st, b->set, b->units_dev, (TailList *)b->tails, b->tscratch, b->ctrl, b->block,
-                           b->sms, b->max_rounds, tns, grid, b->park_percent, b->tail_sweeps, b->tail_cluster);
+    return launch_units(b->launcher, st, b->set, b->units_dev, (TailList *)b->tails, b->ctrl, b->block, b->sms,
+                        b->max_rounds, tns, grid, b->park_percent);
 }
 
 extern "C" eg_status eg_batch_solve(eg_batch *b, eg_batch_stats *stats)
@@ -1739,10 +1849,23 @@ extern "C" eg_status eg_batch_solve(eg_batch *b, eg_batch_stats *stats)
     const size_t nu = b->set.units.size();
     b->last_rounds.assign(nu, 0);
     b->last_status.assign(nu, 0);
-    EG_CUDA(cudaMemcpyAsync(&cv, b->ctrl, sizeof cv, cudaMemcpyDeviceToHost, b->st));
-    EG_CUDA(cudaMemcpyAsync(b->last_rounds.data(), b->u_rounds, sizeof(long long) * nu, cudaMemcpyDeviceToHost, b->st));
-    EG_CUDA(cudaMemcpyAsync(b->last_status.data(), b->u_status, sizeof(int) * nu, cudaMemcpyDeviceToHost, b->st));
-    EG_CUDA(cudaStreamSynchronize(b->st));
+    /* the tail's kernels are launched only when a unit has gone there: with
+     * certificates nearly every unit ends in phase 1 */
+    int in_tail = 0;
+    for (int phase = 0; phase < 2; phase++) {
+        if (phase == 1) {
+            in_tail = tail_entries(b->set, cv);
+            if (in_tail == 0) break;
+            const unsigned long long tns = b->timeout_ms > 0 ? (unsigned long long)(b->timeout_ms * 1e6) : 0ull;
+            EG_TRY(launch_tail(b->launcher, b->st, b->set, b->units_dev, (TailList *)b->tails, b->tscratch, b->ctrl,
+                               b->sms, b->max_rounds, tns, b->tail_sweeps, b->tail_cluster));
+            EG_CUDA(cudaEventRecord(b->ev1, b->st));
+        }
+        EG_CUDA(cudaMemcpyAsync(&cv, b->ctrl, sizeof cv, cudaMemcpyDeviceToHost, b->st));
+        EG_CUDA(cudaMemcpyAsync(b->last_rounds.data(), b->u_rounds, sizeof(long long) * nu, cudaMemcpyDeviceToHost, b->st));
+        EG_CUDA(cudaMemcpyAsync(b->last_status.data(), b->u_status, sizeof(int) * nu, cudaMemcpyDeviceToHost, b->st));
+        EG_CUDA(cudaStreamSynchronize(b->st));
+    }
     UnitCtrl c;
     sum_ctrl(cv, &c);
     /* the two phases on the device clock */
@@ -1754,10 +1877,6 @@ extern "C" eg_status eg_batch_solve(eg_batch *b, eg_batch_stats *stats)
         if (!b0 || x.t_begin < b0) b0 = x.t_begin;
         e0 = std::max(e0, x.t_end);
     }
-    TailList tls[kTailClasses];
-    EG_CUDA(cudaMemcpy(tls, b->tails, sizeof tls, cudaMemcpyDeviceToHost));
-    int tail_entries = 0;
-    for (int t = 0; t < kTailClasses; t++) tail_entries += std::min(tls[t].count, tls[t].cap);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, b->ev0, b->ev1);
     b->solved = true;
@@ -1795,7 +1914,7 @@ extern "C" eg_status eg_batch_solve(eg_batch *b, eg_batch_stats *stats)
         stats->graph_replayed = replay ? 1 : 0;
         stats->num_units = (int32_t)nu;
         stats->smem_bytes = smem;
-        stats->tail_entries = tail_entries;
+        stats->tail_entries = in_tail;
         stats->phase1_ms = p1e > p1b ? (double)(p1e - p1b) * 1e-6 : 0.0;
         stats->tail_ms = te > tb ? (double)(te - tb) * 1e-6 : 0.0;
     }

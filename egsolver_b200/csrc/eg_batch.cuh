@@ -93,7 +93,7 @@ struct UnitDesc {
     int d, k0, variant;
     int pad;                   /* tail units: thresholds the host lists        */
     int srows;                 /* kUnitGlobal: rows held in shared memory       */
-    int pad2;
+    int wpad;                  /* largest |w| + 1                             */
 };
 
 struct UnitCtrl {
@@ -137,6 +137,7 @@ struct UnitParams {
     UnitCtrl *ctrl;
     TailList *tails;           /* kTailClasses lists (parking), or NULL       */
     int *idle;                 /* CTAs of phase 1 that found their queue empty */
+    int *parked;               /* thresholds listed for the tail               */
     int num_units;
     int unit_base;             /* index of units[0] in the whole unit array    */
     int park_total;            /* CTAs of all phase-1 kernels of the launch    */
@@ -237,17 +238,22 @@ struct LaunchCtrl {
     UnitCtrl c[kNumCtrl];
     unsigned long long t_start; /* device clock of the launch's first CTA */
     int idle;
-    int pad[3];
+    int parked;                 /* thresholds that phase 1 listed for the tail */
+    int pad[2];
 };
-/* Launches one persistent kernel per variant present in S (the variant
- * holding the heaviest unit first), each taking its units from its own
- * queue, then one cluster kernel per tail class for the tail lists.  ctrl
- * is reset and the tail lists rewound on `main` first. */
-eg_status launch_unit_set(UnitLauncher &L, cudaStream_t main, const UnitSet &S, const UnitDesc *units_dev,
-                          TailList *tails, void *tail_scratch, LaunchCtrl *ctrl, int block, int num_sms,
-                          long long max_rounds, unsigned long long timeout_ns, int *grid_total,
-                          int park_percent = 10, int tail_sweeps = kTailSweeps,
-                          int tail_cluster = kTailCluster);
+/* Phase 1: launches one persistent kernel per variant present in S (the
+ * variant holding the heaviest unit first), each taking its units from its
+ * own queue.  ctrl is reset and the tail lists rewound on `main` first. */
+eg_status launch_units(UnitLauncher &L, cudaStream_t main, const UnitSet &S, const UnitDesc *units_dev, TailList *tails,
+                       LaunchCtrl *ctrl, int block, int num_sms, long long max_rounds, unsigned long long timeout_ns,
+                       int *grid_total, int park_percent = 10);
+/* Tail entries after phase 1 (host-listed and parked), from a host copy of
+ * ctrl.  When there are any, launch_tail runs one cluster kernel per tail
+ * class on the lists; `tails` and `ctrl` are as phase 1 left them. */
+int tail_entries(const UnitSet &S, const LaunchCtrl &after);
+eg_status launch_tail(UnitLauncher &L, cudaStream_t main, const UnitSet &S, const UnitDesc *units_dev, TailList *tails,
+                      void *tail_scratch, LaunchCtrl *ctrl, int num_sms, long long max_rounds,
+                      unsigned long long timeout_ns, int tail_sweeps = kTailSweeps, int tail_cluster = kTailCluster);
 /* Totals of the per-variant and per-tail-class counters. */
 void sum_ctrl(const LaunchCtrl &c, UnitCtrl *out);
 

@@ -13,10 +13,11 @@
  *      its game is not resident yet, the game's packed layout; idle resident
  *      games are evicted oldest-first when memory is short.  A game stays
  *      resident across all its queries until it is evicted or removed;
- *   3. launch: every admitted query not yet launched goes into one
- *      micro-batch, i.e. one launch of the unit kernel (eg_batch.cu: one CTA
- *      per game x threshold group, credits in shared memory), on the next of
- *      `streams` streams.  Earlier micro-batches keep running; as their CTAs
+ *   3. launch: the admitted queries not yet launched go into one or two
+ *      micro-batches, i.e. launches of the unit kernels (eg_batch.cu: one CTA
+ *      per game x threshold group, credits in shared memory), each on the next
+ *      of `streams` streams.  A micro-batch some of whose units went to the
+ *      cluster tail gets its tail launched when its units have ended.  Earlier micro-batches keep running; as their CTAs
  *      run out of units and exit, the new launch's CTAs take the freed SMs,
  *      so the work of queries that arrived at different times overlaps on
  *      the device.  Each launch records its first CTA start and last CTA end
@@ -118,7 +119,10 @@ struct Launch {
     UnitDesc *dunits = nullptr;
     LaunchCtrl *dctrl = nullptr;
     void *dtails = nullptr;
-    void *dscratch = nullptr;   /* hybrid tail regions */
+    TailList *tl = nullptr;
+    void *dscratch = nullptr;   /* hybrid tail regions                        */
+    UnitSet set;                /* for the tail's launch                      */
+    bool in_tail = false;       /* the tail's kernels are launched            */
 };
 
 }  // namespace
@@ -226,7 +230,7 @@ bool reap(eg_server *s)
     bool any = false;
     for (size_t i = 0; i < s->inflight.size();) {
         Launch &l = s->inflight[i];
-        const cudaError_t e = cudaEventQuery(l.ev);
+        cudaError_t e = cudaEventQuery(l.ev);
         if (e == cudaErrorNotReady) {
             i++;
             continue;
@@ -236,7 +240,20 @@ bool reap(eg_server *s)
         UnitCtrl c;
         LaunchCtrl cv;
         memset(&c, 0, sizeof c);
-        if (e == cudaSuccess && cudaMemcpy(&cv, l.dctrl, sizeof cv, cudaMemcpyDeviceToHost) == cudaSuccess) {
+        const bool have = e == cudaSuccess && cudaMemcpy(&cv, l.dctrl, sizeof cv, cudaMemcpyDeviceToHost) == cudaSuccess;
+        if (have && !l.in_tail && tail_entries(l.set, cv) > 0) {
+            /* some units went to the tail: its kernels run now */
+            cudaStream_t st = s->streams[l.stream];
+            if (launch_tail(s->launchers[(size_t)l.stream], st, l.set, l.dunits, l.tl, l.dscratch, l.dctrl, s->sms,
+                            s->o.max_rounds, 0) == EG_OK &&
+                cudaEventRecord(l.ev, st) == cudaSuccess) {
+                l.in_tail = true;
+                i++;
+                continue;
+            }
+            e = cudaErrorLaunchFailure;
+        }
+        if (have) {
             sum_ctrl(cv, &c);
             if (!s->clock0) s->clock0 = c.t_begin;
             eg_serve_span sp;
@@ -422,23 +439,20 @@ bool admit(eg_server *s, std::unique_lock<std::mutex> &lk)
     return any;
 }
 
-/* One micro-batch of every admitted, not yet launched query (lock held). */
-bool launch_ready(eg_server *s)
+/* Device side of one micro-batch of the queries l.qids, up to its launch
+ * (lock held). */
+eg_status prepare_batch(eg_server *s, Launch &l)
 {
-    if (s->ready.empty() || (int)s->inflight.size() >= s->o.streams) return false;
     std::vector<UnitDesc> all;
     std::vector<long long> cost;
-    Launch l;
-    for (int64_t qid : s->ready) {
+    for (int64_t qid : l.qids) {
         Query &q = *s->queries[qid];
         all.insert(all.end(), q.units.begin(), q.units.end());
         cost.insert(cost.end(), q.cost.begin(), q.cost.end());
-        l.qids.push_back(qid);
     }
-    UnitSet S;
+    UnitSet &S = l.set;
     group_units(all, cost, std::vector<size_t>(all.size(), 0), &S, nullptr);
     l.stream = s->next_stream;
-    l.number = s->micro_batches;
     l.units = (int)S.units.size();
     s->next_stream = (s->next_stream + 1) % s->o.streams;
     cudaStream_t st = s->streams[l.stream];
@@ -451,41 +465,68 @@ bool launch_ready(eg_server *s)
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(l.dunits, S.units.data(), sizeof(UnitDesc) * S.units.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&l.ev, cudaEventDisableTiming);
-    eg_status ls = EG_OK;
-    TailList *tl = nullptr;
-    if (e == cudaSuccess) ls = tail_upload(S, l.dtails, st, &tl);
-    if (e == cudaSuccess && ls == EG_OK) {
+    if (e != cudaSuccess) return EG_ERR_CUDA;
+    return tail_upload(S, l.dtails, st, &l.tl);
+}
+
+/* Launches a prepared micro-batch, or fails its queries (lock held). */
+void start_batch(eg_server *s, Launch &l, eg_status ls)
+{
+    cudaStream_t st = s->streams[l.stream];
+    cudaError_t e = cudaSuccess;
+    if (ls == EG_OK) {
         int grid = 0;
-        ls = launch_unit_set(s->launchers[(size_t)l.stream], st, S, l.dunits, tl, l.dscratch, l.dctrl, s->o.block,
-                             s->sms, s->o.max_rounds, 0, &grid);
+        ls = launch_units(s->launchers[(size_t)l.stream], st, l.set, l.dunits, l.tl, l.dctrl, s->o.block, s->sms,
+                          s->o.max_rounds, 0, &grid);
         if (ls == EG_OK) e = cudaEventRecord(l.ev, st);
-        /* the tail list's host image is copied from pageable memory: wait for
-         * the copy before S goes out of scope */
-        if (ls == EG_OK && e == cudaSuccess) e = cudaStreamSynchronize(s->upload_stream);
     }
-    if (e != cudaSuccess || ls != EG_OK) {
-        cudaGetLastError();
-        const clk::time_point now = clk::now();
-        for (int64_t qid : l.qids) {
-            Query &q = *s->queries[qid];
-            s->device_bytes -= (int64_t)q.dbytes;
-            free_query_device(q, st);
-            s->games[q.game]->active--;
-            s->admitted_now--;
-            finish_query(s, q, ls != EG_OK ? ls : EG_ERR_CUDA, now);
-        }
-        if (l.ev) cudaEventDestroy(l.ev);
-        if (l.dunits) cudaFreeAsync(l.dunits, st);
-        if (l.dctrl) cudaFreeAsync(l.dctrl, st);
-        if (l.dtails) cudaFreeAsync(l.dtails, st);
-        if (l.dscratch) cudaFreeAsync(l.dscratch, st);
-        s->ready.clear();
-        s->cv_done.notify_all();
-        return true;
+    if (e == cudaSuccess && ls == EG_OK) {
+        l.number = s->micro_batches++;
+        s->inflight.push_back(std::move(l));
+        return;
     }
-    s->ready.clear();
-    s->inflight.push_back(l);
-    s->micro_batches++;
+    cudaGetLastError();
+    const clk::time_point now = clk::now();
+    for (int64_t qid : l.qids) {
+        Query &q = *s->queries[qid];
+        s->device_bytes -= (int64_t)q.dbytes;
+        free_query_device(q, st);
+        s->games[q.game]->active--;
+        s->admitted_now--;
+        finish_query(s, q, ls != EG_OK ? ls : EG_ERR_CUDA, now);
+    }
+    if (l.ev) cudaEventDestroy(l.ev);
+    if (l.dunits) cudaFreeAsync(l.dunits, st);
+    if (l.dctrl) cudaFreeAsync(l.dctrl, st);
+    if (l.dtails) cudaFreeAsync(l.dtails, st);
+    if (l.dscratch) cudaFreeAsync(l.dscratch, st);
+    s->cv_done.notify_all();
+}
+
+/* Launches the admitted queries (lock held): in two micro-batches where two
+ * streams are free, the queries dealt heaviest first, so that the first's
+ * read-back overlaps the second's run.  Both are prepared before the first
+ * is launched: they start a kernel launch apart. */
+bool launch_ready(eg_server *s)
+{
+    const int free_streams = s->o.streams - (int)s->inflight.size();
+    if (s->ready.empty() || free_streams <= 0) return false;
+    std::vector<int64_t> ready;
+    ready.swap(s->ready);
+    auto cost_of = [&](int64_t qid) {
+        long long c = 0;
+        for (long long x : s->queries[qid]->cost) c += x;
+        return c;
+    };
+    std::stable_sort(ready.begin(), ready.end(), [&](int64_t a, int64_t b) { return cost_of(a) > cost_of(b); });
+    const size_t parts = std::min<size_t>({2, (size_t)free_streams, ready.size()});
+    std::vector<Launch> ls(parts);
+    std::vector<eg_status> prep(parts, EG_OK);
+    for (size_t k = 0; k < parts; k++) {
+        for (size_t i = k; i < ready.size(); i += parts) ls[k].qids.push_back(ready[i]);
+        prep[k] = prepare_batch(s, ls[k]);
+    }
+    for (size_t k = 0; k < parts; k++) start_batch(s, ls[k], prep[k]);
     return true;
 }
 

@@ -186,3 +186,20 @@ def test_tail_shapes_give_identical_credits(tail_sweeps, tail_cluster):
         _, st = b.solve()
         assert st.games_failed == 0 and st.tail_entries == len(games) * 4
         check_batch(b, games, p, 2)
+
+
+@pytest.mark.parametrize("n,wmax,d,p", [
+    (200, 3000, 400, [-900000, 0, 5000, 700000]),       # 32-bit credits, weights too large for a potential
+    (200, 2600, 400, [-1000, 0, 7, 1000]),              # the largest weights that still have one
+    (300, 20, 1 << 16, [-(1 << 19), 0, 3, 1 << 19]),    # 64-bit credits
+    (2531, 100, 8, [473, -473, 0, 600]),                # several attempts: finite credits settle after 270 sweeps
+])
+def test_unit_certificates(n, wmax, d, p):
+    g = workloads.cfg4_games(64)[62] if n == 2531 else eg.generate(4, n, 9, wmax, 90 + n, param=2)
+    assert g.num_nodes == n
+    games, thresholds = [g, g], np.array([p, p[::-1]], dtype=np.int32)
+    with eg.Batch(games, thresholds=4, scale=d) as b:
+        b.set_thresholds(thresholds)
+        _, st = b.solve()
+        assert st.games_failed == 0
+        check_batch(b, games, thresholds, d)
