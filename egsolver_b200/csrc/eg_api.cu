@@ -79,9 +79,14 @@ struct eg_dgame {
     long long *d_rowptr;
     int *d_succ, *d_w;
     unsigned char *d_owner;
-    /* sweep solver: credits, potentials and their copy (n each), control */
-    long long *d_sweep;
+    /* sweep solver: control block, scratch of the grid kernel (see SweepPlan) */
     SweepCtrl *d_sctrl;
+    long long *d_sF, *d_sD, *d_sK;
+    int2 *d_sE;
+    int *d_svid, *d_soff;
+    void *sweep_block;
+    SweepPlan sweep_have;
+    size_t sweep_bytes;
     bool swept; /* d_out holds the last solve's credits, solved_bits wide */
     /* the arrays above and below, in one allocation each; the second (frontier
      * and dense rounds) is made by the first solve that runs those rounds */
@@ -102,7 +107,7 @@ struct eg_dgame {
     int *d_k0, *d_v0, *d_k1, *d_v1, *d_scratch;
     int *d_counts;
     unsigned long long *d_mg;
-    void *d_F, *d_out;
+    void *d_F, *d_out, *d_conv; /* d_conv: credits in another width */
     uint32_t *d_B;
     Ctrl *d_ctrl;
     /* heavy vertices cut into edge tasks (AUTO layout) */
@@ -267,11 +272,33 @@ extern "C" void eg_dgame_free(eg_dgame *g)
     if (g->st) cudaStreamSynchronize(g->st);
     if (g->block) cudaFree(g->block);
     if (g->rounds_block) cudaFree(g->rounds_block);
+    if (g->sweep_block) cudaFree(g->sweep_block);
     for (int i = 0; i < 6; i++)
         if (g->ev[i]) cudaEventDestroy(g->ev[i]);
     if (g->st) cudaStreamDestroy(g->st);
     cudaSetDevice(prev);
     free(g);
+}
+
+/* The sweep solver, unless the options ask for a kernel or for kinds of rounds
+ * of their own: a variant, a direction or its thresholds, the pair format or
+ * launch shape of those kernels, or their phase timers.  It was the faster one
+ * at every size measured, 100 to 2^20 vertices (0.5 ms against 0.03 ms, 9.3 s
+ * against 12 ms). */
+static bool routes_to_sweeps(const eg_opts *o)
+{
+    return !o || (o->variant == EG_VARIANT_AUTO && o->direction == EG_DIRECTION_SWITCH && o->dense_permille == 0 &&
+                  o->sparse_permille == 0 && !o->wide_pairs && o->schedule == 0 && o->ctas_per_sm == 0 && !o->profile);
+}
+
+static void sweep_arrays(eg_dgame *g, const SweepPlan &plan, Arena *ar)
+{
+    ar->add(&g->d_sF, plan.values);
+    ar->add(&g->d_sD, plan.values);
+    ar->add(&g->d_sK, plan.values);
+    ar->add(&g->d_sE, plan.edges);
+    ar->add(&g->d_svid, plan.vids);
+    ar->add(&g->d_soff, plan.offs);
 }
 
 static eg_status dgame_alloc(const eg_game *game, const eg_opts *opts, eg_dgame **out)
@@ -318,14 +345,40 @@ static eg_status dgame_alloc(const eg_game *game, const eg_opts *opts, eg_dgame 
     ar.add(&g->d_w, (size_t)g->m);
     if (g->has_owner) ar.add(&g->d_owner, (size_t)g->n);
     ar.add((int64_t **)&g->d_out, (size_t)g->n);
-    ar.add(&g->d_sweep, 3 * (size_t)g->n);
+    ar.add((int64_t **)&g->d_conv, (size_t)g->n);
     ar.add(&g->d_sctrl, 1);
+    SweepPlan plan;
+    memset(&plan, 0, sizeof plan);
+    if (s == EG_OK && routes_to_sweeps(opts)) s = sweep_plan(g->n, g->m, opts ? opts->grid_ctas : 0, &plan);
+    sweep_arrays(g, plan, &ar);
     if (s == EG_OK) s = ar.get(g, &g->block);
+    if (s == EG_OK) g->sweep_have = plan;
     if (s != EG_OK) {
         eg_dgame_free(g);
         return s;
     }
     *out = g;
+    return EG_OK;
+}
+
+/* The plan of a sweep solve and its scratch: that of the upload's options, or
+ * made again for a plan that needs more (another grid_ctas). */
+static eg_status sweep_reserve(eg_dgame *g, const eg_opts *opts, SweepPlan *plan)
+{
+    EG_TRY(sweep_plan(g->n, g->m, opts ? opts->grid_ctas : 0, plan));
+    const SweepPlan &have = g->sweep_have;
+    if (plan->values <= have.values && plan->edges <= have.edges && plan->vids <= have.vids && plan->offs <= have.offs)
+        return EG_OK;
+    if (g->sweep_block) cudaFree(g->sweep_block);
+    g->sweep_block = nullptr;
+    g->bytes -= g->sweep_bytes;
+    g->sweep_bytes = 0;
+    memset(&g->sweep_have, 0, sizeof g->sweep_have);
+    Arena ar;
+    sweep_arrays(g, *plan, &ar);
+    EG_TRY(ar.get(g, &g->sweep_block));
+    g->sweep_bytes = ar.total;
+    g->sweep_have = *plan;
     return EG_OK;
 }
 
@@ -545,11 +598,11 @@ static eg_status dgame_prepare(eg_dgame *g, const eg_opts *opts)
  * at TOP yet). */
 static void add_sweeps(const SweepCtrl &c, eg_stats *stats)
 {
-    stats->rounds += c.rounds;
+    stats->rounds += c.s.rounds;
     stats->lifts += (int64_t)c.lifts;
     stats->edges += (int64_t)c.edges;
     stats->changes += (int64_t)c.changes;
-    stats->dense_rounds += (int32_t)std::min<long long>(c.sweeps, INT32_MAX - stats->dense_rounds);
+    stats->dense_rounds += (int32_t)std::min<long long>(c.s.sweeps, INT32_MAX - stats->dense_rounds);
     stats->dense_launches++;
     stats->dense_changes += (int64_t)c.changes;
 }
@@ -614,7 +667,7 @@ static eg_status dgame_rounds(eg_dgame *g, const eg_opts *opts, const SweepCtrl 
     p.CH1 = g->d_B + 3 * wds;
     p.ctrl = g->d_ctrl;
     p.mg = g->mg;
-    p.max_rounds = before && opts->max_rounds >= 0 ? opts->max_rounds - before->rounds : opts->max_rounds;
+    p.max_rounds = before && opts->max_rounds >= 0 ? opts->max_rounds - before->s.rounds : opts->max_rounds;
     p.timeout_ns = opts->timeout_ms > 0 ? (unsigned long long)(opts->timeout_ms * 1e6) : 0ull;
     p.wait_limit_ns = kWaitLimitNs;
     p.cancel = nullptr;
@@ -800,9 +853,6 @@ static eg_status dgame_sweeps(eg_dgame *g, const eg_opts *opts, eg_stats *stats)
     p.n = g->n;
     p.n0 = g->n0;
     p.m = g->m;
-    p.F = g->d_sweep;
-    p.D = p.F + g->n;
-    p.K = p.D + g->n;
     p.out = g->d_out;
     p.ctrl = g->d_sctrl;
     p.max_rounds = opts->max_rounds;
@@ -813,21 +863,25 @@ static eg_status dgame_sweeps(eg_dgame *g, const eg_opts *opts, eg_stats *stats)
         EG_CUDA(cudaHostGetDevicePointer(&dp, (void *)opts->cancel, 0));
         p.cancel = (const int *)dp;
     }
-    p.lanes = 1;
-    while (p.lanes < 32 && 2LL * p.lanes * g->n <= g->m) p.lanes *= 2;
     p.sweeps = opts->dense_sweeps ? opts->dense_sweeps : kMaxDenseSweeps;
-    p.nshift = std::min(20, bits_for(g->n));
     p.bits = opts->credit_bits == 32 ? 32 : 64;
     p.narrow = opts->narrow;
     if (g->m >= kHandEdges) {
         p.hand_sweeps = kHandSweeps;
         p.hand_raised = kSparsePermille * g->n / 1000;
     }
+    SweepPlan plan;
+    EG_TRY(sweep_reserve(g, opts, &plan));
+    p.F = g->d_sF;
+    p.D = g->d_sD;
+    p.K = g->d_sK;
+    p.E = g->d_sE;
+    p.vid = g->d_svid;
+    p.soff = g->d_soff;
     EG_CUDA(cudaEventRecord(g->ev[0], st));
     EG_CUDA(cudaMemsetAsync(g->d_sctrl, 0, sizeof(SweepCtrl), st));
     EG_CUDA(cudaEventRecord(g->ev[1], st));
-    int grid = 0, block = 0;
-    EG_TRY(launch_sweep(p, st, opts->grid_ctas, &grid, &block));
+    EG_TRY(launch_sweep(p, plan, st));
     g->launches++;
     EG_CUDA(cudaEventRecord(g->ev[3], st));
     SweepCtrl c;
@@ -835,9 +889,10 @@ static eg_status dgame_sweeps(eg_dgame *g, const eg_opts *opts, eg_stats *stats)
     EG_CUDA(cudaStreamSynchronize(st));
     g->mg = (long long)c.mg;
     g->wmax = (long long)c.wmax;
-    if (c.stop == EG_ERR_OVERFLOW)
+    const int stop = c.abort ? (int)EG_ERR_TIMEOUT : c.s.stop;
+    if (stop == EG_ERR_OVERFLOW)
         return eg_set_error(EG_ERR_OVERFLOW, "MG = %lld does not fit 32-bit credits", g->mg);
-    if (c.phase == SWEEP_HANDOVER && !c.stop) return dgame_rounds(g, opts, &c, stats);
+    if (c.s.phase == SWEEP_HANDOVER && !stop) return dgame_rounds(g, opts, &c, stats);
     g->solved_bits = c.out_bits;
     g->solved = true;
     g->swept = true;
@@ -853,11 +908,11 @@ static eg_status dgame_sweeps(eg_dgame *g, const eg_opts *opts, eg_stats *stats)
         stats->dense_ms = lift_ms;
         stats->kernel_launches = g->launches;
         stats->credit_bits = c.out_bits;
-        stats->grid = grid;
-        stats->block = block;
+        stats->grid = plan.grid;
+        stats->block = plan.block;
         add_sweeps(c, stats);
     }
-    return stop_status(c.stop, c.abort, c.wait_site, opts);
+    return stop_status(stop, c.abort, c.wait_site, opts);
 }
 
 extern "C" eg_status eg_dgame_solve(eg_dgame *g, const eg_opts *opts_in, eg_stats *stats)
@@ -870,15 +925,7 @@ extern "C" eg_status eg_dgame_solve(eg_dgame *g, const eg_opts *opts_in, eg_stat
     EG_CUDA(cudaSetDevice(g->device));
     g->launches = 0;
     g->solved = false;
-    /* The sweep solver, unless the options ask for a kernel or for kinds of
-     * rounds of their own: a variant, a direction or its thresholds, the
-     * pair format or launch shape of those kernels, or their phase timers.
-     * It was the faster one at every size measured, 100 to 2^20 vertices
-     * (0.5 ms against 0.05 ms, 9.3 s against 16 ms). */
-    const bool sweeps = opts->variant == EG_VARIANT_AUTO && opts->direction == EG_DIRECTION_SWITCH &&
-                        opts->dense_permille == 0 && opts->sparse_permille == 0 && !opts->wide_pairs &&
-                        opts->schedule == 0 && opts->ctas_per_sm == 0 && !opts->profile;
-    return sweeps ? dgame_sweeps(g, opts, stats) : dgame_rounds(g, opts, nullptr, stats);
+    return routes_to_sweeps(opts) ? dgame_sweeps(g, opts, stats) : dgame_rounds(g, opts, nullptr, stats);
 }
 
 template <class O>
@@ -893,8 +940,8 @@ static eg_status dgame_credits(eg_dgame *g, O *host, int obits)
     if (!g->swept) {
         launch_gather_out(g->solved_bits, obits, g->n, g->d_iperm, g->d_F, g->d_out, g->st);
     } else if (obits != g->solved_bits) {
-        launch_gather_out(g->solved_bits, obits, g->n, nullptr, g->d_out, g->d_sweep, g->st);
-        src = g->d_sweep;
+        launch_gather_out(g->solved_bits, obits, g->n, nullptr, g->d_out, g->d_conv, g->st);
+        src = g->d_conv;
     }
     EG_CUDA(cudaMemcpyAsync(host, src, sizeof(O) * (size_t)g->n, cudaMemcpyDeviceToHost, g->st));
     EG_CUDA(cudaStreamSynchronize(g->st));

@@ -28,7 +28,7 @@
  * dual sum, so the certificate is complete; N is 2^nshift <= 2^20, and a
  * game that is not decided by it is decided by the climb.
  *
- * Schedule (advanced by each round's last arriver, on the device):
+ * Schedule (advanced by every CTA in the same way after each round):
  *   primal   sweeps of credit lifts; a round without a raise ends the solve;
  *   dual     sweeps that raise D, without a barrier between them, then a
  *            copy K = D;
@@ -41,448 +41,825 @@
  * without a newly certified vertex has lifted every vertex against the final
  * credits: the result is the least fixed point, as of any fair schedule.
  *
- * Layout.  The grid kernel runs one 1024-thread CTA per SM.  A CTA owns a
- * contiguous vertex range, cut so that 8 B per edge + 28 B per vertex is the
- * same for all; it keeps its vertices' credits and potentials, row offsets
- * and (when they fit) edges in shared memory for the whole solve, so a sweep
- * reads only the successors' values from L2.  `lanes` lanes share a vertex
- * (the mean out-degree rounded down to a power of two); vertices with more
- * out-edges than kHubEdges are cut into segments dealt to the CTA's warps.
- * Nothing is renumbered and no transpose is needed.  A game of at most
- * sweep_cta_bytes() <= the shared memory of a CTA runs in one CTA, with every
- * value in shared memory and __syncthreads for a barrier.
+ * Layout.  The grid kernel runs one CTA per SM.  A CTA owns a contiguous part
+ * of player 0's vertices and one of player 1's, cut so that 8 B per edge + 28 B
+ * per vertex is the same for all (both, because whole parts of one player's
+ * vertices are done early), and keeps their credits and potentials and their
+ * edges in shared memory for the whole solve: a sweep reads only the
+ * successors' values from L2.  Vertices of at most kLightDeg out-edges are
+ * sorted by (owner, out-degree) and cut into slices of 32, a warp's lanes; a
+ * slice's edges lie column by column, so a thread walks its vertex without
+ * bank conflicts, shuffles or much divergence.  A warp's lanes share a vertex
+ * of more edges; one of more than kHubEdges is cut into segments dealt to the
+ * CTA's warps.  The values that gathers read are numbered the same way (the
+ * CTA's base + slot), so a slice's raises are written as whole sectors.  No
+ * transpose is needed.  A game that fits one CTA runs in one, every value in
+ * shared memory and __syncthreads for a barrier.
  *
- * What bounds it: the chain of a sweep (shared-memory edge, L2 gather, store,
- * barrier) on small games, one gather per clock and SM on large ones.
- * Measured, whole solve on the device, against the frontier and dense rounds
- * that climb to MG: random 2..16-regular game of 131,072 vertices 684 ms ->
- * 0.43 ms (16 primal sweeps for 40,000), of 16,000 vertices 82 ms -> 0.18 ms;
- * power-law game of 2^20 vertices and 8.3 M edges 9.3 s -> 16 ms; complete
- * digraph of 2,000 vertices 14.2 ms -> 0.49 ms; 4-regular game of 1,000
- * vertices (one CTA) 4.1 ms -> 0.11 ms.
+ * What bounds it: instructions of the control between rounds and shared-memory
+ * latency in one CTA; the chain of a sweep (edge, L2 gather, store) and the
+ * barrier on games of some thousand vertices; the sectors that L2 delivers to
+ * random gathers on larger ones.
+ * Measured, device time of a whole solve: by frontier and dense rounds that
+ * climb to MG / by a first form of this kernel (lanes sharing a vertex in
+ * input order, 64-bit values, a barrier with a last arriver) / this one:
+ * uniform game of 131,072 vertices 684 ms / 0.41 / 0.28 ms, of 16,381 at a
+ * threshold 85 ms / 0.16 / 0.13 ms; power-law game of 2^20 vertices and 8.3 M
+ * edges 9.3 s / 15.9 / 4.2 ms, of 6,007 59 ms / 1.25 / 0.35 ms; complete digraph
+ * of 2,000 14.2 ms / 0.47 / 0.23 ms; 4-regular game of 1,000 4.1 ms / 0.11 /
+ * 0.05 ms (one CTA).
  *
- * Credits are int64 with TOP = 2^62 while the solve runs: OMINUS(a, w) is
- * g(a - w) with g(x) = x > MG ? TOP : max(x, 0), and MG + max |w| < 2^62
- * for every game that fits the 32-bit sizes, so a TOP successor always gives
- * TOP; g is monotone and is applied once, after the min or max.
+ * Credits are CT integers with TOP = Lim::top while the solve runs: OMINUS(a,
+ * w) is g(a - w) with g(x) = x > MG ? TOP : max(x, 0).  With MG + max |w| <
+ * TOP a TOP successor always gives TOP; g is monotone and is applied once,
+ * after the min or max.  CT is int32 (TOP = 2^30) where that bound and the
+ * potentials' allow, else int64 (TOP = 2^62, always enough: MG <= n 2^31).
  */
 #include "eg_sweep.cuh"
 
 #include <algorithm>
+#include <cstring>
 
 namespace eg {
 
-constexpr int kSweepBlock = 1024;
-constexpr int kHubEdges = 256;  /* out-edges above which a vertex is cut      */
-constexpr int kMaxTasks = 1040; /* segments of a CTA's cut vertices           */
-constexpr int kMaxHubs = 520;
-constexpr int kVertexBytes = 28; /* row offset, credit, potential, its copy   */
-constexpr int kFirstPrimal = 4, kFirstDual = 8, kSecondPrimal = 16, kMaxDual = 32, kMaxPrimal = 1 << 16;
-constexpr int kKillSweeps = 2;   /* kill sweeps between two grid barriers     */
+constexpr int kBlock = 512;      /* threads of a CTA: registers for eight gathers in flight each */
+constexpr int kWarps = kBlock / 32;
+constexpr int kLightDeg = 16;    /* out-edges up to which a thread may walk a vertex */
+constexpr int kHubEdges = 256;   /* out-edges above which a vertex is cut      */
+constexpr int kMaxTasks = 1040;  /* segments of a CTA's cut vertices           */
+constexpr int kBins = 2 * (kLightDeg + 1);
+constexpr int kVertexBytes = 28; /* credit, potential, its copy (8 B each), id */
+/* What a CTA's tables may take beyond 8 B per edge (8.5 B with the heavy
+ * vertices' heads) and 28 B per vertex: the slices' pads, at most 2 x 32 x
+ * kLightDeg edges per owner, and up to 62 slots without a vertex. */
+constexpr int kPadEdges = 4 * 32 * kLightDeg + 64, kPadSlots = 64, kSlackBytes = 8 * kPadEdges + 8192;
+/* Sweeps of the phases; the next dual and primal phases are twice as long.
+ * Measured on 131 K vertices / a power-law game of 2^20: first dual phase 6
+ * 284 us / 4.5 ms, 8 302 / 4.3; second primal phase 32 against 16, with which
+ * many games need a second attempt, 300 us / 4.3 ms against 301 / 5.6. */
+constexpr int kFirstPrimal = 2, kFirstDual = 6, kSecondPrimal = 32, kMaxDual = 32, kMaxPrimal = 1 << 16;
 
-constexpr long long kTop = 1LL << 62;    /* credit TOP; potential "out of S"  */
-constexpr long long kLow = -(1LL << 62); /* potential of a vertex at TOP      */
-constexpr long long kDualMax = 1LL << 61;
+/* flags of a round barrier's word */
+constexpr unsigned long long kTimeoutBit = 1ull << 40, kCancelBit = 1ull << 41, kRaiseMask = kTimeoutBit - 1;
 
-/* What a CTA knows of its vertex range. */
-struct Range {
-    int va, nv;              /* vertices [va, va + nv)                       */
-    int ne;                  /* their edges                                  */
-    const unsigned *off;     /* shared: first edge | owner << 31; or null    */
-    const long long *rp;     /* global row offsets of the range              */
-    long long e0;
-    const int2 *Es;          /* the edges in shared memory, or null          */
-    const int *succ, *w;     /* global, at the range's first edge            */
-    const unsigned char *owner;
-    int n0;
-    long long *myF, *myD, *myK; /* own values (shared, or global at va)      */
-    long long *gF, *gD, *gK; /* grid: the global values at va, which gathers read */
-    int lanes, nshift;
-    __device__ __forceinline__ void vertex(int i, int &b, int &e, bool &own) const
-    {
-        if (off) {
-            const unsigned x = off[i];
-            b = (int)(x & 0x7fffffffu);
-            e = (int)(off[i + 1] & 0x7fffffffu);
-            own = (x >> 31) != 0u;
-        } else {
-            b = (int)(rp[i] - e0);
-            e = (int)(rp[i + 1] - e0);
-            own = owner ? owner[va + i] != 0 : va + i >= n0;
-        }
-    }
+template <typename CT> struct Lim;
+template <> struct Lim<int> {
+    static constexpr int top = 1 << 30;      /* credit TOP; potential "out of S" */
+    static constexpr int low = -(1 << 30);   /* potential of a vertex at TOP     */
+    static constexpr int dual_max = 1 << 29;
+    static constexpr int weight_max = 1 << 20; /* of 2^nshift |w|                */
+    static constexpr int none = INT32_MAX;   /* the min over no edge             */
+};
+template <> struct Lim<long long> {
+    static constexpr long long top = 1LL << 62;
+    static constexpr long long low = -(1LL << 62);
+    static constexpr long long dual_max = 1LL << 61;
+    static constexpr long long weight_max = 1LL << 52;
+    static constexpr long long none = INT64_MAX;
 };
 
+/* Where a solve keeps what: KIND_CTA, one CTA with every value in shared
+ * memory; KIND_STAGED, the grid with each CTA's values and sliced edges in
+ * shared memory; KIND_GLOBAL, the grid with one or both in global memory. */
+enum { KIND_CTA, KIND_STAGED, KIND_GLOBAL };
+
+/* A CTA's vertices: slots 0 .. 32 ns - 1 hold the light ones (slice s = slots
+ * 32 s ..), slots 32 ns + h the heavy ones. */
+struct Range {
+    int ns, s0;              /* slices; first slice of player 1              */
+    int nh, nmed;            /* heavy vertices; those not cut (the first)    */
+    int base;                /* the grid's number of slot 0                  */
+    int own_smem;            /* own values, ids and offsets: shared memory   */
+    int stride;              /* bytes from credits to potentials to their copy there */
+    int at_vid, at_soff, at_E; /* offsets in shared memory of:               */
+    const int *vid;          /* vertex of each slot, -1: none                */
+    const int *soff;         /* slices' first column << 5 | columns          */
+    const int2 *E;           /* sliced edges: {successor's number, weight}   */
+    const int2 *head;        /* heavy vertices: {first edge in H, edges | owner << 31} */
+    const int2 *H;           /* their edges                                  */
+    void *g[3];              /* grid: F, D, K by number                      */
+    const long long *rp;     /* the input's row offsets                      */
+    int out_bits, round;     /* primal and kill sweeps between two barriers  */
+    long long mg, scale;
+};
+
+/* Vertices cut into segments (in shared memory). */
 struct Hubs {
-    int count, tasks, seg;
-    int hub[kMaxHubs], first[kMaxHubs]; /* vertex index; its first segment    */
-    unsigned task[kMaxTasks];           /* hub | segment << 16                */
+    int tasks, seg;
+    int first[kMaxTasks / 2];
+    unsigned task[kMaxTasks]; /* hub | segment << 16                          */
     long long part[kMaxTasks];
 };
 
-struct SweepCount {
-    unsigned raised, lifts;
-    unsigned long long edges;
+/* A thread's counts.  Lifts and scanned edges are counted once per vertex,
+ * when it reaches TOP or at the end: until then every primal sweep lifts it. */
+struct Count {
+    unsigned raised;
+    unsigned sweeps;          /* primal sweeps begun                         */
+    unsigned long long changes, lifts, edges;
+    __device__ __forceinline__ void settle(const long long *rp, int v)
+    {
+        lifts += sweeps;
+        edges += (unsigned long long)sweeps * (unsigned long long)(rp[v + 1] - rp[v]);
+    }
 };
 
-enum { MODE_PRIMAL, MODE_DUAL, MODE_KILL, MODE_SETUP };
+extern __shared__ __align__(16) unsigned char smem[];
 
-__device__ __forceinline__ long long shfl_xor_ll(long long v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+/* One kind of sweep: which array it lifts (0: credits, 1: potentials, 2:
+ * their copy) and how.  Primal: x = the min (player 0) or max (player 1) of
+ * f(v) - w; dual and kill: the max or min of D(v) + scale w + 1.  All are
+ * taken as a min, of `sign` x the edge's value, with sign = -1 for a max:
+ *   sign y + sign mul w,  mul = -1 (primal) or scale,
+ * and the result is sign x min + add. */
+template <typename CT>
+struct Kind {
+    int mode;
+    int mul;
+    CT cap, add;             /* largest value short of TOP; 0 or 1           */
+};
 
-/* Values read by gathers: other SMs write them (grid), or shared memory. */
-template <bool GRID>
-__device__ __forceinline__ long long gather(const long long *p)
+__device__ __forceinline__ int edge_value(int sign, int y, int mul, int w) { return sign * y + mul * w; }
+__device__ __forceinline__ long long edge_value(int sign, long long y, int mul, int w)
 {
-    return GRID ? __ldcg(p) : *p;
+    return (sign < 0 ? -y : y) + (long long)mul * (long long)w;
 }
 
-/* One edge's value in "min space": the lane keeps the least.  A max is the
- * min of negated values. */
-template <int MODE>
-__device__ __forceinline__ long long edge_value(long long x, int w, bool own, int nshift)
-{
-    if (MODE == MODE_PRIMAL) {
-        const long long v = x - (long long)w;
-        return own ? -v : v;
+/* Access to the places of a KIND: own values by slot; successors' by slot in
+ * one CTA, by number on the grid.  A slot without a vertex holds TOP,
+ * potential LOW. */
+template <typename CT, int KIND>
+struct Mem {
+    static __device__ __forceinline__ int vid(const Range &r, int slot)
+    {
+        return KIND == KIND_GLOBAL ? r.vid[slot] : *(const int *)(smem + r.at_vid + 4 * slot);
     }
-    const long long v = x + ((long long)w << nshift) + 1;
-    return own ? v : -v;
+    static __device__ __forceinline__ int soff(const Range &r, int s)
+    {
+        return KIND == KIND_GLOBAL ? r.soff[s] : *(const int *)(smem + r.at_soff + 4 * s);
+    }
+    static __device__ __forceinline__ CT own(const Range &r, int which, int slot)
+    {
+        if (KIND != KIND_GLOBAL || r.own_smem) return *(const CT *)(smem + which * r.stride + (int)sizeof(CT) * slot);
+        return ((const CT *)r.g[which])[r.base + slot];
+    }
+    static __device__ __forceinline__ void set(const Range &r, int which, int slot, CT x)
+    {
+        if (KIND != KIND_GLOBAL || r.own_smem) *(CT *)(smem + which * r.stride + (int)sizeof(CT) * slot) = x;
+        if (KIND == KIND_CTA) return;
+        if (sizeof(CT) == 4) __stcg((int *)r.g[which] + r.base + slot, (int)x);
+        else __stcg((long long *)r.g[which] + r.base + slot, (long long)x);
+    }
+    /* a successor's value; g, at_g: the array's global and shared place */
+    static __device__ __forceinline__ CT gather(const CT *g, int at_g, int at)
+    {
+        if (KIND == KIND_CTA) return *(const CT *)(smem + at_g + (int)sizeof(CT) * at);
+        if (sizeof(CT) == 4) return (CT)__ldcg((const int *)g + at);
+        return (CT)__ldcg((const long long *)g + at);
+    }
+};
+
+/* The last step of a vertex, by one thread. */
+template <typename CT, int KIND>
+__device__ __forceinline__ void finish_vertex(const Range &r, const Kind<CT> &k, int sign, int slot, CT old, CT acc,
+                                              Count &cnt)
+{
+    using M = Mem<CT, KIND>;
+    constexpr CT top = Lim<CT>::top;
+    const CT x = (sign < 0 ? -acc : acc) + k.add;
+    CT nv = x > 0 ? x : (CT)0;
+    if (nv > k.cap) nv = top;
+    if (nv <= old) return;
+    cnt.raised++;
+    if (k.mode == SWEEP_KILL) nv = top;
+    M::set(r, k.mode, slot, nv);
+    if (k.mode == SWEEP_PRIMAL && nv == top) {
+        M::set(r, 1, slot, Lim<CT>::low);
+        cnt.settle(r.rp, M::vid(r, slot));
+    }
 }
 
-template <bool GRID, bool ES, int MODE>
-__device__ __forceinline__ long long walk_edges(const Range &r, const long long *G, int k, int e, int step, bool own,
-                                                int nshift)
+/* U edges of each lane, `step` apart: their loads, then the gathers, then the
+ * values. */
+template <typename CT, int KIND, int U>
+__device__ __forceinline__ CT walk(const int2 *E, int left, int step, const CT *g, int at_g, int sign, int mul, CT acc)
 {
-    long long acc = INT64_MAX;
-    for (; k < e; k += 2 * step) {
-        const bool two = k + step < e;
-        int s0, w0, s1 = 0, w1 = 0;
-        if (ES) {
-            const int2 q = r.Es[k];
-            s0 = q.x;
-            w0 = q.y;
-            if (two) {
-                const int2 t = r.Es[k + step];
-                s1 = t.x;
-                w1 = t.y;
-            }
-        } else {
-            s0 = MODE == MODE_SETUP ? 0 : __ldg(r.succ + k);
-            w0 = __ldg(r.w + k);
-            if (two) {
-                s1 = MODE == MODE_SETUP ? 0 : __ldg(r.succ + k + step);
-                w1 = __ldg(r.w + k + step);
-            }
-        }
-        if (MODE == MODE_SETUP) { /* the least weight; largest |weight| in the high part is kept by the caller */
-            acc = min(acc, (long long)w0);
-            if (two) acc = min(acc, (long long)w1);
-        } else {
-            const long long x0 = gather<GRID>(G + s0);
-            const long long x1 = two ? gather<GRID>(G + s1) : 0;
-            acc = min(acc, edge_value<MODE>(x0, w0, own, nshift));
-            if (two) acc = min(acc, edge_value<MODE>(x1, w1, own, nshift));
-        }
+    int2 q[U];
+    CT y[U];
+#pragma unroll
+    for (int j = 0; j < U; j++) {
+        q[j].x = -1;
+        if (j * step < left) q[j] = E[j * step];
     }
+#pragma unroll
+    for (int j = 0; j < U; j++)
+        if (q[j].x >= 0) y[j] = Mem<CT, KIND>::gather(g, at_g, q[j].x);
+#pragma unroll
+    for (int j = 0; j < U; j++)
+        if (q[j].x >= 0) acc = min(acc, edge_value(sign, y[j], mul, q[j].y));
     return acc;
 }
 
-/* The vertex's own value, and whether this kind of sweep passes it over. */
-template <int MODE>
-__device__ __forceinline__ bool own_value(const Range &r, int i, long long &old)
-{
-    if (MODE == MODE_SETUP) return true;
-    old = MODE == MODE_PRIMAL ? r.myF[i] : MODE == MODE_DUAL ? r.myD[i] : r.myK[i];
-    return old < kTop && old != kLow;
-}
+/* Loads in flight per lane: a few for shared-memory gathers, enough to cover
+ * an L2 gather for all but the longest rows. */
+template <int KIND> constexpr int kUnroll = KIND == KIND_CTA ? 2 : 8;
 
-/* The last step of a vertex (one lane): acc is the min-space result. */
-template <bool GRID, int MODE>
-__device__ __forceinline__ void finish_vertex(const Range &r, int i, bool own, long long old,
-                                              long long acc, int deg, long long mg, unsigned long long &mg_sum,
-                                              SweepCount &cnt)
+/* The heavy vertices of one sweep: first the segments of those that are cut,
+ * then a warp per vertex of the others (the warps with the fewest slices
+ * first), then the cut ones' results. */
+template <typename CT, int KIND>
+__device__ __forceinline__ void sweep_heavy(const Range &r, const Kind<CT> &kd, Hubs &hb, Count &cnt)
 {
-    if (MODE == MODE_SETUP) {
-        if (acc < 0) mg_sum += (unsigned long long)(-acc);
-        return;
-    }
-    if (MODE == MODE_PRIMAL) {
-        const long long x = own ? -acc : acc;
-        const long long nv = x > mg ? kTop : (x > 0 ? x : 0);
-        cnt.lifts++;
-        cnt.edges += (unsigned)deg;
-        if (nv > old) {
-            cnt.raised++;
-            r.myF[i] = nv;
-            if (GRID) __stcg(r.gF + i, nv);
-            if (nv == kTop) {
-                r.myD[i] = kLow;
-                if (GRID) __stcg(r.gD + i, kLow);
-            }
-        }
-        return;
-    }
-    long long y = own ? acc : -acc;
-    y = y > 0 ? y : 0;
-    if (y <= old) return;
-    if (MODE == MODE_DUAL) {
-        if (y > kDualMax) y = kTop;
-        r.myD[i] = y;
-        if (GRID) __stcg(r.gD + i, y);
-    } else {
-        cnt.raised++;
-        r.myK[i] = kTop;
-        if (GRID) __stcg(r.gK + i, kTop);
-    }
-}
-
-/* One sweep of the CTA's vertices. */
-template <bool GRID, bool ES, int MODE>
-__device__ __forceinline__ void sweep(const Range &range, Hubs &hb, const long long *G, long long mg,
-                                   unsigned long long &mg_out, SweepCount &cnt_out)
-{
-    /* copies in registers: stores to credits cannot alias them */
-    const Range r = range;
-    SweepCount cnt = cnt_out;
-    unsigned long long mg_sum = 0;
+    using M = Mem<CT, KIND>;
+    constexpr int U = kUnroll<KIND>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    constexpr int nwarps = kSweepBlock / 32;
-    const int g = r.lanes, gl = lane & (g - 1);
-    const int nshift = r.nshift;
-    const bool hubs = hb.count > 0;
+    const int slot0 = 32 * r.ns;
+    const bool hubs = r.nh > r.nmed;
+    const CT *g = (const CT *)r.g[kd.mode];
+    const int at_g = kd.mode * r.stride;
+    int2 hd;
+    int sign;
+    CT old;
+    auto open = [&](int h) {
+        old = M::own(r, kd.mode, slot0 + h);
+        if (old >= Lim<CT>::top || old == Lim<CT>::low) return false;
+        hd = r.head[h];
+        sign = (hd.y < 0) == (kd.mode == SWEEP_PRIMAL) ? -1 : 1;
+        hd.y &= INT32_MAX;
+        return true;
+    };
+    auto lanes_min = [&](int k0, int k1) {
+        CT acc = Lim<CT>::none;
+#pragma unroll 1
+        for (int k = k0 + lane; k < k1; k += 32 * U)
+            acc = walk<CT, KIND, U>(r.H + hd.x + k, k1 - k, 32, g, at_g, sign, sign * kd.mul, acc);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc = min(acc, (CT)__shfl_xor_sync(0xffffffffu, acc, o));
+        return acc;
+    };
     if (hubs) {
-        for (int t = warp; t < hb.tasks; t += nwarps) {
+        for (int t = warp; t < hb.tasks; t += kWarps) {
             const unsigned tk = hb.task[t];
-            const int i = hb.hub[tk & 0xffffu];
-            int b, e;
-            bool own;
-            long long old = 0;
-            r.vertex(i, b, e, own);
-            long long acc = INT64_MAX;
-            if (own_value<MODE>(r, i, old)) {
-                const int k0 = b + (int)(tk >> 16) * hb.seg;
-                acc = walk_edges<GRID, ES, MODE>(r, G, k0 + lane, min(e, k0 + hb.seg), 32, own, nshift);
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc = min(acc, shfl_xor_ll(acc, o));
-            if (lane == 0) hb.part[t] = acc;
+            if (!open(r.nmed + (int)(tk & 0xffffu))) continue;
+            const int k0 = (int)(tk >> 16) * hb.seg;
+            const CT acc = lanes_min(k0, min(hd.y, k0 + hb.seg));
+            if (lane == 0) hb.part[t] = (long long)acc;
         }
     }
-    const int per = 32 / g;
-    for (int i0 = warp * per; i0 < r.nv; i0 += nwarps * per) {
-        const int i = i0 + lane / g;
-        int b = 0, e = 0;
-        bool own = false;
-        long long old = 0;
-        bool act = i < r.nv;
-        if (act) {
-            r.vertex(i, b, e, own);
-            act = (e - b <= hb.seg || !hubs) && own_value<MODE>(r, i, old);
-        }
-        long long acc = INT64_MAX;
-        if (act) acc = walk_edges<GRID, ES, MODE>(r, G, b + gl, e, g, own, nshift);
-        __syncwarp();
-        for (int o = g >> 1; o > 0; o >>= 1) acc = min(acc, shfl_xor_ll(acc, o));
-        if (act && gl == 0) finish_vertex<GRID, MODE>(r, i, own, old, acc, e - b, mg, mg_sum, cnt);
+    for (int h = (warp - r.ns) & (kWarps - 1); h < r.nmed; h += kWarps) {
+        if (!open(h)) continue;
+        const CT acc = lanes_min(0, hd.y);
+        if (lane == 0) finish_vertex<CT, KIND>(r, kd, sign, slot0 + h, old, acc, cnt);
     }
     if (hubs) {
         __syncthreads();
-        for (int h = warp; h < hb.count; h += nwarps) {
-            const int i = hb.hub[h];
-            int b, e;
-            bool own;
-            long long old = 0;
-            r.vertex(i, b, e, own);
-            const int nt = (e - b + hb.seg - 1) / hb.seg;
-            long long acc = INT64_MAX;
-            for (int t = lane; t < nt; t += 32) acc = min(acc, hb.part[hb.first[h] + t]);
+        for (int h = r.nmed + warp; h < r.nh; h += kWarps) {
+            if (!open(h)) continue;
+            const int nt = (hd.y + hb.seg - 1) / hb.seg, t0 = hb.first[h - r.nmed];
+            CT acc = Lim<CT>::none;
+            for (int t = lane; t < nt; t += 32) acc = min(acc, (CT)hb.part[t0 + t]);
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc = min(acc, shfl_xor_ll(acc, o));
-            if (lane == 0 && own_value<MODE>(r, i, old))
-                finish_vertex<GRID, MODE>(r, i, own, old, acc, e - b, mg, mg_sum, cnt);
+            for (int o = 16; o > 0; o >>= 1) acc = min(acc, (CT)__shfl_xor_sync(0xffffffffu, acc, o));
+            if (lane == 0) finish_vertex<CT, KIND>(r, kd, sign, slot0 + h, old, acc, cnt);
         }
         __syncthreads();
     }
-    cnt_out = cnt;
-    if (MODE == MODE_SETUP) mg_out += mg_sum;
 }
 
-/* The schedule after a round in which `raised` values changed. */
-__device__ __forceinline__ void advance(const SweepParams &p, SweepCtrl *c, int ran, unsigned long long raised)
+/* One sweep of the CTA's vertices: the light ones here, a slice per warp, a
+ * vertex per lane. */
+template <typename CT, int KIND>
+__device__ __forceinline__ void sweep(const Range &r, const Kind<CT> &kd, Hubs &hb, Count &cnt)
 {
-    if (c->phase == SWEEP_PRIMAL) {
-        const long long round = c->rounds;
-        c->rounds = round + 1;
-        c->sweeps += ran;
-        c->left -= ran;
-        c->changes += raised;
+    using M = Mem<CT, KIND>;
+    constexpr int U = kUnroll<KIND>;
+    const int lane = threadIdx.x & 31;
+    const CT *g = (const CT *)r.g[kd.mode];
+    const int at_g = kd.mode * r.stride;
+    for (int s = threadIdx.x >> 5; s < r.ns; s += kWarps) {
+        const int slot = 32 * s + lane;
+        const int x = M::soff(r, s);
+        const int sign = (s >= r.s0) == (kd.mode == SWEEP_PRIMAL) ? -1 : 1;
+        const CT old = M::own(r, kd.mode, slot);
+        if (old >= Lim<CT>::top || old == Lim<CT>::low) continue;
+        const int2 *E = KIND == KIND_GLOBAL ? r.E + 32 * (long long)(x >> 5) + lane
+                                            : (const int2 *)(smem + r.at_E) + 32 * (x >> 5) + lane;
+        CT acc = Lim<CT>::none;
+#pragma unroll 1
+        for (int left = 32 * (x & 31); left > 0; left -= 32 * U, E += 32 * U)
+            acc = walk<CT, KIND, U>(E, left, 32, g, at_g, sign, sign * kd.mul, acc);
+        finish_vertex<CT, KIND>(r, kd, sign, slot, old, acc, cnt);
+    }
+    if (r.nh) sweep_heavy<CT, KIND>(r, kd, hb, cnt);
+}
+
+/* The schedule after a round of `ran` sweeps in which `raised` values changed
+ * (any number but 0 where it is only compared with that). */
+__device__ __forceinline__ void advance(const SweepParams &p, SweepState &c, int ran, unsigned long long raised, int stop)
+{
+    if (c.phase == SWEEP_PRIMAL) {
+        c.rounds++;
+        c.sweeps += ran;
+        c.left -= ran;
         if (raised == 0ull) {
-            c->phase = SWEEP_DONE;
+            c.phase = SWEEP_DONE;
             return;
         }
-        if (p.max_rounds >= 0 && round + 1 >= p.max_rounds) c->stop = (int)EG_ERR_LOOPCAP;
-        else if (p.timeout_ns && globaltimer_ns() - c->t_start > p.timeout_ns) c->stop = (int)EG_ERR_TIMEOUT;
-        else if (p.cancel && (round & 63) == 0 && ld_volatile(p.cancel)) c->stop = (int)EG_ERR_CANCELLED;
-        if (c->stop) return;
-        if (c->left <= 0) {
-            if (p.hand_sweeps && c->sweeps >= p.hand_sweeps && (long long)raised < p.hand_raised) {
-                c->phase = SWEEP_HANDOVER;
-                return;
-            }
-            c->phase = SWEEP_DUAL;
-            c->left = c->dual_len;
+        c.stop = p.max_rounds >= 0 && c.rounds >= p.max_rounds ? (int)EG_ERR_LOOPCAP : stop;
+        if (c.left > 0) return;
+        if (p.hand_sweeps && c.sweeps >= p.hand_sweeps && (long long)raised < p.hand_raised) {
+            c.phase = SWEEP_HANDOVER;
+            return;
         }
-    } else if (c->phase == SWEEP_DUAL) {
-        c->dual_sweeps += ran;
-        c->dual_len = min(2 * c->dual_len, kMaxDual);
-        c->phase = SWEEP_KILL;
-    } else {
-        c->kill_sweeps += ran;
-        if (raised == 0ull) {
-            c->attempts++;
-            c->phase = SWEEP_PRIMAL;
-            c->left = c->primal_len;
-            c->primal_len = min(2 * c->primal_len, kMaxPrimal);
-        }
+        c.phase = SWEEP_DUAL;
+        c.left = c.dual_len;
+    } else if (c.phase == SWEEP_DUAL) {
+        c.dual_len = min(2 * c.dual_len, kMaxDual);
+        c.phase = SWEEP_KILL;
+    } else if (raised == 0ull) {
+        c.phase = SWEEP_PRIMAL;
+        c.left = c.primal_len;
+        c.primal_len = min(2 * c.primal_len, kMaxPrimal);
     }
 }
 
-/* First vertex v with 8 rp[v] + 28 v >= target, for two targets at once: a
- * search in which every thread probes one place per step. */
-__device__ __forceinline__ void find_range(const SweepParams &p, unsigned long long ta, unsigned long long tb, int &va,
-                                           int &vb)
+__device__ __forceinline__ unsigned long long ld_acquire_gpu64(const unsigned long long *p)
 {
-    constexpr int half = kSweepBlock / 2;
-    const bool first = threadIdx.x < half;
-    const int t = threadIdx.x & (half - 1);
-    const unsigned long long target = first ? ta : tb;
-    int lo[2] = {0, 0}, hi[2] = {p.n, p.n}; /* the answer is in [lo, hi] */
-    while (lo[0] < hi[0] || lo[1] < hi[1]) {
-        const int l = first ? lo[0] : lo[1], h = first ? hi[0] : hi[1];
-        const int step = (h - l + half - 1) / half;
-        const long long at = (long long)l + (long long)t * step;
-        const bool below = at < h && (unsigned long long)p.rp[at] * 8ull + (unsigned long long)at * kVertexBytes < target;
-        const int ca = __syncthreads_count(below && first);
-        const int cb = __syncthreads_count(below && !first);
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const int c = k ? cb : ca;
-            const int l2 = lo[k], h2 = hi[k];
-            if (l2 >= h2) continue;
-            const int st = (h2 - l2 + half - 1) / half;
-            const long long next = (long long)l2 + (long long)c * st; /* first probe not below */
-            if (c > 0) lo[k] = (int)(l2 + (long long)(c - 1) * st + 1);
-            if (next < h2) hi[k] = (int)next;
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
+/* Round barrier `it` of the grid (thread 0 of each CTA): one atomic carries
+ * the arrival, this CTA's raises and (CTA 0) the stop flags, and everybody
+ * polls that word until all have arrived, so it also brings the sum of the
+ * raises: one round trip and a poll, 2,400 cycles with 148 CTAs (a flag per
+ * CTA that all poll: 4,500 to 7,300; a last arriver that publishes a decision:
+ * about 10,000).  Words are used in turn; word it + 2 was last read at
+ * barrier it - 2, which all CTAs have left.  Bounded by wait_limit_ns; returns
+ * false when a CTA gave up. */
+__device__ __forceinline__ bool round_barrier(const SweepParams &p, SweepCtrl *c, unsigned it, unsigned long long give,
+                                              unsigned long long *sum)
+{
+    unsigned long long *w = &c->word[it & 3][0];
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(w), "l"((1ull << 48) | give) : "memory");
+    unsigned long long v, t0 = 0;
+    unsigned spins = 0;
+    while (((v = ld_acquire_gpu64(w)) >> 48) != gridDim.x) {
+        if ((++spins & 255) == 0) {
+            if (ld_volatile(&c->abort)) return false;
+            const unsigned long long now = globaltimer_ns();
+            if (!t0) t0 = now;
+            else if (now - t0 > p.wait_limit_ns) {
+                c->wait_site = it;
+                atomicExch(&c->abort, 1);
+                return false;
+            }
         }
     }
-    va = lo[0];
-    vb = lo[1];
+    if (blockIdx.x == 0) c->word[(it + 2) & 3][0] = 0ull;
+    *sum = v & ((1ull << 48) - 1);
+    return true;
+}
+
+/* What a CTA's threads tell each other at the end of a round. */
+struct Turn {
+    unsigned raised[2];       /* by parity                                   */
+    unsigned long long sum;   /* grid: the barrier's sum and flags           */
+    int ok, stop;
+};
+
+/* Everything after the set-up, for one credit width and kind.  Not inlined:
+ * each has its registers to itself. */
+template <typename CT, int KIND>
+__device__ __noinline__ void solve(const SweepParams *pp, const Range &rs, Hubs &hb, Turn &turn, SweepState &state,
+                                   unsigned it, Count &count)
+{
+    using M = Mem<CT, KIND>;
+    constexpr bool GRID = KIND != KIND_CTA;
+    constexpr CT top = Lim<CT>::top, low = Lim<CT>::low;
+    const SweepParams &p = *pp;
+    const Range r = rs;
+    SweepState st = state;
+    Count cnt = count;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int nslots = 32 * r.ns + r.nh;
+    const bool watch = p.timeout_ns || p.cancel;
+    bool ok = turn.ok != 0, mark = false;
+    /* slots without a vertex are never lifted (the others start at 0) */
+    for (int i = tid; i < 32 * r.ns; i += kBlock) {
+        if (M::vid(r, i) < 0) {
+            M::set(r, 0, i, top);
+            M::set(r, 1, i, low);
+        }
+    }
+    __syncthreads();
+    while (ok && !st.stop && st.phase < SWEEP_DONE) {
+        const int phase = st.phase;
+        cnt.raised = 0u;
+        if (mark) { /* the certified vertices: TOP */
+            for (int i = tid; i < nslots; i += kBlock) {
+                const CT k = M::own(r, 2, i);
+                if (k < top && k != low) {
+                    M::set(r, 0, i, top);
+                    M::set(r, 1, i, low);
+                    cnt.raised++;
+                    cnt.settle(r.rp, M::vid(r, i));
+                }
+            }
+            __syncthreads();
+        }
+        Kind<CT> kd;
+        kd.mode = phase;
+        kd.mul = phase == SWEEP_PRIMAL ? -1 : (int)r.scale;
+        kd.cap = phase == SWEEP_PRIMAL ? (CT)r.mg : Lim<CT>::dual_max;
+        kd.add = phase == SWEEP_PRIMAL ? (CT)0 : (CT)1;
+        const int ran = phase == SWEEP_DUAL ? st.left : phase == SWEEP_KILL ? min(r.round, 2) : min(r.round, st.left);
+#pragma unroll 1
+        for (int s = 0; s < ran; s++) {
+            if (phase == SWEEP_PRIMAL) cnt.sweeps++;
+            sweep<CT, KIND>(r, kd, hb, cnt);
+        }
+        if (phase == SWEEP_PRIMAL) cnt.changes += cnt.raised;
+        if (phase == SWEEP_DUAL) {
+            __syncthreads();
+            for (int i = tid; i < nslots; i += kBlock) M::set(r, 2, i, M::own(r, 1, i));
+        }
+        /* the round's raises and the next step of the schedule */
+        unsigned long long raised;
+        int stop = 0;
+        if (tid == 0 && watch && blockIdx.x == 0 && phase == SWEEP_PRIMAL) {
+            if (p.timeout_ns && globaltimer_ns() - p.ctrl->t_start > p.timeout_ns) stop = (int)EG_ERR_TIMEOUT;
+            else if (p.cancel && (st.rounds & 63) == 0 && ld_volatile(p.cancel)) stop = (int)EG_ERR_CANCELLED;
+        }
+        if (GRID) {
+            const unsigned d = __reduce_add_sync(0xffffffffu, cnt.raised);
+            if (lane == 0 && d) atomicAdd(&turn.raised[it & 1], d);
+            __syncthreads();
+            if (tid == 0) {
+                unsigned long long give = turn.raised[it & 1], got = 0ull;
+                turn.raised[it & 1] = 0u; /* next used two rounds on */
+                if (stop) give |= stop == (int)EG_ERR_TIMEOUT ? kTimeoutBit : kCancelBit;
+                turn.ok = round_barrier(p, p.ctrl, it, give, &got);
+                turn.sum = got;
+            }
+            __syncthreads();
+            ok = turn.ok != 0;
+            raised = turn.sum & kRaiseMask;
+            stop = turn.sum & kTimeoutBit ? (int)EG_ERR_TIMEOUT : turn.sum & kCancelBit ? (int)EG_ERR_CANCELLED : 0;
+        } else {
+            if (tid == 0 && watch) turn.stop = stop;
+            raised = (unsigned long long)__syncthreads_or((int)cnt.raised);
+            if (watch) {
+                stop = turn.stop;
+                __syncthreads();
+            }
+        }
+        advance(p, st, ran, raised, stop);
+        mark = phase == SWEEP_KILL && st.phase == SWEEP_PRIMAL;
+        it++;
+    }
+    __syncthreads();
+    /* credits out; TOPs are counted in `raised` */
+    cnt.raised = 0u;
+    for (int i = tid; i < nslots; i += kBlock) {
+        const int v = M::vid(r, i);
+        if (v < 0) continue;
+        const CT f = M::own(r, 0, i);
+        if (f == top) cnt.raised++;
+        else cnt.settle(r.rp, v);
+        if (r.out_bits == 32) ((int *)p.out)[v] = f == top ? INT32_MAX : (int)f;
+        else ((long long *)p.out)[v] = f == top ? (long long)INT64_MAX : (long long)f;
+    }
+    count = cnt;
+    state = st;
+}
+
+__device__ __forceinline__ unsigned long long cost_before(const SweepParams &p, long long v)
+{
+    return (unsigned long long)p.rp[v] * 8ull + (unsigned long long)v * kVertexBytes;
+}
+
+/* Cuts both players' vertices into gridDim.x parts of equal cost: cut[0] ..
+ * cut[1] of player 0's [0, split) and cut[2] .. cut[3] of player 1's [split,
+ * n) are this CTA's.  A search in which 128 threads probe places for each cut
+ * at a time. */
+__device__ __forceinline__ void find_cuts(const SweepParams &p, int split, int *s_probe, int *cut)
+{
+    const int q = threadIdx.x >> 7, t = threadIdx.x & 127;
+    const int b0 = q < 2 ? 0 : split, b1 = q < 2 ? split : p.n;
+    const unsigned long long c0 = cost_before(p, b0), total = cost_before(p, b1) - c0;
+    const unsigned long long part = blockIdx.x + (q & 1), parts = gridDim.x;
+    const unsigned long long target = c0 + total / parts * part + total % parts * part / parts;
+    int lo = b0, hi = part == parts ? b0 : b1; /* the answer is in [lo, hi] */
+    if (part == parts) lo = hi = b1;
+    if (threadIdx.x < 4) s_probe[threadIdx.x] = 0;
+    for (;;) {
+        const int step = (hi - lo + 127) >> 7;
+        const long long at = (long long)lo + (long long)t * step;
+        const bool below = at < hi && cost_before(p, at) < target;
+        const unsigned m = __ballot_sync(0xffffffffu, below);
+        if (!__syncthreads_or(lo < hi)) break;
+        if ((threadIdx.x & 31) == 0 && m) atomicAdd(&s_probe[q], __popc(m));
+        __syncthreads();
+        const int c = s_probe[q]; /* probes below the target: the first c */
+        __syncthreads();
+        if (threadIdx.x < 4) s_probe[threadIdx.x] = 0;
+        if (lo < hi) {
+            const long long next = (long long)lo + (long long)c * step;
+            if (c > 0) lo = (int)((long long)lo + (long long)(c - 1) * step + 1);
+            if (next < hi) hi = (int)next;
+        }
+    }
+    if (t == 0) s_probe[q] = lo;
+    __syncthreads();
+    for (int k = 0; k < 4; k++) cut[k] = s_probe[k];
+    __syncthreads();
 }
 
 template <bool GRID>
-__global__ void __launch_bounds__(kSweepBlock, 1) k_sweep(const __grid_constant__ SweepParams p)
+__global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ SweepParams p)
 {
-    extern __shared__ __align__(16) unsigned char smem[];
     __shared__ Hubs hb;
-    __shared__ unsigned long long s_sum[4];
-    __shared__ SweepCtrl s_ctrl; /* one-CTA kernel */
-    SweepCtrl *c = GRID ? p.ctrl : &s_ctrl;
-    const int tid = threadIdx.x, lane = tid & 31;
-    if (!GRID) {
-        for (int i = tid; i < (int)(sizeof(SweepCtrl) / 4); i += kSweepBlock) ((int *)&s_ctrl)[i] = 0;
-        __syncthreads();
+    __shared__ Turn turn;
+    __shared__ Range r;
+    __shared__ SweepParams ps;
+    __shared__ unsigned long long s_sum[4]; /* MG, largest |weight|; then TOPs, lifts, edges, raises */
+    __shared__ int s_bin[kBins];            /* light vertices by owner and out-degree, then their next slot */
+    __shared__ int s_cls[4];                /* first slot past the light vertices of player 0; of player 1; columns; light */
+    __shared__ int s_heavy[4];              /* heavy vertices: not cut, cut; their edges; next offset */
+    __shared__ int s_scan[kWarps];
+    SweepCtrl *c = p.ctrl;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    /* with an owner array the players' vertices are not apart: one part */
+    const int split = p.owner ? p.n : p.n0;
+    int cut[4] = {0, split, split, p.n};
+    if (GRID) find_cuts(p, split, s_heavy, cut);
+    const int nv0 = cut[1] - cut[0], nv = nv0 + cut[3] - cut[2];
+    const int gap = cut[2] - nv0; /* vertex i of the CTA: cut[0] + i, or gap + i from nv0 on */
+    const long long e0 = p.rp[cut[0]], e1 = p.rp[cut[2]];
+    const int ne = (int)(p.rp[cut[1]] - e0 + p.rp[cut[3]] - e1);
+    const int seg = max(kHubEdges, (ne / 512 + 31) & ~31); /* at most 512 + 512 segments */
+    __syncthreads();
+    if (tid < kBins) s_bin[tid] = 0;
+    if (tid < 4) {
+        s_sum[tid] = 0ull;
+        s_heavy[tid] = 0;
     }
-    if (tid == 0 && blockIdx.x == 0) c->t_start = globaltimer_ns();
-    Range r;
-    int vb;
-    if (GRID) {
-        const unsigned long long total = (unsigned long long)p.m * 8ull + (unsigned long long)p.n * kVertexBytes;
-        const unsigned long long g = gridDim.x, b = blockIdx.x;
-        find_range(p, total / g * b + total % g * b / g, total / g * (b + 1) + total % g * (b + 1) / g, r.va, vb);
-        if (b + 1 == g) vb = p.n;
-    } else {
-        r.va = 0;
-        vb = p.n;
-    }
-    r.nv = vb - r.va;
-    r.e0 = p.rp[r.va];
-    r.ne = (int)(p.rp[vb] - r.e0);
-    r.rp = p.rp + r.va;
-    r.succ = p.succ + r.e0;
-    r.w = p.w + r.e0;
-    r.owner = p.owner;
-    r.n0 = p.n0;
-    r.gF = p.F + r.va;
-    r.gD = p.D + r.va;
-    r.gK = p.K + r.va;
-    r.lanes = p.lanes;
-    r.nshift = p.nshift;
-    /* shared memory: own values and row offsets, then the edges */
-    const long long own_bytes = ((long long)r.nv * kVertexBytes + 4 + 15) & ~15LL;
-    const bool own_fits = own_bytes <= p.smem_bytes;
-    r.off = nullptr;
-    r.Es = nullptr;
-    if (own_fits) {
-        r.myF = (long long *)smem;
-        r.myD = r.myF + r.nv;
-        r.myK = r.myD + r.nv;
-        unsigned *off = (unsigned *)(r.myK + r.nv);
-        r.off = off;
-        for (int i = tid; i <= r.nv; i += kSweepBlock) {
-            unsigned own = 0;
-            if (i < r.nv) own = p.owner ? (unsigned)(p.owner[r.va + i] != 0) : (unsigned)(r.va + i >= p.n0);
-            off[i] = (unsigned)(r.rp[i] - r.e0) | own << 31;
-        }
-        if (own_bytes + 8LL * r.ne <= p.smem_bytes) {
-            int2 *Es = (int2 *)(smem + own_bytes);
-            r.Es = Es;
-            for (int k = tid; k < r.ne; k += kSweepBlock) Es[k] = make_int2(__ldg(r.succ + k), __ldg(r.w + k));
-        }
-    } else {
-        r.myF = r.gF;
-        r.myD = r.gD;
-        r.myK = r.gK;
-    }
-    for (int i = tid; i < r.nv; i += kSweepBlock) {
-        r.myF[i] = 0;
-        r.myD[i] = 0;
-        if (GRID && own_fits) {
-            __stcg(r.gF + i, 0LL);
-            __stcg(r.gD + i, 0LL);
-        }
-    }
-    /* the range's heavy vertices, cut into at most kMaxTasks segments */
-    const int seg = max(kHubEdges, (r.ne / 512 + 31) & ~31);
     if (tid == 0) {
-        hb.count = 0;
+        if (blockIdx.x == 0) c->t_start = globaltimer_ns();
         hb.tasks = 0;
         hb.seg = seg;
+        turn.raised[0] = turn.raised[1] = 0u;
+        turn.sum = 0ull;
+        turn.ok = 1;
+        turn.stop = 0;
     }
-    if (tid < 4) s_sum[tid] = 0ull;
     __syncthreads();
-    for (int i = tid; i < r.nv; i += kSweepBlock) {
-        int b, e;
-        bool own;
-        r.vertex(i, b, e, own);
-        if (e - b > seg) {
-            const int h = atomicAdd(&hb.count, 1);
-            const int nt = (e - b + seg - 1) / seg;
-            const int t0 = atomicAdd(&hb.tasks, nt);
-            hb.hub[h] = i;
-            hb.first[h] = t0;
-            for (int t = 0; t < nt; t++) hb.task[t0 + t] = (unsigned)h | (unsigned)t << 16;
+    /* 1. vertices by kind */
+    for (int i = tid; i < nv; i += kBlock) {
+        const int v = i < nv0 ? cut[0] + i : gap + i;
+        const int deg = (int)(p.rp[v + 1] - p.rp[v]);
+        if (deg <= kLightDeg) {
+            const int own1 = p.owner ? p.owner[v] != 0 : v >= p.n0;
+            atomicAdd(&s_bin[own1 * (kLightDeg + 1) + deg], 1);
+        } else {
+            atomicAdd(&s_heavy[deg > seg], 1);
+            atomicAdd(&s_heavy[2], deg);
         }
     }
     __syncthreads();
-    /* MG and the largest |weight| */
-    SweepCount cnt = {0u, 0u, 0ull};
-    unsigned long long mg_sum = 0;
-    if (r.Es) sweep<GRID, true, MODE_SETUP>(r, hb, nullptr, 0, mg_sum, cnt);
-    else sweep<GRID, false, MODE_SETUP>(r, hb, nullptr, 0, mg_sum, cnt);
-    unsigned wmax = 0;
-    for (int k = tid; k < r.ne; k += kSweepBlock) {
-        const int x = r.Es ? r.Es[k].y : __ldg(r.w + k);
-        wmax = max(wmax, (unsigned)(x < 0 ? -(long long)x : (long long)x));
+    if (tid < 2) {
+        /* Up to how many out-edges a thread walks a vertex: a warp's second
+         * batch of loads (columns 9 to 16) costs another L2 latency, so where
+         * the vertices that need it find a warp each beside the slices, they
+         * get one (games of 4,000 to 6,000 vertices: 215 -> 133 us, 510 -> 425
+         * us; of 16,000, whose CTAs have too many, 143 -> 239 us). */
+        int few[2] = {0, 0}, many = 0, edges = 0;
+        for (int o = 0; o < 2; o++) {
+            for (int d = 0; d <= kLightDeg; d++) {
+                const int x = s_bin[o * (kLightDeg + 1) + d];
+                few[o] += d <= kLightDeg / 2 ? x : 0;
+                many += d > kLightDeg / 2 ? x : 0;
+                edges += d > kLightDeg / 2 ? d * x : 0;
+            }
+        }
+        const bool half = ((few[0] + 31) >> 5) + ((few[1] + 31) >> 5) + s_heavy[0] + many <= kWarps;
+        const int light = half ? kLightDeg / 2 : kLightDeg;
+        __syncwarp(3u);
+        if (half && tid == 0) {
+            s_heavy[0] += many;
+            s_heavy[2] += edges;
+        }
+        if (tid == 0) s_cls[3] = light;
+        /* the first slot of every (owner, out-degree); player 1's start a slice */
+        int total0 = 0;
+        for (int d = 0; d <= light; d++) total0 += s_bin[d];
+        int at = tid ? (total0 + 31) & ~31 : 0;
+        __syncwarp(3u);
+        for (int d = 0; d <= light; d++) {
+            const int k = tid * (kLightDeg + 1) + d, x = s_bin[k];
+            s_bin[k] = at;
+            at += x;
+        }
+        s_cls[tid] = at;
+    }
+    __syncthreads();
+    const int light = s_cls[3];
+    const int nmed = s_heavy[0], nh = nmed + s_heavy[1], he = s_heavy[2];
+    /* 2. shared memory: own values, ids, slice offsets; then sliced edges;
+     * then heavy ones -- what does not fit is in global memory */
+    const int s0 = (s_cls[0] + 31) >> 5, ns = (s_cls[1] + 31) >> 5, nslots = 32 * ns + nh;
+    const int stride = 8 * nslots;
+    const int base = GRID ? cut[0] + cut[2] - split + kPadSlots * (int)blockIdx.x : 0;
+    long long at = 28LL * nslots + 4LL * ns;
+    const bool own_smem = at <= p.smem_bytes;
+    int *vid, *soff;
+    if (own_smem) {
+        vid = (int *)(smem + 3 * stride);
+        soff = vid + nslots;
+        at = (at + 15) & ~15LL;
+    } else {
+        vid = p.vid + base;
+        soff = p.soff + (base >> 5) + 4 * (long long)blockIdx.x;
+        at = 0;
+    }
+    /* slice widths: the out-degree of a slice's last vertex; their sums */
+    {
+        int run = 0;
+        for (int first = 0; first < ns; first += kBlock) {
+            const int s = first + tid;
+            int W = 0;
+            if (s < ns) {
+                const int own1 = s >= s0;
+                const int last = min(32 * s + 31, s_cls[own1] - 1);
+                for (int d = 1; d <= light; d++) W += s_bin[own1 * (kLightDeg + 1) + d] <= last;
+            }
+            int x = W;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (lane == 31) s_scan[warp] = x;
+            __syncthreads();
+            int before = 0, all = 0;
+            for (int k = 0; k < kWarps; k++) {
+                before += k < warp ? s_scan[k] : 0;
+                all += s_scan[k];
+            }
+            if (s < ns) soff[s] = (run + before + x - W) << 5 | W;
+            run += all;
+            __syncthreads();
+        }
+        if (tid == 0) s_cls[2] = run;
+    }
+    for (int i = tid; i < 32 * ns; i += kBlock) vid[i] = -1;
+    if (own_smem)
+        for (int i = tid; i < 2 * nslots; i += kBlock) ((long long *)smem)[i] = 0;
+    if (GRID) {
+        /* up to the next CTA's numbers: 32-bit values lie elsewhere in the arrays */
+        for (int i = tid; i < nv + kPadSlots; i += kBlock) {
+            __stcg((long long *)p.F + base + i, 0LL);
+            __stcg((long long *)p.D + base + i, 0LL);
+        }
+    }
+    __syncthreads();
+    const long long ell = 32LL * s_cls[2]; /* edges with pads */
+    const int at_E = (int)at;
+    const bool edges_smem = at + 8 * ell <= p.smem_bytes;
+    const bool heavy_smem = at + 8 * (ell + nh + he) <= p.smem_bytes;
+    int2 *E, *rest = nullptr; /* where the sliced edges are, and the heavy heads and edges */
+    int2 *out_of_smem = p.E + (e0 + e1 - p.rp[split]) + ((e0 + e1 - p.rp[split]) >> 4) + kPadEdges * (long long)blockIdx.x;
+    E = edges_smem ? (int2 *)(smem + at) : out_of_smem;
+    rest = heavy_smem ? (int2 *)(smem + at) + ell : edges_smem ? out_of_smem : out_of_smem + ell;
+    int2 *head = rest, *H = rest + nh;
+    if (tid < 2) s_heavy[tid] = 0;
+    if (tid == 0) {
+        ps = p;
+        r.ns = ns;
+        r.s0 = s0;
+        r.nh = nh;
+        r.nmed = nmed;
+        r.base = base;
+        r.own_smem = own_smem;
+        r.stride = stride;
+        r.at_vid = 3 * stride;
+        r.at_soff = r.at_vid + 4 * nslots;
+        r.at_E = at_E;
+        r.vid = vid;
+        r.soff = soff;
+        r.E = E;
+        r.head = head;
+        r.H = H;
+        r.g[0] = p.F;
+        r.g[1] = p.D;
+        r.g[2] = p.K;
+        r.rp = p.rp;
+        /* with four sweeps more of them come after the last raise */
+        r.round = GRID ? min(p.sweeps, 2) : 1;
+    }
+    int *number = GRID ? (int *)p.K : (int *)(smem + 2 * stride); /* of every vertex, where K is later */
+    __syncthreads();
+    /* 3. slots */
+    for (int i = tid; i < nv; i += kBlock) {
+        const int v = i < nv0 ? cut[0] + i : gap + i;
+        const int deg = (int)(p.rp[v + 1] - p.rp[v]);
+        const int own1 = p.owner ? p.owner[v] != 0 : v >= p.n0;
+        int slot;
+        if (deg <= light) {
+            slot = atomicAdd(&s_bin[own1 * (kLightDeg + 1) + deg], 1);
+        } else {
+            const int hub = deg > seg;
+            const int h = (hub ? nmed : 0) + atomicAdd(&s_heavy[hub], 1);
+            slot = 32 * ns + h;
+            head[h] = make_int2(atomicAdd(&s_heavy[3], deg), (int)((unsigned)deg | (unsigned)own1 << 31));
+            if (hub) {
+                const int nt = (deg + seg - 1) / seg, t0 = atomicAdd(&hb.tasks, nt), k = h - nmed;
+                hb.first[k] = t0;
+                for (int t = 0; t < nt; t++) hb.task[t0 + t] = (unsigned)k | (unsigned)t << 16;
+            }
+        }
+        vid[slot] = v;
+        if (GRID) __stcg(number + v, base + slot);
+        else number[v] = slot;
+    }
+    __syncthreads();
+    unsigned it = 0;
+    unsigned long long got = 0ull;
+    if (GRID) { /* every vertex has its number */
+        if (tid == 0) turn.ok = round_barrier(p, c, it, 0ull, &got);
+        it++;
+        __syncthreads();
+    }
+    /* 4. edges; MG and the largest |weight| on the way */
+    unsigned long long mg_sum = 0ull;
+    unsigned wmax = 0u;
+    if (turn.ok) {
+        for (int s = warp; s < ns; s += kWarps) {
+            const int v = vid[32 * s + lane], b = soff[s] >> 5, W = soff[s] & 31;
+            long long k0 = 0;
+            int deg = 0, lo = INT32_MAX, hi = INT32_MIN;
+            if (v >= 0) {
+                k0 = p.rp[v];
+                deg = (int)(p.rp[v + 1] - k0);
+            }
+            int2 *out = E + 32 * (long long)b + lane;
+            for (int j0 = 0; j0 < W; j0 += 8) {
+                int2 q[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    q[j] = j0 + j < deg ? make_int2(__ldg(p.succ + k0 + j0 + j), __ldg(p.w + k0 + j0 + j)) : make_int2(-1, 0);
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (j0 + j < deg) q[j].x = GRID ? __ldcg(number + q[j].x) : number[q[j].x];
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    if (j0 + j < deg) {
+                        lo = min(lo, q[j].y);
+                        hi = max(hi, q[j].y);
+                    }
+                    if (j0 + j < W) out[32 * (j0 + j)] = q[j];
+                }
+            }
+            if (deg > 0) {
+                if (lo < 0) mg_sum += (unsigned long long)(-(long long)lo);
+                wmax = max(wmax, max(lo < 0 ? 0u - (unsigned)lo : (unsigned)lo, hi < 0 ? 0u - (unsigned)hi : (unsigned)hi));
+            }
+        }
+        /* the heavy ones a warp each, the cut ones a warp per segment */
+        auto copy = [&](int h, int k0, int k1) {
+            const long long from = p.rp[vid[32 * ns + h]];
+            const int2 hd = head[h];
+            int lo = INT32_MAX, hi = INT32_MIN;
+            for (int k = k0 + lane; k < k1; k += 32) {
+                const int x = __ldg(p.succ + from + k), w = __ldg(p.w + from + k);
+                H[hd.x + k] = make_int2(GRID ? __ldcg(number + x) : number[x], w);
+                lo = min(lo, w);
+                hi = max(hi, w);
+            }
+            lo = __reduce_min_sync(0xffffffffu, lo);
+            hi = __reduce_max_sync(0xffffffffu, hi);
+            wmax = max(wmax, max(lo < 0 ? 0u - (unsigned)lo : (unsigned)lo, hi < 0 ? 0u - (unsigned)hi : (unsigned)hi));
+            return lo;
+        };
+        for (int h = warp; h < nmed; h += kWarps) {
+            const int lo = copy(h, 0, head[h].y & INT32_MAX);
+            if (lane == 0 && lo < 0) mg_sum += (unsigned long long)(-(long long)lo);
+        }
+        for (int t = warp; t < hb.tasks; t += kWarps) {
+            const int h = nmed + (int)(hb.task[t] & 0xffffu), k0 = (int)(hb.task[t] >> 16) * seg;
+            const int lo = copy(h, k0, min(head[h].y & INT32_MAX, k0 + seg));
+            if (lane == 0) hb.part[t] = lo;
+        }
+        __syncthreads();
+        for (int h = nmed + tid; h < nh; h += kBlock) {
+            const int nt = ((head[h].y & INT32_MAX) + seg - 1) / seg;
+            long long lo = 0;
+            for (int t = 0; t < nt; t++) lo = min(lo, hb.part[hb.first[h - nmed] + t]);
+            mg_sum += (unsigned long long)(-lo);
+        }
+        __syncthreads();
     }
     wmax = __reduce_max_sync(0xffffffffu, wmax);
 #pragma unroll
@@ -492,143 +869,75 @@ __global__ void __launch_bounds__(kSweepBlock, 1) k_sweep(const __grid_constant_
         atomicMax(&s_sum[1], (unsigned long long)wmax);
     }
     __syncthreads();
-    if (tid == 0) {
-        atomicAdd(&c->mg, s_sum[0]);
-        atomicMax(&c->wmax, s_sum[1]);
-    }
-    auto first = [&]() {
-        const bool fast32 = c->mg + c->wmax < (unsigned long long)INT32_MAX;
-        c->out_bits = p.bits == 32 || (p.narrow && fast32) ? 32 : 64;
-        if (c->out_bits == 32 && c->mg > (unsigned long long)INT32_MAX) c->stop = (int)EG_ERR_OVERFLOW;
-        c->phase = SWEEP_PRIMAL;
-        c->left = kFirstPrimal;
-        c->primal_len = kSecondPrimal;
-        c->dual_len = kFirstDual;
-    };
-    bool ok = true;
     if (GRID) {
-        ok = grid_barrier(c, p.wait_limit_ns, first);
-    } else {
-        __syncthreads();
-        if (tid == 0) first();
+        if (tid == 0 && turn.ok) {
+            atomicAdd(&c->mg, s_sum[0]);
+            atomicMax(&c->wmax, s_sum[1]);
+            turn.ok = round_barrier(p, c, it, 0ull, &got);
+            s_sum[0] = __ldcg(&c->mg);
+            s_sum[1] = __ldcg(&c->wmax);
+        }
+        it++;
         __syncthreads();
     }
-    const long long mg = (long long)ld_volatile_u64(&c->mg);
-    /* values that gathers read: own arrays of the one CTA, or the global ones */
-    const long long *GF = GRID ? p.F : r.myF, *GD = GRID ? p.D : r.myD, *GK = GRID ? p.K : r.myK;
-    unsigned certified = 0;
-    int phase = SWEEP_PRIMAL;
-    for (unsigned it = 0; ok && !ld_volatile(&c->stop); it++) {
-        const int was = phase;
-        phase = ld_volatile(&c->phase);
-        if (phase == SWEEP_DONE || phase == SWEEP_HANDOVER) break;
-        const int left = ld_volatile(&c->left);
-        const unsigned raised0 = cnt.raised;
-        int ran;
-        if (phase == SWEEP_PRIMAL) {
-            if (was == SWEEP_KILL) {
-                /* the certified vertices: TOP */
-                for (int i = tid; i < r.nv; i += kSweepBlock) {
-                    const long long k = r.myK[i];
-                    if (k < kTop && k != kLow) {
-                        r.myF[i] = kTop;
-                        r.myD[i] = kLow;
-                        if (GRID) {
-                            __stcg(r.gF + i, kTop);
-                            __stcg(r.gD + i, kLow);
-                        }
-                        cnt.raised++;
-                        certified++;
-                    }
-                }
-                __syncthreads();
-            }
-            ran = GRID ? min(p.sweeps, left) : 1;
-            for (int s = 0; s < ran; s++) {
-                if (r.Es) sweep<GRID, true, MODE_PRIMAL>(r, hb, GF, mg, mg_sum, cnt);
-                else sweep<GRID, false, MODE_PRIMAL>(r, hb, GF, mg, mg_sum, cnt);
-            }
-        } else if (phase == SWEEP_DUAL) {
-            ran = left;
-            for (int s = 0; s < ran; s++) {
-                if (r.Es) sweep<GRID, true, MODE_DUAL>(r, hb, GD, mg, mg_sum, cnt);
-                else sweep<GRID, false, MODE_DUAL>(r, hb, GD, mg, mg_sum, cnt);
-            }
-            __syncthreads();
-            for (int i = tid; i < r.nv; i += kSweepBlock) {
-                const long long d = r.myD[i];
-                r.myK[i] = d;
-                if (GRID) __stcg(r.gK + i, d);
-            }
-        } else {
-            ran = GRID ? kKillSweeps : 1;
-            for (int s = 0; s < ran; s++) {
-                if (r.Es) sweep<GRID, true, MODE_KILL>(r, hb, GK, mg, mg_sum, cnt);
-                else sweep<GRID, false, MODE_KILL>(r, hb, GK, mg, mg_sum, cnt);
-            }
-        }
-        const unsigned d = __reduce_add_sync(0xffffffffu, cnt.raised - raised0);
-        if (GRID) {
-            if (tid == 0) s_sum[2] = 0ull;
-            __syncthreads();
-            if (lane == 0 && d) atomicAdd(&s_sum[2], (unsigned long long)d);
-            __syncthreads();
-            if (tid == 0 && s_sum[2]) atomicAdd(&c->raised[it & 1], s_sum[2]);
-            ok = grid_barrier(c, p.wait_limit_ns, [&]() {
-                const unsigned long long raised = c->raised[it & 1];
-                c->raised[(it + 1) & 1] = 0ull;
-                advance(p, c, ran, raised);
-            });
-        } else {
-            if (lane == 0 && d) atomicAdd(&c->raised[it & 1], (unsigned long long)d);
-            __syncthreads();
-            if (tid == 0) {
-                const unsigned long long raised = c->raised[it & 1];
-                c->raised[(it + 1) & 1] = 0ull;
-                advance(p, c, ran, raised);
-            }
-            __syncthreads();
-        }
-    }
+    /* 5. the width of the credits, here and in the result */
+    const unsigned long long mg = s_sum[0], big = s_sum[1];
+    const int out_bits = p.bits == 32 || (p.narrow && mg + big < (unsigned long long)INT32_MAX) ? 32 : 64;
+    const bool fits32 = mg + big < (unsigned long long)Lim<int>::top && big <= (unsigned long long)Lim<int>::weight_max;
+    SweepState st;
+    st.phase = SWEEP_PRIMAL;
+    st.left = kFirstPrimal;
+    st.primal_len = kSecondPrimal;
+    st.dual_len = kFirstDual;
+    st.stop = out_bits == 32 && mg > (unsigned long long)INT32_MAX ? (int)EG_ERR_OVERFLOW : 0;
+    st.rounds = st.sweeps = 0;
     __syncthreads();
-    /* credits out */
-    const int out_bits = ld_volatile(&c->out_bits);
-    unsigned tops = 0;
-    for (int i = tid; i < r.nv; i += kSweepBlock) {
-        const long long f = r.myF[i];
-        tops += f == kTop;
-        if (out_bits == 32) ((int *)p.out)[r.va + i] = f == kTop ? INT32_MAX : (int)f;
-        else ((long long *)p.out)[r.va + i] = f == kTop ? (long long)INT64_MAX : f;
-    }
-    tops = __reduce_add_sync(0xffffffffu, tops);
-    certified = __reduce_add_sync(0xffffffffu, certified);
-    const unsigned lifts = __reduce_add_sync(0xffffffffu, cnt.lifts);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cnt.edges += __shfl_xor_sync(0xffffffffu, cnt.edges, o);
     if (tid < 4) s_sum[tid] = 0ull;
+    if (tid == 0) {
+        if (!GRID) {
+            c->mg = mg;
+            c->wmax = big;
+        }
+        /* potentials count weights 2^nshift-fold: more than n times where
+         * that fits */
+        const unsigned long long limit =
+            fits32 ? (unsigned long long)Lim<int>::weight_max : (unsigned long long)Lim<long long>::weight_max;
+        int nshift = 0;
+        while (nshift < 20 && (1ll << nshift) <= p.n && (big << (nshift + 1)) <= limit) nshift++;
+        r.out_bits = out_bits;
+        r.mg = (long long)mg;
+        r.scale = 1ll << nshift;
+    }
+    Count cnt = {0u, 0u, 0ull, 0ull, 0ull};
     __syncthreads();
-    if (lane == 0) {
-        atomicAdd(&s_sum[0], (unsigned long long)tops);
-        atomicAdd(&s_sum[1], (unsigned long long)certified);
-        atomicAdd(&s_sum[2], (unsigned long long)lifts);
-        atomicAdd(&s_sum[3], cnt.edges);
+    if (!GRID) {
+        if (fits32) solve<int, KIND_CTA>(&ps, r, hb, turn, st, it, cnt);
+        else solve<long long, KIND_CTA>(&ps, r, hb, turn, st, it, cnt);
+    } else if (own_smem && edges_smem) {
+        if (fits32) solve<int, KIND_STAGED>(&ps, r, hb, turn, st, it, cnt);
+        else solve<long long, KIND_STAGED>(&ps, r, hb, turn, st, it, cnt);
+    } else {
+        if (fits32) solve<int, KIND_GLOBAL>(&ps, r, hb, turn, st, it, cnt);
+        else solve<long long, KIND_GLOBAL>(&ps, r, hb, turn, st, it, cnt);
+    }
+    unsigned long long sums[4] = {cnt.raised, cnt.lifts, cnt.edges, cnt.changes};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sums[k] += __shfl_xor_sync(0xffffffffu, sums[k], o);
+        if (lane == 0) atomicAdd(&s_sum[k], sums[k]);
     }
     __syncthreads();
     if (tid == 0) {
         atomicAdd(&c->num_top, s_sum[0]);
-        atomicAdd(&c->certified, s_sum[1]);
-        atomicAdd(&c->lifts, s_sum[2]);
-        atomicAdd(&c->edges, s_sum[3]);
+        atomicAdd(&c->lifts, s_sum[1]);
+        atomicAdd(&c->edges, s_sum[2]);
+        atomicAdd(&c->changes, s_sum[3]);
+        if (blockIdx.x == 0) {
+            c->s = st;
+            c->out_bits = out_bits;
+        }
     }
-    if (!GRID) {
-        __syncthreads();
-        for (int i = tid; i < (int)(sizeof(SweepCtrl) / 4); i += kSweepBlock) ((int *)p.ctrl)[i] = ((int *)&s_ctrl)[i];
-    }
-}
-
-long long sweep_cta_bytes(long long n, long long m)
-{
-    return ((n * kVertexBytes + 4 + 15) & ~15LL) + 8 * m;
 }
 
 /* Dynamic shared memory a CTA of the kernel may have. */
@@ -640,36 +949,53 @@ static eg_status sweep_smem(const void *fn, int dev, int *bytes)
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fn);
     if (e != cudaSuccess) return eg_set_error(EG_ERR_CUDA, "sweep kernel attributes: %s", cudaGetErrorString(e));
     *bytes = optin - (int)fa.sharedSizeBytes;
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, *bytes);
+    if (e != cudaSuccess) return eg_set_error(EG_ERR_CUDA, "sweep kernel attributes: %s", cudaGetErrorString(e));
     return EG_OK;
 }
 
-eg_status launch_sweep(SweepParams p, cudaStream_t st, int max_ctas, int *grid, int *block)
+eg_status sweep_plan(int n, long long m, int max_ctas, SweepPlan *plan)
 {
-    const void *one = (const void *)k_sweep<false>, *all = (const void *)k_sweep<true>;
     int dev = 0, sms = 0, bytes = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return eg_set_error(EG_ERR_CUDA, "sweep kernel set-up: %s", cudaGetErrorString(e));
-    *block = kSweepBlock;
-    const long long need = sweep_cta_bytes(p.n, p.m);
-    eg_status s = sweep_smem(one, dev, &bytes);
+    const long long total = 8 * m + m / 2 + (long long)kVertexBytes * n;
+    memset(plan, 0, sizeof *plan);
+    plan->block = kBlock;
+    eg_status s = sweep_smem((const void *)k_sweep<false>, dev, &bytes);
     if (s != EG_OK) return s;
-    if (need <= bytes) {
-        *grid = 1;
-        p.smem_bytes = (int)need;
-        e = cudaFuncSetAttribute(one, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        void *args[] = {(void *)&p};
-        if (e == cudaSuccess) e = cudaLaunchKernel(one, dim3(1), dim3(kSweepBlock), args, (size_t)need, st);
-    } else {
-        s = sweep_smem(all, dev, &bytes);
-        if (s != EG_OK) return s;
-        *grid = max_ctas > 0 && max_ctas < sms ? max_ctas : sms;
-        p.smem_bytes = bytes;
-        e = cudaFuncSetAttribute(all, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        void *args[] = {(void *)&p};
-        if (e == cudaSuccess)
-            e = cudaLaunchCooperativeKernel(all, dim3(*grid), dim3(kSweepBlock), args, (size_t)bytes, st);
+    plan->grid = 1;
+    if (total + kSlackBytes <= bytes) {
+        plan->one_cta = 1;
+        plan->smem_bytes = (int)(total + kSlackBytes);
+        return EG_OK;
     }
+    s = sweep_smem((const void *)k_sweep<true>, dev, &bytes);
+    if (s != EG_OK) return s;
+    plan->grid = max_ctas > 0 && max_ctas < sms ? max_ctas : sms;
+    plan->smem_bytes = bytes;
+    plan->values = (size_t)n + (size_t)kPadSlots * plan->grid;
+    /* a part that ends with a vertex of many edges may not fit shared memory
+     * even where the mean part does */
+    plan->edges = (size_t)(m + m / 16) + (size_t)kPadEdges * plan->grid;
+    if (total / plan->grid + kSlackBytes > bytes) {
+        plan->vids = plan->values;
+        plan->offs = plan->values / 32 + 4 * (size_t)plan->grid + 4;
+    }
+    return EG_OK;
+}
+
+eg_status launch_sweep(SweepParams p, const SweepPlan &plan, cudaStream_t st)
+{
+    p.smem_bytes = plan.smem_bytes;
+    void *args[] = {(void *)&p};
+    cudaError_t e;
+    if (plan.one_cta)
+        e = cudaLaunchKernel((const void *)k_sweep<false>, dim3(1), dim3(kBlock), args, (size_t)plan.smem_bytes, st);
+    else
+        e = cudaLaunchCooperativeKernel((const void *)k_sweep<true>, dim3(plan.grid), dim3(kBlock), args,
+                                        (size_t)plan.smem_bytes, st);
     if (e != cudaSuccess) return eg_set_error(EG_ERR_CUDA, "launch of the sweep kernel failed: %s", cudaGetErrorString(e));
     return EG_OK;
 }

@@ -12,24 +12,26 @@ namespace eg {
 /* Phases of a sweep solve, as SweepCtrl::phase holds them between rounds. */
 enum { SWEEP_PRIMAL = 0, SWEEP_DUAL = 1, SWEEP_KILL = 2, SWEEP_DONE = 3, SWEEP_HANDOVER = 4 };
 
-struct SweepCtrl {
-    /* grid_barrier's fields */
-    unsigned bar_count, bar_gen;
-    int stop, abort;
+/* The schedule, held by every thread and advanced by each in the same way
+ * after every round. */
+struct SweepState {
+    int phase;
+    int left;                            /* sweeps left in this phase          */
+    int primal_len, dual_len;            /* sweeps of the next phases          */
+    int stop;                            /* 0 running; else an eg_status       */
     long long rounds;                    /* primal rounds completed            */
+    long long sweeps;                    /* primal sweeps run                  */
+};
+
+struct SweepCtrl {
+    SweepState s;                        /* as the solve ended                 */
+    unsigned long long word[4][16];      /* round barriers: arrivals << 48 | flags | raises */
+    int abort;                           /* a CTA gave up waiting              */
+    int out_bits;                        /* width of the credits in `out`      */
     unsigned long long wait_site;
     unsigned long long t_start;
-    /* the schedule, advanced by each round's last arriver */
-    int phase;
-    int left;                            /* primal sweeps left in this phase   */
-    int primal_len, dual_len;            /* sweeps of the next phases          */
-    long long sweeps, dual_sweeps, kill_sweeps; /* run so far                  */
-    int attempts;                        /* certificates tried                 */
-    int out_bits;                        /* width of the credits in `out`      */
-    unsigned long long raised[2];        /* raises of a round, by parity       */
-    /* of the game and of the solve */
     unsigned long long mg, wmax;
-    unsigned long long lifts, edges, changes, certified, num_top;
+    unsigned long long lifts, edges, changes, num_top;
 };
 
 struct SweepParams {
@@ -38,15 +40,15 @@ struct SweepParams {
     const unsigned char *owner;          /* or null: vertex >= n0 is player 1  */
     int n, n0;
     long long m;
-    long long *F, *D, *K;                /* grid kernel: credits, potentials   */
+    void *F, *D, *K;                     /* grid kernel: credits, potentials, their copy (plan.values of 8 B each) */
+    int2 *E;                             /* where a CTA's values or edges do not fit its shared memory: */
+    int *vid, *soff;                     /* sliced edges, vertices and slice offsets; else null */
     void *out;                           /* credits, int32 or int64            */
     SweepCtrl *ctrl;
     long long max_rounds;                /* < 0: no cap                        */
     unsigned long long timeout_ns, wait_limit_ns;
     const int *cancel;
-    int lanes;                           /* lanes per vertex: 1 .. 32          */
-    int sweeps;                          /* primal sweeps between two barriers */
-    int nshift;                          /* potentials count weights 2^nshift-fold */
+    int sweeps;                          /* most sweeps between two barriers   */
     int bits;                            /* 32, 64: width asked for            */
     int narrow;                          /* 64: may come out in 32 bits        */
     int smem_bytes;                      /* dynamic shared memory              */
@@ -54,11 +56,16 @@ struct SweepParams {
     long long hand_raised;               /* "few": raises per round            */
 };
 
-/* Bytes of dynamic shared memory with which the one-CTA kernel holds a game. */
-long long sweep_cta_bytes(long long n, long long m);
+/* Which kernel a game takes and what global scratch it needs. */
+struct SweepPlan {
+    int one_cta, grid, block, smem_bytes;
+    size_t values;                       /* entries of F, D and K              */
+    size_t edges, vids, offs;            /* entries of E, vid and soff         */
+};
+eg_status sweep_plan(int n, long long m, int max_ctas, SweepPlan *plan);
 /* Launches the one-CTA kernel (game in shared memory) or the persistent
- * grid kernel on `st`; *grid gets the CTAs. */
-eg_status launch_sweep(SweepParams p, cudaStream_t st, int max_ctas, int *grid, int *block);
+ * grid kernel on `st`. */
+eg_status launch_sweep(SweepParams p, const SweepPlan &plan, cudaStream_t st);
 
 }  // namespace eg
 
