@@ -10,6 +10,7 @@
  * at once and no global state is shared between solves.
  */
 #include "eg_lift.cuh"
+#include "eg_pool.cuh"
 #include "eg_prep.cuh"
 #include "eg_sweep.cuh"
 
@@ -55,6 +56,8 @@ constexpr int kSmallGameMaxPad = 1 << 19;
  * a frontier round */
 constexpr long long kHandEdges = 1 << 22;
 constexpr long long kHandSweeps = 2048;
+constexpr size_t kEarlyAt = 2048; /* credits behind the control block in a lane's pinned memory */
+static_assert(sizeof(SweepCtrl) <= kEarlyAt, "");
 
 inline unsigned grid_for(long long items, int block, int cap = 148 * 32)
 {
@@ -70,7 +73,8 @@ inline int align32(long long x) { return (int)((x + 31) & ~31LL); }
 
 struct eg_dgame {
     int device;
-    cudaStream_t st;
+    Lane *lane;
+    cudaStream_t st;   /* the lane's, as the events */
     cudaEvent_t ev[6]; /* solve start, lift start, lift end, solve end; dense launch start / end */
     int n, n0;
     long long m;
@@ -251,11 +255,9 @@ struct Arena {
     eg_status get(eg_dgame *g, void **block)
     {
         char *base = nullptr;
-        cudaError_t e = cudaMalloc((void **)&base, total);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            return eg_set_error(EG_ERR_OOM, "cudaMalloc of %zu bytes failed: %s", total, cudaGetErrorString(e));
-        }
+        cudaError_t e = pool_alloc((void **)&base, total, g->device, g->st);
+        if (e != cudaSuccess)
+            return eg_set_error(EG_ERR_OOM, "device allocation of %zu bytes failed: %s", total, cudaGetErrorString(e));
         *block = base;
         for (const Part &x : parts) *x.p = base + x.at;
         g->bytes += total;
@@ -269,13 +271,12 @@ extern "C" void eg_dgame_free(eg_dgame *g)
     int prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(g->device);
-    if (g->st) cudaStreamSynchronize(g->st);
-    if (g->block) cudaFree(g->block);
-    if (g->rounds_block) cudaFree(g->rounds_block);
-    if (g->sweep_block) cudaFree(g->sweep_block);
-    for (int i = 0; i < 6; i++)
-        if (g->ev[i]) cudaEventDestroy(g->ev[i]);
-    if (g->st) cudaStreamDestroy(g->st);
+    if (g->lane) {
+        pool_free(g->block, g->st);
+        pool_free(g->rounds_block, g->st);
+        pool_free(g->sweep_block, g->st);
+        lane_give(g->lane);
+    }
     cudaSetDevice(prev);
     free(g);
 }
@@ -335,10 +336,13 @@ static eg_status dgame_alloc(const eg_game *game, const eg_opts *opts, eg_dgame 
     g->tmp_cap = std::max<long long>(g->m, g->n) + 1;
     g->scratch_ints = radix_scratch_ints(g->tmp_cap) + scan_scratch_ints(g->n_pad_cap + 1) + 64;
     eg_status s = EG_OK;
-    cudaError_t e = cudaStreamCreateWithFlags(&g->st, cudaStreamNonBlocking);
-    if (e != cudaSuccess) s = eg_set_error(EG_ERR_CUDA, "cudaStreamCreate failed: %s", cudaGetErrorString(e));
-    for (int i = 0; i < 6 && s == EG_OK; i++)
-        if (cudaEventCreate(&g->ev[i]) != cudaSuccess) s = eg_set_error(EG_ERR_CUDA, "cudaEventCreate failed");
+    g->lane = lane_take(dev);
+    if (g->lane) {
+        g->st = g->lane->st;
+        memcpy(g->ev, g->lane->ev, sizeof g->ev);
+    } else {
+        s = eg_set_error(EG_ERR_CUDA, "creation of a stream and its events failed");
+    }
     Arena ar;
     ar.add(&g->d_rowptr, (size_t)g->n + 1);
     ar.add(&g->d_succ, (size_t)g->m);
@@ -369,7 +373,7 @@ static eg_status sweep_reserve(eg_dgame *g, const eg_opts *opts, SweepPlan *plan
     const SweepPlan &have = g->sweep_have;
     if (plan->values <= have.values && plan->edges <= have.edges && plan->vids <= have.vids && plan->offs <= have.offs)
         return EG_OK;
-    if (g->sweep_block) cudaFree(g->sweep_block);
+    pool_free(g->sweep_block, g->st);
     g->sweep_block = nullptr;
     g->bytes -= g->sweep_bytes;
     g->sweep_bytes = 0;
@@ -427,15 +431,20 @@ extern "C" eg_status eg_dgame_upload(const eg_game *game, const eg_opts *opts, e
     EG_TRY(check_lanes(opts));
     eg_dgame *g = nullptr;
     EG_TRY(dgame_alloc(game, opts, &g));
-    cudaError_t e = cudaMemcpyAsync(g->d_rowptr, game->row_ptr, sizeof(long long) * ((size_t)g->n + 1),
-                                    cudaMemcpyHostToDevice, g->st);
-    if (e == cudaSuccess && g->m)
-        e = cudaMemcpyAsync(g->d_succ, game->succ, sizeof(int) * (size_t)g->m, cudaMemcpyHostToDevice, g->st);
-    if (e == cudaSuccess && g->m)
-        e = cudaMemcpyAsync(g->d_w, game->weight, sizeof(int) * (size_t)g->m, cudaMemcpyHostToDevice, g->st);
-    if (e == cudaSuccess && g->has_owner)
-        e = cudaMemcpyAsync(g->d_owner, game->owner, (size_t)g->n, cudaMemcpyHostToDevice, g->st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(g->st);
+    const char *block = (const char *)g->block;
+    CopyPart parts[4];
+    int np = 0;
+    size_t end = 0;
+    auto part = [&](const void *dst, const void *src, size_t bytes) {
+        if (!bytes) return;
+        parts[np++] = {src, (size_t)((const char *)dst - block), bytes};
+        end = std::max(end, parts[np - 1].at + bytes);
+    };
+    part(g->d_rowptr, game->row_ptr, sizeof(long long) * ((size_t)g->n + 1));
+    part(g->d_succ, game->succ, sizeof(int) * (size_t)g->m);
+    part(g->d_w, game->weight, sizeof(int) * (size_t)g->m);
+    if (g->has_owner) part(g->d_owner, game->owner, (size_t)g->n);
+    const cudaError_t e = copy_parts_to_device(g->block, parts, np, end, g->device, g->st);
     if (e != cudaSuccess) {
         eg_status s = eg_set_error(EG_ERR_CUDA, "upload failed: %s", cudaGetErrorString(e));
         eg_dgame_free(g);
@@ -840,8 +849,10 @@ static eg_status dgame_rounds(eg_dgame *g, const eg_opts *opts, const SweepCtrl 
 
 /* The solve by sweeps with certificates (eg_sweep.cu); a large game whose
  * credits still rise in a few places after kHandSweeps sweeps goes on with
- * frontier and dense rounds. */
-static eg_status dgame_sweeps(eg_dgame *g, const eg_opts *opts, eg_stats *stats)
+ * frontier and dense rounds.  With `early` (a one-call solve) small results
+ * come along with the control block, and *early says whether they did: they
+ * are in the lane's pinned memory behind it. */
+static eg_status dgame_sweeps(eg_dgame *g, const eg_opts *opts, eg_stats *stats, bool *early)
 {
     cudaStream_t st = g->st;
     SweepParams p;
@@ -884,15 +895,20 @@ static eg_status dgame_sweeps(eg_dgame *g, const eg_opts *opts, eg_stats *stats)
     EG_TRY(launch_sweep(p, plan, st));
     g->launches++;
     EG_CUDA(cudaEventRecord(g->ev[3], st));
-    SweepCtrl c;
-    EG_CUDA(cudaMemcpyAsync(&c, g->d_sctrl, sizeof c, cudaMemcpyDeviceToHost, st));
+    EG_CUDA(cudaMemcpyAsync(g->lane->page, g->d_sctrl, sizeof(SweepCtrl), cudaMemcpyDeviceToHost, st));
+    const size_t out_bytes = (size_t)g->n * (size_t)(p.bits / 8);
+    const bool along = early && !p.narrow && kEarlyAt + out_bytes <= kLanePage;
+    if (along)
+        EG_CUDA(cudaMemcpyAsync((char *)g->lane->page + kEarlyAt, g->d_out, out_bytes, cudaMemcpyDeviceToHost, st));
     EG_CUDA(cudaStreamSynchronize(st));
+    const SweepCtrl &c = *(const SweepCtrl *)g->lane->page;
     g->mg = (long long)c.mg;
     g->wmax = (long long)c.wmax;
     const int stop = c.abort ? (int)EG_ERR_TIMEOUT : c.s.stop;
     if (stop == EG_ERR_OVERFLOW)
         return eg_set_error(EG_ERR_OVERFLOW, "MG = %lld does not fit 32-bit credits", g->mg);
     if (c.s.phase == SWEEP_HANDOVER && !stop) return dgame_rounds(g, opts, &c, stats);
+    if (early) *early = along;
     g->solved_bits = c.out_bits;
     g->solved = true;
     g->swept = true;
@@ -915,7 +931,7 @@ static eg_status dgame_sweeps(eg_dgame *g, const eg_opts *opts, eg_stats *stats)
     return stop_status(stop, c.abort, c.wait_site, opts);
 }
 
-extern "C" eg_status eg_dgame_solve(eg_dgame *g, const eg_opts *opts_in, eg_stats *stats)
+static eg_status dgame_solve(eg_dgame *g, const eg_opts *opts_in, eg_stats *stats, bool *early)
 {
     if (!g) return eg_set_error(EG_ERR_INVALID, "game handle is NULL");
     eg_opts dflt;
@@ -925,7 +941,12 @@ extern "C" eg_status eg_dgame_solve(eg_dgame *g, const eg_opts *opts_in, eg_stat
     EG_CUDA(cudaSetDevice(g->device));
     g->launches = 0;
     g->solved = false;
-    return routes_to_sweeps(opts) ? dgame_sweeps(g, opts, stats) : dgame_rounds(g, opts, nullptr, stats);
+    return routes_to_sweeps(opts) ? dgame_sweeps(g, opts, stats, early) : dgame_rounds(g, opts, nullptr, stats);
+}
+
+extern "C" eg_status eg_dgame_solve(eg_dgame *g, const eg_opts *opts, eg_stats *stats)
+{
+    return dgame_solve(g, opts, stats, nullptr);
 }
 
 template <class O>
@@ -943,8 +964,7 @@ static eg_status dgame_credits(eg_dgame *g, O *host, int obits)
         launch_gather_out(g->solved_bits, obits, g->n, nullptr, g->d_out, g->d_conv, g->st);
         src = g->d_conv;
     }
-    EG_CUDA(cudaMemcpyAsync(host, src, sizeof(O) * (size_t)g->n, cudaMemcpyDeviceToHost, g->st));
-    EG_CUDA(cudaStreamSynchronize(g->st));
+    EG_CUDA(copy_to_host(host, src, sizeof(O) * (size_t)g->n, g->device, g->st));
     return EG_OK;
 }
 
@@ -978,8 +998,11 @@ static eg_status solve_once(const eg_game *game, const eg_opts *opts, O *credits
     if (obits == 32 && o.credit_bits == 64) o.credit_bits = 64; /* solve wide, narrow on output */
     eg_dgame *g = nullptr;
     EG_TRY(eg_dgame_upload(game, &o, &g));
-    eg_status s = eg_dgame_solve(g, &o, stats);
-    if (s == EG_OK || s == EG_ERR_LOOPCAP || s == EG_ERR_TIMEOUT || s == EG_ERR_CANCELLED) {
+    bool early = false;
+    eg_status s = dgame_solve(g, &o, stats, &early);
+    if (early && g->solved_bits == obits) {
+        memcpy(credits, (const char *)g->lane->page + kEarlyAt, sizeof(O) * (size_t)g->n);
+    } else if (s == EG_OK || s == EG_ERR_LOOPCAP || s == EG_ERR_TIMEOUT || s == EG_ERR_CANCELLED) {
         char msg[512];
         snprintf(msg, sizeof msg, "%s", eg_last_error());
         eg_status s2 = dgame_credits<O>(g, credits, obits);
@@ -1014,63 +1037,71 @@ extern "C" eg_status eg_csr2csc_i32(int32_t num_rows, int32_t num_cols, int64_t 
         return eg_set_error(EG_ERR_INVALID, "NULL array");
     if (row_ptr[0] != 0 || row_ptr[num_rows] != nnz)
         return eg_set_error(EG_ERR_INVALID, "row_ptr must start at 0 and end at nnz");
-    for (int32_t r = 0; r < num_rows; r++)
-        if (row_ptr[r + 1] < row_ptr[r]) return eg_set_error(EG_ERR_INVALID, "row_ptr not monotone at row %d", r);
-    for (int64_t j = 0; j < nnz; j++)
-        if (col_idx[j] < 0 || col_idx[j] >= num_cols)
-            return eg_set_error(EG_ERR_INVALID, "column %d of entry %lld out of range", col_idx[j], (long long)j);
     int count = 0;
     if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0) {
         cudaGetLastError();
+        EG_TRY(eg_check_csr(num_rows, num_cols, nnz, row_ptr, col_idx));
         return eg_set_error(EG_ERR_NO_DEVICE, "no CUDA device available");
     }
-    cudaStream_t st;
-    EG_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    int dev = 0;
+    EG_CUDA(cudaGetDevice(&dev));
+    Lane *lane = lane_take(dev);
+    if (!lane) return eg_set_error(EG_ERR_CUDA, "creation of a stream and its events failed");
+    cudaStream_t st = lane->st;
     const long long cap = std::max<long long>(nnz, 1);
     long long *d_rp = nullptr, *d_cp64 = nullptr;
     int *d_col = nullptr, *d_val = nullptr, *d_k0 = nullptr, *d_v0 = nullptr, *d_k1 = nullptr, *d_v1 = nullptr;
     int *d_rows = nullptr, *d_cnt = nullptr, *d_orow = nullptr, *d_oval = nullptr, *d_scr = nullptr;
     const long long scr = radix_scratch_ints(cap) + scan_scratch_ints((long long)num_cols + 1) + 64;
-    cudaError_t e = cudaSuccess;
-#define EG_MALLOC(p, n) \
-    if (e == cudaSuccess) e = cudaMalloc((void **)&p, sizeof(*p) * (size_t)(n))
-    EG_MALLOC(d_rp, (long long)num_rows + 1);
-    EG_MALLOC(d_col, cap);
-    EG_MALLOC(d_val, cap);
-    EG_MALLOC(d_k0, cap);
-    EG_MALLOC(d_v0, cap);
-    EG_MALLOC(d_k1, cap);
-    EG_MALLOC(d_v1, cap);
-    EG_MALLOC(d_rows, cap);
-    EG_MALLOC(d_orow, cap);
-    EG_MALLOC(d_oval, cap);
-    EG_MALLOC(d_cnt, (long long)num_cols + 1);
-    EG_MALLOC(d_cp64, (long long)num_cols + 1);
-    EG_MALLOC(d_scr, scr);
-#undef EG_MALLOC
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_rp, row_ptr, sizeof(long long) * ((size_t)num_rows + 1), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && nnz) e = cudaMemcpyAsync(d_col, col_idx, sizeof(int) * (size_t)nnz, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && nnz) e = cudaMemcpyAsync(d_val, val, sizeof(int) * (size_t)nnz, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_cnt, 0, sizeof(int) * ((size_t)num_cols + 1), st);
+    Arena ar;
+    ar.add(&d_rp, (size_t)num_rows + 1);
+    ar.add(&d_col, (size_t)cap);
+    ar.add(&d_val, (size_t)cap);
+    const size_t inputs = ar.total;
+    ar.add(&d_k0, (size_t)cap);
+    ar.add(&d_v0, (size_t)cap);
+    ar.add(&d_k1, (size_t)cap);
+    ar.add(&d_v1, (size_t)cap);
+    ar.add(&d_rows, (size_t)cap);
+    ar.add(&d_orow, (size_t)cap);
+    ar.add(&d_oval, (size_t)cap);
+    ar.add(&d_cnt, (size_t)num_cols + 2); /* columns' counts; then the check's flag */
+    ar.add(&d_cp64, (size_t)num_cols + 1);
+    ar.add(&d_scr, (size_t)scr);
+    char *block = nullptr;
+    cudaError_t e = pool_alloc((void **)&block, ar.total, dev, st);
     if (e == cudaSuccess) {
+        for (const Arena::Part &x : ar.parts) *x.p = block + x.at;
+        const CopyPart parts[3] = {{row_ptr, 0, sizeof(long long) * ((size_t)num_rows + 1)},
+                                   {col_idx, (size_t)((char *)d_col - block), sizeof(int) * (size_t)nnz},
+                                   {val, (size_t)((char *)d_val - block), sizeof(int) * (size_t)nnz}};
+        e = copy_parts_to_device(block, parts, nnz ? 3 : 1, inputs, dev, st);
+    }
+    int *d_bad = d_cnt + num_cols + 1, *h_bad = (int *)lane->page;
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_cnt, 0, sizeof(int) * ((size_t)num_cols + 2), st);
+    if (e == cudaSuccess) {
+        k_check_csr<<<grid_for(std::max<long long>(nnz, num_rows), 256), 256, 0, st>>>(num_rows, num_cols, nnz, d_rp, d_col,
+                                                                                    d_bad);
         const unsigned gw = grid_for((long long)num_rows * 32, 256);
-        k_csr_expand<<<gw, 256, 0, st>>>(num_rows, d_rp, d_col, d_k0, d_v0, d_cnt);
-        k_edge_rows<<<gw, 256, 0, st>>>(num_rows, d_rp, d_rows);
+        k_csr_expand<<<gw, 256, 0, st>>>(num_rows, d_rp, d_col, d_bad, d_k0, d_v0, d_rows, d_cnt);
         excl_scan(d_cnt, (long long)num_cols + 1, d_scr, st);
         int *sk, *sv;
         radix_sort_pairs(d_k0, d_v0, d_k1, d_v1, nnz, bits_for(num_cols), d_scr, st, &sk, &sv);
-        k_csc_gather<<<grid_for(nnz, 256), 256, 0, st>>>(nnz, sv, d_rows, d_val, d_orow, d_oval);
+        k_csc_gather<<<grid_for(nnz, 256), 256, 0, st>>>(nnz, d_bad, sv, d_rows, d_val, d_orow, d_oval);
         k_widen<<<grid_for((long long)num_cols + 1, 256), 256, 0, st>>>((long long)num_cols + 1, d_cnt, d_cp64);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(csc_ptr, d_cp64, sizeof(long long) * ((size_t)num_cols + 1), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && nnz) e = cudaMemcpyAsync(csc_row, d_orow, sizeof(int) * (size_t)nnz, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && nnz) e = cudaMemcpyAsync(csc_val, d_oval, sizeof(int) * (size_t)nnz, cudaMemcpyDeviceToHost, st);
+    const CopyItem outs[3] = {{csc_ptr, d_cp64, sizeof(long long) * ((size_t)num_cols + 1)},
+                              {csc_row, d_orow, sizeof(int) * (size_t)nnz},
+                              {csc_val, d_oval, sizeof(int) * (size_t)nnz}};
+    bool bad = false;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h_bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    void *ptrs[] = {d_rp, d_cp64, d_col, d_val, d_k0, d_v0, d_k1, d_v1, d_rows, d_cnt, d_orow, d_oval, d_scr};
-    for (void *ptr : ptrs)
-        if (ptr) cudaFree(ptr);
-    cudaStreamDestroy(st);
+    if (e == cudaSuccess) bad = *h_bad != 0;
+    if (e == cudaSuccess && !bad) e = copy_list(outs, 3, true, dev, st);
+    pool_free(block, st);
+    lane_give(lane);
+    if (bad) return eg_check_csr(num_rows, num_cols, nnz, row_ptr, col_idx); /* says what is wrong */
     if (e != cudaSuccess) {
         cudaGetLastError();
         return eg_set_error(e == cudaErrorMemoryAllocation ? EG_ERR_OOM : EG_ERR_CUDA, "transpose failed: %s",
@@ -1138,7 +1169,7 @@ extern "C" eg_status eg_dgame_tune(eg_dgame *g, const eg_opts *base_in, int64_t 
     if (base.variant != EG_VARIANT_AUTO) return eg_set_error(EG_ERR_INVALID, "the tuner tunes the AUTO layout");
     EG_CUDA(cudaSetDevice(g->device));
     std::vector<long long> rp((size_t)g->n + 1);
-    EG_CUDA(cudaMemcpy(rp.data(), g->d_rowptr, sizeof(long long) * rp.size(), cudaMemcpyDeviceToHost));
+    EG_CUDA(copy_to_host(rp.data(), g->d_rowptr, sizeof(long long) * rp.size(), g->device, g->st));
     const std::string key = shape_key(rp, g->n, g->m) + "|" + std::to_string(base.credit_bits) + "|" +
                             std::to_string(base.narrow);
     eg_tune_report r;

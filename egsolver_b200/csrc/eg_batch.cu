@@ -33,6 +33,7 @@
  * from an atomic counter.
  */
 #include "eg_batch.cuh"
+#include "eg_pool.cuh"
 
 #include <cooperative_groups.h>
 
@@ -1928,9 +1929,7 @@ extern "C" eg_status eg_batch_credits(eg_batch *b, int32_t game, int64_t *credit
     if (!b->solved) return eg_set_error(EG_ERR_INVALID, "batch not solved");
     EG_CUDA(cudaSetDevice(b->device));
     const long long cnt = b->f_off[(size_t)game + 1] - b->f_off[(size_t)game];
-    EG_CUDA(cudaMemcpyAsync(credits, b->F + b->f_off[(size_t)game], sizeof(long long) * (size_t)cnt,
-                            cudaMemcpyDeviceToHost, b->st));
-    EG_CUDA(cudaStreamSynchronize(b->st));
+    EG_CUDA(copy_to_host(credits, b->F + b->f_off[(size_t)game], sizeof(long long) * (size_t)cnt, b->device, b->st));
     return EG_OK;
 }
 

@@ -91,19 +91,44 @@ eg_status eg_validate(const eg_game *g)
         return eg_set_error(EG_ERR_INVALID, "num_nodes0 %d outside [0, %d]", g->num_nodes0, g->num_nodes);
     if (g->row_ptr[0] != 0 || g->row_ptr[g->num_nodes] != g->num_edges)
         return eg_set_error(EG_ERR_INVALID, "row_ptr must start at 0 and end at num_edges");
-    for (int64_t v = 0; v < g->num_nodes; v++) {
+    /* first whether anything is wrong (loops that vectorise), then what */
+    const int64_t n = g->num_nodes, m = g->num_edges;
+    int bad = 0;
+    for (int64_t v = 0; v < n; v++) bad |= g->row_ptr[v + 1] <= g->row_ptr[v];
+    if (g->owner)
+        for (int64_t v = 0; v < n; v++) bad |= g->owner[v] > 1;
+    if (!bad)
+        for (int64_t j = 0; j < m; j++) bad |= (uint32_t)g->succ[j] >= (uint32_t)n;
+    if (!bad) return EG_OK;
+    for (int64_t v = 0; v < n; v++) {
         if (g->row_ptr[v + 1] <= g->row_ptr[v])
             return eg_set_error(EG_ERR_INVALID, "vertex %lld has no successor", (long long)v);
         if (g->owner && g->owner[v] > 1)
             return eg_set_error(EG_ERR_INVALID, "vertex %lld has owner %d (expected 0 or 1)",
                                 (long long)v, (int)g->owner[v]);
     }
-    for (int64_t j = 0; j < g->num_edges; j++) {
-        if (g->succ[j] < 0 || g->succ[j] >= g->num_nodes)
+    for (int64_t j = 0; j < m; j++) {
+        if (g->succ[j] < 0 || g->succ[j] >= n)
             return eg_set_error(EG_ERR_INVALID, "edge %lld has successor %d outside [0, %d)",
                                 (long long)j, g->succ[j], g->num_nodes);
     }
     (void)owner_of;
+    return EG_OK;
+}
+
+/* The transpose's input: offsets monotone, columns in range. */
+eg_status eg_check_csr(int32_t num_rows, int32_t num_cols, int64_t nnz, const int64_t *row_ptr, const int32_t *col_idx)
+{
+    int bad = 0;
+    for (int64_t r = 0; r < num_rows; r++) bad |= row_ptr[r + 1] < row_ptr[r];
+    for (int64_t j = 0; j < nnz; j++) bad |= (uint32_t)col_idx[j] >= (uint32_t)num_cols;
+    if (!bad) return EG_OK;
+    for (int64_t r = 0; r < num_rows; r++)
+        if (row_ptr[r + 1] < row_ptr[r])
+            return eg_set_error(EG_ERR_INVALID, "row_ptr not monotone at row %d", (int)r);
+    for (int64_t j = 0; j < nnz; j++)
+        if (col_idx[j] < 0 || col_idx[j] >= num_cols)
+            return eg_set_error(EG_ERR_INVALID, "column %d of entry %lld out of range", col_idx[j], (long long)j);
     return EG_OK;
 }
 

@@ -20,6 +20,9 @@ eg_status eg_owner_sort(int32_t n, int64_t m, const int64_t *ptr, const int32_t 
                         const int32_t *w, const uint8_t *owner, const int32_t *ext_of_file,
                         eg_owned_game **out);
 
+/* Checks the transpose's input (see eg_host.c). */
+eg_status eg_check_csr(int32_t num_rows, int32_t num_cols, int64_t nnz, const int64_t *row_ptr, const int32_t *col_idx);
+
 #ifdef __cplusplus
 }
 #endif

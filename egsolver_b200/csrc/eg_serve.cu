@@ -34,6 +34,7 @@
  * unit's work depends only on its own game and thresholds.
  */
 #include "eg_batch.cuh"
+#include "eg_pool.cuh"
 #include "../../include/egsolver_b200_serve.h"
 
 #include <algorithm>
@@ -93,7 +94,8 @@ struct Query {
     eg_status status = EG_OK;
     clk::time_point t_submit, t_done;
     long long rounds = 0;
-    std::vector<int64_t> result; /* threshold-major */
+    std::unique_ptr<int64_t[]> result; /* threshold-major, n * K */
+    size_t result_len = 0;
     std::vector<long long> mg;   /* MG per threshold                         */
     /* device buffers while admitted: credits n*K (threshold-major),
      * thresholds, MG, per-unit rounds and status, global credit scratch */
@@ -103,7 +105,7 @@ struct Query {
     long long *drounds = nullptr;
     int *dstatus = nullptr;
     void *dscratch = nullptr;
-    size_t dbytes = 0;
+    size_t dbytes = 0, o_rounds = 0, o_status = 0, o_end = 0; /* places in the block */
     std::vector<UnitDesc> units; /* planned at admission                     */
     std::vector<long long> cost;
     int smem = 16;
@@ -116,9 +118,9 @@ struct Launch {
     int units = 0;
     cudaEvent_t ev = nullptr;
     std::vector<int64_t> qids;
+    void *block = nullptr;      /* device memory of what follows              */
     UnitDesc *dunits = nullptr;
     LaunchCtrl *dctrl = nullptr;
-    void *dtails = nullptr;
     TailList *tl = nullptr;
     void *dscratch = nullptr;   /* hybrid tail regions                        */
     UnitSet set;                /* for the tail's launch                      */
@@ -167,7 +169,7 @@ size_t query_bytes(const ServedGame &g, int K, size_t scratch)
 
 void free_query_device(Query &q, cudaStream_t st)
 {
-    if (q.dF) cudaFreeAsync(q.dF, st);
+    pool_free(q.dF, st);
     if (q.ready) cudaEventDestroy(q.ready);
     q.ready = nullptr;
     q.dF = nullptr;
@@ -181,7 +183,7 @@ void free_query_device(Query &q, cudaStream_t st)
 void drop_resident(eg_server *s, ServedGame &g)
 {
     s->device_bytes -= (int64_t)g.pd.bytes;
-    if (g.pd.block) cudaFreeAsync(g.pd.block, s->upload_stream);
+    pool_free(g.pd.block, s->upload_stream);
     cudaStreamSynchronize(s->upload_stream);
     g.pd = PackedDev();
     g.resident = false;
@@ -240,7 +242,7 @@ bool reap(eg_server *s)
         UnitCtrl c;
         LaunchCtrl cv;
         memset(&c, 0, sizeof c);
-        const bool have = e == cudaSuccess && cudaMemcpy(&cv, l.dctrl, sizeof cv, cudaMemcpyDeviceToHost) == cudaSuccess;
+        const bool have = e == cudaSuccess && copy_to_host(&cv, l.dctrl, sizeof cv, s->o.device, s->streams[l.stream]) == cudaSuccess;
         if (have && !l.in_tail && tail_entries(l.set, cv) > 0) {
             /* some units went to the tail: its kernels run now */
             cudaStream_t st = s->streams[l.stream];
@@ -271,13 +273,15 @@ bool reap(eg_server *s)
             eg_status st = e == cudaSuccess ? EG_OK : EG_ERR_CUDA;
             if (st == EG_OK) {
                 const size_t nu = q.units.size();
-                std::vector<long long> rr(nu);
-                std::vector<int> ss(nu);
-                q.result.assign((size_t)g.n * q.K, 0);
-                cudaError_t cp = cudaMemcpy(q.result.data(), q.dF, sizeof(long long) * q.result.size(),
-                                            cudaMemcpyDeviceToHost);
-                if (cp == cudaSuccess) cp = cudaMemcpy(ss.data(), q.dstatus, sizeof(int) * nu, cudaMemcpyDeviceToHost);
-                if (cp == cudaSuccess) cp = cudaMemcpy(rr.data(), q.drounds, sizeof(long long) * nu, cudaMemcpyDeviceToHost);
+                /* rounds and status lie behind one another in the block */
+                std::vector<char> tail(q.o_end - q.o_rounds);
+                q.result_len = (size_t)g.n * q.K;
+                q.result.reset(new int64_t[q.result_len]);
+                cudaStream_t qs = s->streams[l.stream];
+                cudaError_t cp = copy_to_host(q.result.get(), q.dF, sizeof(long long) * q.result_len, s->o.device, qs);
+                if (cp == cudaSuccess) cp = copy_to_host(tail.data(), q.drounds, tail.size(), s->o.device, qs);
+                const long long *rr = (const long long *)tail.data();
+                const int *ss = (const int *)(tail.data() + (q.o_status - q.o_rounds));
                 if (cp != cudaSuccess) {
                     st = EG_ERR_CUDA;
                 } else {
@@ -295,10 +299,7 @@ bool reap(eg_server *s)
             finish_query(s, q, st, now);
         }
         cudaEventDestroy(l.ev);
-        cudaFreeAsync(l.dunits, s->streams[l.stream]);
-        cudaFreeAsync(l.dctrl, s->streams[l.stream]);
-        cudaFreeAsync(l.dtails, s->streams[l.stream]);
-        if (l.dscratch) cudaFreeAsync(l.dscratch, s->streams[l.stream]);
+        pool_free(l.block, s->streams[l.stream]);
         s->inflight.erase(s->inflight.begin() + (long)i);
     }
     if (any) s->cv_done.notify_all();
@@ -359,8 +360,7 @@ bool admit(eg_server *s, std::unique_lock<std::mutex> &lk)
             const size_t pb = packed_dev_bytes(g.hp);
             eg_status st = EG_OK;
             lk.unlock();
-            if (cudaMallocAsync(&blk, pb, s->upload_stream) != cudaSuccess) {
-                cudaGetLastError();
+            if (pool_alloc(&blk, pb, s->o.device, s->upload_stream) != cudaSuccess) {
                 st = eg_set_error(EG_ERR_OOM, "device allocation of a game failed");
             }
             PackedDev pd;
@@ -369,7 +369,7 @@ bool admit(eg_server *s, std::unique_lock<std::mutex> &lk)
                 st = eg_set_error(EG_ERR_CUDA, "game upload failed");
             lk.lock();
             if (st != EG_OK) {
-                if (blk) cudaFreeAsync(blk, s->upload_stream);
+                pool_free(blk, s->upload_stream);
                 s->pending.pop_front();
                 finish_query(s, q, st, clk::now());
                 s->cv_done.notify_all();
@@ -391,10 +391,7 @@ bool admit(eg_server *s, std::unique_lock<std::mutex> &lk)
         const size_t o_scr = o_status + ((nu * sizeof(int) + 255) & ~(size_t)255);
         const size_t total = o_scr + scratch;
         char *blk = nullptr;
-        if (cudaMallocAsync((void **)&blk, total, s->upload_stream) != cudaSuccess) {
-            cudaGetLastError();
-            break;
-        }
+        if (pool_alloc((void **)&blk, total, s->o.device, s->upload_stream) != cudaSuccess) break;
         q.dF = (long long *)blk;
         q.dthr = (int *)(blk + o_thr);
         q.dmg = (long long *)(blk + o_mg);
@@ -402,6 +399,9 @@ bool admit(eg_server *s, std::unique_lock<std::mutex> &lk)
         q.dstatus = (int *)(blk + o_status);
         q.dscratch = scratch ? (void *)(blk + o_scr) : nullptr;
         q.dbytes = total;
+        q.o_rounds = o_rounds;
+        q.o_status = o_status;
+        q.o_end = o_status + nu * sizeof(int);
         size_t goff = 0;
         for (size_t u = 0; u < nu; u++) {
             UnitDesc &d = units[u];
@@ -421,11 +421,21 @@ bool admit(eg_server *s, std::unique_lock<std::mutex> &lk)
         q.units.swap(units);
         q.cost.swap(cost);
         q.smem = smem;
-        cudaMemcpyAsync(q.dthr, q.p.data(), sizeof(int) * (size_t)q.K, cudaMemcpyHostToDevice, s->upload_stream);
-        cudaMemcpyAsync(q.dmg, q.mg.data(), sizeof(long long) * (size_t)q.K, cudaMemcpyHostToDevice, s->upload_stream);
-        cudaEventCreateWithFlags(&q.ready, cudaEventDisableTiming);
-        cudaEventRecord(q.ready, s->upload_stream);
-        cudaStreamSynchronize(s->upload_stream); /* q.p / q.mg are host memory that may go away */
+        /* thresholds and MG in one copy (through a staging buffer: no wait) */
+        const CopyPart parts[2] = {{q.p.data(), 0, sizeof(int) * (size_t)q.K},
+                                   {q.mg.data(), o_mg - o_thr, sizeof(long long) * (size_t)q.K}};
+        cudaError_t ce = copy_parts_to_device(q.dthr, parts, 2, o_mg - o_thr + parts[1].bytes, s->o.device, s->upload_stream);
+        if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&q.ready, cudaEventDisableTiming);
+        if (ce == cudaSuccess) ce = cudaEventRecord(q.ready, s->upload_stream);
+        if (ce != cudaSuccess) {
+            cudaGetLastError();
+            free_query_device(q, s->upload_stream);
+            s->pending.pop_front();
+            finish_query(s, q, EG_ERR_CUDA, clk::now());
+            s->cv_done.notify_all();
+            any = true;
+            continue;
+        }
         s->device_bytes += (int64_t)q.dbytes;
         g.active++;
         g.last_use = ++s->tick;
@@ -457,16 +467,19 @@ eg_status prepare_batch(eg_server *s, Launch &l)
     s->next_stream = (s->next_stream + 1) % s->o.streams;
     cudaStream_t st = s->streams[l.stream];
     for (int64_t qid : l.qids) cudaStreamWaitEvent(st, s->queries[qid]->ready, 0);
-    cudaError_t e = cudaMallocAsync((void **)&l.dunits, sizeof(UnitDesc) * S.units.size(), st);
-    if (e == cudaSuccess) e = cudaMallocAsync((void **)&l.dctrl, sizeof(LaunchCtrl), st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&l.dtails, tail_bytes(S), st);
     const size_t tsb = tail_scratch_bytes(S, s->sms);
-    if (e == cudaSuccess && tsb) e = cudaMallocAsync(&l.dscratch, tsb, st);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(l.dunits, S.units.data(), sizeof(UnitDesc) * S.units.size(), cudaMemcpyHostToDevice, st);
+    const size_t ub = (sizeof(UnitDesc) * S.units.size() + 255) & ~(size_t)255;
+    const size_t cb = (sizeof(LaunchCtrl) + 255) & ~(size_t)255, tb = (tail_bytes(S) + 255) & ~(size_t)255;
+    cudaError_t e = pool_alloc(&l.block, ub + cb + tb + tsb, s->o.device, st);
+    if (e != cudaSuccess) return EG_ERR_OOM;
+    char *at = (char *)l.block;
+    l.dunits = (UnitDesc *)at;
+    l.dctrl = (LaunchCtrl *)(at + ub);
+    if (tsb) l.dscratch = at + ub + cb + tb;
+    e = copy_to_device(l.dunits, S.units.data(), sizeof(UnitDesc) * S.units.size(), s->o.device, st);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&l.ev, cudaEventDisableTiming);
     if (e != cudaSuccess) return EG_ERR_CUDA;
-    return tail_upload(S, l.dtails, st, &l.tl);
+    return tail_upload(S, at + ub + cb, st, &l.tl);
 }
 
 /* Launches a prepared micro-batch, or fails its queries (lock held). */
@@ -496,10 +509,7 @@ void start_batch(eg_server *s, Launch &l, eg_status ls)
         finish_query(s, q, ls != EG_OK ? ls : EG_ERR_CUDA, now);
     }
     if (l.ev) cudaEventDestroy(l.ev);
-    if (l.dunits) cudaFreeAsync(l.dunits, st);
-    if (l.dctrl) cudaFreeAsync(l.dctrl, st);
-    if (l.dtails) cudaFreeAsync(l.dtails, st);
-    if (l.dscratch) cudaFreeAsync(l.dscratch, st);
+    pool_free(l.block, st);
     s->cv_done.notify_all();
 }
 
@@ -532,6 +542,8 @@ bool launch_ready(eg_server *s)
 
 void worker_main(eg_server *s)
 {
+    constexpr int kSpins = 2000;
+    int quiet = 0;
     cudaSetDevice(s->o.device);
     std::unique_lock<std::mutex> lk(s->mu);
     for (;;) {
@@ -539,7 +551,17 @@ void worker_main(eg_server *s)
         progress |= admit(s, lk);
         progress |= launch_ready(s);
         if (s->stop && s->pending.empty() && s->ready.empty() && s->inflight.empty()) break;
-        if (!progress) s->cv_work.wait_for(lk, std::chrono::microseconds(200));
+        if (progress) {
+            quiet = 0;
+        } else if (!s->inflight.empty() && ++quiet < kSpins) {
+            /* a micro-batch of certified units ends within a millisecond:
+             * look again at once instead of sleeping through its end */
+            lk.unlock();
+            std::this_thread::yield();
+            lk.lock();
+        } else {
+            s->cv_work.wait_for(lk, std::chrono::microseconds(200));
+        }
     }
 }
 
@@ -565,7 +587,7 @@ void large_main(eg_server *s)
         const int K = q.K, d = q.d;
         const std::vector<int> p = q.p;
         lk.unlock();
-        std::vector<int64_t> result((size_t)g.n * K);
+        std::unique_ptr<int64_t[]> result(new int64_t[(size_t)g.n * K]());
         std::vector<int32_t> wt((size_t)g.m);
         eg_status st = EG_OK;
         long long rounds = 0;
@@ -591,12 +613,13 @@ void large_main(eg_server *s)
             st = eg_dgame_upload(&tg, &o, &dg);
             eg_stats ss;
             if (st == EG_OK) st = eg_dgame_solve(dg, &o, &ss);
-            if (st == EG_OK) st = eg_dgame_credits_i64(dg, result.data() + (size_t)k * g.n);
+            if (st == EG_OK) st = eg_dgame_credits_i64(dg, result.get() + (size_t)k * g.n);
             if (st == EG_OK) rounds = std::max(rounds, (long long)ss.rounds);
             eg_dgame_free(dg);
         }
         lk.lock();
         q.result.swap(result);
+        q.result_len = (size_t)g.n * K;
         q.rounds = rounds;
         g.active--;
         finish_query(s, q, st, clk::now());
@@ -773,7 +796,7 @@ extern "C" eg_status eg_serve_result(eg_server *s, int64_t query_id, int64_t *cr
         return eg_set_error(st, "query %lld failed with status %d", (long long)query_id, (int)st);
     }
     if (q.state != EG_QUERY_DONE) return eg_set_error(EG_ERR_BUSY, "query %lld not finished", (long long)query_id);
-    memcpy(credits, q.result.data(), sizeof(int64_t) * q.result.size());
+    memcpy(credits, q.result.get(), sizeof(int64_t) * q.result_len);
     if (rounds) *rounds = q.rounds;
     s->queries.erase(it);
     return EG_OK;
@@ -837,7 +860,7 @@ extern "C" eg_status eg_serve_destroy(eg_server *s)
     cudaSetDevice(s->o.device);
     for (auto &kv : s->queries) free_query_device(*kv.second, s->upload_stream);
     for (auto &kv : s->games)
-        if (kv.second->resident && kv.second->pd.block) cudaFreeAsync(kv.second->pd.block, s->upload_stream);
+        if (kv.second->resident) pool_free(kv.second->pd.block, s->upload_stream);
     cudaStreamSynchronize(s->upload_stream);
     for (UnitLauncher &L : s->launchers) L.destroy();
     for (cudaStream_t st : s->streams) cudaStreamDestroy(st);

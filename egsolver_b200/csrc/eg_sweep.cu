@@ -78,6 +78,7 @@
 #include "eg_sweep.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 
 namespace eg {
@@ -940,39 +941,55 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
     }
 }
 
-/* Dynamic shared memory a CTA of the kernel may have. */
-static eg_status sweep_smem(const void *fn, int dev, int *bytes)
+/* What the kernels may use of a device, asked for once: SMs, and dynamic
+ * shared memory per CTA of the one-CTA and the grid kernel (to which they are
+ * opted in). */
+struct SweepDevice {
+    std::atomic<int> sms, smem[2];
+};
+static SweepDevice g_device[64];
+
+static eg_status sweep_device(int *sms, int *smem)
 {
-    int optin = 0;
-    cudaFuncAttributes fa;
-    cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fn);
-    if (e != cudaSuccess) return eg_set_error(EG_ERR_CUDA, "sweep kernel attributes: %s", cudaGetErrorString(e));
-    *bytes = optin - (int)fa.sharedSizeBytes;
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, *bytes);
-    if (e != cudaSuccess) return eg_set_error(EG_ERR_CUDA, "sweep kernel attributes: %s", cudaGetErrorString(e));
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess || dev >= 64) return eg_set_error(EG_ERR_CUDA, "sweep kernel set-up: %s", cudaGetErrorString(e));
+    SweepDevice &d = g_device[dev];
+    if (!d.sms.load()) {
+        int count = 0, optin = 0;
+        e = cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        for (int k = 0; k < 2; k++) {
+            const void *fn = k ? (const void *)k_sweep<true> : (const void *)k_sweep<false>;
+            cudaFuncAttributes fa;
+            if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fn);
+            if (e == cudaSuccess) d.smem[k] = optin - (int)fa.sharedSizeBytes;
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem[k].load());
+        }
+        if (e != cudaSuccess) return eg_set_error(EG_ERR_CUDA, "sweep kernel set-up: %s", cudaGetErrorString(e));
+        d.sms = count;
+    }
+    *sms = d.sms;
+    smem[0] = d.smem[0];
+    smem[1] = d.smem[1];
     return EG_OK;
 }
 
 eg_status sweep_plan(int n, long long m, int max_ctas, SweepPlan *plan)
 {
-    int dev = 0, sms = 0, bytes = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return eg_set_error(EG_ERR_CUDA, "sweep kernel set-up: %s", cudaGetErrorString(e));
+    int sms = 0, smem_of[2];
+    eg_status s = sweep_device(&sms, smem_of);
+    if (s != EG_OK) return s;
     const long long total = 8 * m + m / 2 + (long long)kVertexBytes * n;
     memset(plan, 0, sizeof *plan);
     plan->block = kBlock;
-    eg_status s = sweep_smem((const void *)k_sweep<false>, dev, &bytes);
-    if (s != EG_OK) return s;
     plan->grid = 1;
-    if (total + kSlackBytes <= bytes) {
+    if (total + kSlackBytes <= smem_of[0]) {
         plan->one_cta = 1;
         plan->smem_bytes = (int)(total + kSlackBytes);
         return EG_OK;
     }
-    s = sweep_smem((const void *)k_sweep<true>, dev, &bytes);
-    if (s != EG_OK) return s;
+    const int bytes = smem_of[1];
     plan->grid = max_ctas > 0 && max_ctas < sms ? max_ctas : sms;
     plan->smem_bytes = bytes;
     plan->values = (size_t)n + (size_t)kPadSlots * plan->grid;

@@ -1,0 +1,64 @@
+"""GPU tests of what calls share (eg_pool.cu): staged copies at the edges of
+their chunks, threads that solve at once, and the transpose's device check."""
+from __future__ import annotations
+
+import threading
+
+import numpy as np
+import pytest
+
+import egsolver_b200 as eg
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def csr(rng, rows, cols, nnz):
+    rp = np.concatenate([[0], np.cumsum(np.bincount(rng.integers(0, rows, nnz), minlength=rows))]).astype(np.int64)
+    return rp, rng.integers(0, cols, nnz).astype(np.int32), rng.integers(-9, 9, nnz).astype(np.int32)
+
+
+# 131,072 entries of 4 bytes fill half a staging buffer
+@pytest.mark.parametrize("nnz", [1, 65536, 65537, 131071, 131072, 131073, 2_300_003])
+def test_staged_copies_of_the_transpose(nnz):
+    rng = np.random.default_rng(nnz)
+    rows, cols = 65535, 65537
+    rp, col, val = csr(rng, rows, cols, nnz)
+    for a, b in zip(eg.csr2csc(rows, cols, rp, col, val), O.csr2csc(rows, cols, rp, col, val)):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_malformed_transposes_are_refused():
+    rng = np.random.default_rng(2)
+    rp, col, val = csr(rng, 3000, 2000, 40000)
+    for bad_rp, bad_col in ((None, 2000), (None, -1), (1500, None)):
+        r, c = rp.copy(), col.copy()
+        if bad_col is not None:
+            c[39999] = bad_col
+        else:
+            r[bad_rp] = 1 << 40
+        with pytest.raises(eg.EGError) as ei:
+            eg.csr2csc(3000, 2000, r, c, val)
+        assert ei.value.name == "EG_ERR_INVALID"
+    for a, b in zip(eg.csr2csc(3000, 2000, rp, col, val), O.csr2csc(3000, 2000, rp, col, val)):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_threads_share_the_pools():
+    """Games of several sizes solved by four threads at once, twice each."""
+    games = [eg.generate(4, n, 16, 50, 5 + i, param=2) for i, n in enumerate((60, 900, 4000, 70000, 3000, 150))]
+    alone = [eg.solve(g)[0] for g in games]
+    wrong = []
+
+    def work(k):
+        for i in range(2 * len(games)):
+            j = (i + k) % len(games)
+            if not np.array_equal(eg.solve(games[j])[0], alone[j]):
+                wrong.append(j)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
