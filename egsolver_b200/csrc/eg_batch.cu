@@ -119,7 +119,13 @@ struct Shared {
 /* What a unit's sweep computes: lifts of the credits; lifts of a potential;
  * or the removal of vertices whose potential is not one.  See run_unit. */
 enum { UNIT_PRIMAL, UNIT_DUAL, UNIT_KILL };
-constexpr int kUnitFirstPrimal = 4, kUnitSecondPrimal = 16, kUnitFirstDual = 8, kUnitMaxDual = 128;
+/* The lengths: thresholds far from the game's value end in the first primal
+ * or dual stretch, most others after one certificate of six sweeps, and 32
+ * primal sweeps then finish what is left in one go.  (4, 16, 8): 32 games of
+ * 16K-147K edges x 8 thresholds 8% slower; (2, 16, 6): 10% faster on 64 games of 1024-65536
+ * nodes, 25-50% slower on three other sets, whose near-critical units then
+ * restart once more. */
+constexpr int kUnitFirstPrimal = 2, kUnitSecondPrimal = 32, kUnitFirstDual = 6, kUnitMaxDual = 128;
 constexpr long long kUnitMaxPrimal = 1 << 20;
 /* Units below this many sweeps do not park: all but 1 in 500 of the
  * thresholds of random games at uniform thresholds end within it, and the
@@ -997,6 +1003,19 @@ void split_thresholds(int K, int kg_max, std::vector<std::pair<int, int>> *group
     }
 }
 
+long long sweep_cost(long long m, int kg)
+{
+    const long long waves = kg >= 8 ? 34 : kg >= 4 ? 22 : kg >= 2 ? 12 : 7;
+    return (m + 31) / 32 * waves / 2;
+}
+
+int group_for(long long m, int kg_max, long long limit)
+{
+    int kg = kg_max;
+    while (m > kSplitEdges && kg > 1 && sweep_cost(m, kg) > limit) kg >>= 1;
+    return kg;
+}
+
 eg_status make_units(const HostPacked &h, const PackedDev &pd, int K, int d, const int *p, const long long *mg,
                      const int *p_dev, const long long *mg_dev, long long *F_dev, int smem_budget, int kg_cap,
                      std::vector<UnitDesc> *units, std::vector<size_t> *gneed, std::vector<long long> *cost,
@@ -1470,6 +1489,7 @@ struct eg_batch {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int num_games = 0, K = 0, d = 1;
     long long total_nodes = 0, total_edges = 0;
+    bool split = true;               /* smaller groups for large games while SMs are idle */
     int block = 1024, kg_cap = 8, smem_budget = 0, sms = 148, tail_rows = 0, park_percent = 10;
     int tail_sweeps = kTailSweeps;
     int tail_cluster = kTailCluster;
@@ -1623,6 +1643,7 @@ extern "C" eg_status eg_batch_create(const eg_game *games, int32_t num_games, co
     b->total_edges = tm;
     b->block = opts->block ? opts->block : 1024;
     b->kg_cap = opts->group_max ? opts->group_max : 8;
+    b->split = opts->group_max == 0;
     b->tail_rows = opts->tail_rows > 0 ? opts->tail_rows : 0;
     b->park_percent = opts->park_percent > 0 ? opts->park_percent : 10;
     b->tail_sweeps = opts->tail_sweeps > 0 ? opts->tail_sweeps : kTailSweeps;
@@ -1695,11 +1716,33 @@ static eg_status batch_plan(eg_batch *b)
     std::vector<long long> cost;
     std::vector<size_t> gneed; /* global scratch bytes per unit (0: shared memory) */
     int smem = 16;
+    /* the groups of large games, halved while SMs are left for the units: the
+     * least cost of a sweep at which the batch still fits the GPU at once.
+     * 32 games of 1024-16384 nodes x 8 thresholds, 16 edges a node at most:
+     * 43 units, bound by the bank conflicts of the largest, 835-983 us; 135
+     * units 488-528 us.  16 games of 1024-65536 nodes: 9.5 -> 3.2 ms; 100 games of
+     * 1024-8192 nodes 8.3 -> 7.8 ms; 400 games are not split. */
+    long long limit = sweep_cost(kSplitEdges, 8);
+    if (b->split) {
+        for (;; limit += limit / 4) {
+            long long count = 0;
+            bool least = true;
+            for (int g = 0; g < b->num_games; g++) {
+                const int kg = group_for(b->hp[(size_t)g].m, b->kg_cap, limit);
+                least = least && kg == b->kg_cap;
+                count += K / kg + __builtin_popcount((unsigned)(K % kg)); /* as split_thresholds */
+            }
+            if (count <= b->sms || least) break;
+        }
+    } else {
+        limit = INT64_MAX;
+    }
     for (int g = 0; g < b->num_games; g++) {
         const size_t before = units.size();
         EG_TRY(make_units(b->hp[(size_t)g], b->pd[(size_t)g], K, b->d, b->p_host.data() + (size_t)g * K,
                           b->mg_host.data() + (size_t)g * K, b->p_dev + (size_t)g * K, b->mg_dev + (size_t)g * K,
-                          b->F + b->f_off[(size_t)g], b->smem_budget, b->kg_cap, &units, &gneed, &cost, &smem,
+                          b->F + b->f_off[(size_t)g], b->smem_budget,
+                          group_for(b->hp[(size_t)g].m, b->kg_cap, limit), &units, &gneed, &cost, &smem,
                           b->tail_rows));
         for (size_t i = before; i < units.size(); i++) ugame.push_back(g);
     }

@@ -174,6 +174,18 @@ UnitPlan plan_game(const HostPacked &h, bool credit64, int smem_budget, int kg_c
  * groups of one, credits in global scratch); appends (k0, log2 kg). */
 void split_thresholds(int K, int kg_max, std::vector<std::pair<int, int>> *groups);
 
+/* Shared-memory cycles of a sweep of m edges for kg thresholds, which bound
+ * it: a warp's gathers of kg random 4-byte credits take 3.5, 6.2, 11 or 17
+ * wavefronts for 1, 2, 4 or 8 of them (the fullest of the banks that 32 random
+ * rows meet).  A group of eight needs 60% of the wavefronts of eight single
+ * thresholds, so groups are cut only while SMs are idle, and not for games of
+ * up to kSplitEdges edges, whose sweeps take less than 5 us whatever the
+ * group. */
+constexpr long long kSplitEdges = 16384;
+long long sweep_cost(long long m, int kg);
+/* The largest group (halving kg_max) whose sweep costs at most `limit`. */
+int group_for(long long m, int kg_max, long long limit);
+
 /* Appends the units of one game at K thresholds: p / mg are the host
  * values, p_dev / mg_dev / F_dev the device arrays the units read and
  * write (F_dev[k * n + v]).  Per unit it also appends the global scratch

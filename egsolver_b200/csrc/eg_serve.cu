@@ -331,8 +331,16 @@ bool admit(eg_server *s, std::unique_lock<std::mutex> &lk)
         std::vector<size_t> gneed;
         std::vector<long long> cost;
         int smem = 16;
+        /* a large game's group: the smallest with which the queries at hand
+         * leave no more units than SMs (12 queries of 6 thresholds on games of
+         * 1000-8000 nodes: 2.42-2.55 -> 2.15-2.40 ms) */
+        int kg = 8;
+        if (g.m > kSplitEdges) {
+            const long long at_hand = (long long)s->pending.size() + s->admitted_now;
+            while (kg > 1 && at_hand * ((q.K + kg / 2 - 1) / (kg / 2)) <= s->sms) kg >>= 1;
+        }
         eg_status ps = make_units(g.hp, PackedDev(), q.K, q.d, q.p.data(), q.mg.data(), nullptr, nullptr, nullptr,
-                                  s->smem_budget, 8, &units, &gneed, &cost, &smem);
+                                  s->smem_budget, kg, &units, &gneed, &cost, &smem);
         if (ps != EG_OK) {
             s->pending.pop_front();
             finish_query(s, q, ps, clk::now());

@@ -203,3 +203,45 @@ def test_unit_certificates(n, wmax, d, p):
         _, st = b.solve()
         assert st.games_failed == 0
         check_batch(b, games, thresholds, d)
+
+
+def planned_units(edges, K, sms=148):
+    """The units of a batch by the rule of its groups: halved from eight in games
+    of more than 16,384 edges, to the least cost of a sweep that fits the SMs."""
+    def cost(m, kg):
+        return (m + 31) // 32 * {8: 34, 4: 22, 2: 12, 1: 7}[kg] // 2
+
+    def group(m, limit):
+        kg = 8
+        while m > 16384 and kg > 1 and cost(m, kg) > limit:
+            kg //= 2
+        return kg
+
+    limit = cost(16384, 8)
+    while True:
+        groups = [group(m, limit) for m in edges]
+        count = sum(K // kg + (K % kg).bit_count() for kg in groups)
+        if count <= sms or min(groups) == 8:
+            return count
+        limit += limit // 4
+
+
+@pytest.mark.parametrize("num,nodes,K", [
+    (3, 1024, 8), (3, 1025, 8), (3, 1900, 8), (3, 3000, 8), (3, 12000, 3),  # idle SMs
+    (60, 4096, 8), (100, 1100, 8), (100, 2400, 8),                          # as many as fit
+    (150, 1100, 5), (150, 2400, 5),                                         # more games than SMs
+])
+def test_groups_of_large_games(num, nodes, K):
+    games = [eg.generate(4, nodes, 16, 20, 300 + i, param=2) for i in range(num)]
+    rng = np.random.default_rng(num)
+    p = rng.integers(-60, 61, size=(num, K)).astype(np.int32)
+    got = []
+    for group_max in (0, 8):
+        with eg.Batch(games, thresholds=K, scale=4, group_max=group_max) as b:
+            b.set_thresholds(p)
+            _, st = b.solve()
+            got.append((st.num_units, [b.credits(g) for g in range(num)]))
+    assert got[0][0] == planned_units([g.num_edges for g in games], K)
+    assert got[1][0] == num * (K // 8 + (K % 8).bit_count())
+    for a, b in zip(got[0][1], got[1][1]):
+        np.testing.assert_array_equal(a, b)
