@@ -13,6 +13,7 @@
 #include "eg_pool.cuh"
 #include "eg_prep.cuh"
 #include "eg_sweep.cuh"
+#include "eg_transpose.cuh"
 
 #include <algorithm>
 #include <cstdio>
@@ -1027,6 +1028,39 @@ extern "C" eg_status eg_solve_i64(const eg_game *game, const eg_opts *opts, int6
 /* Standalone transpose                                                 */
 /* ------------------------------------------------------------------ */
 
+/* The transpose by a radix sort of (column, edge) pairs: for columns too long
+ * for k_transpose.  The inputs are checked. */
+static cudaError_t radix_transpose(const TransposeParams &t, int dev, cudaStream_t st)
+{
+    const long long cap = std::max(t.nnz, 1);
+    int *d_k0 = nullptr, *d_v0 = nullptr, *d_k1 = nullptr, *d_v1 = nullptr, *d_rows = nullptr, *d_cnt = nullptr, *d_scr = nullptr;
+    Arena ar;
+    ar.add(&d_k0, (size_t)cap);
+    ar.add(&d_v0, (size_t)cap);
+    ar.add(&d_k1, (size_t)cap);
+    ar.add(&d_v1, (size_t)cap);
+    ar.add(&d_rows, (size_t)cap);
+    ar.add(&d_cnt, (size_t)t.ncols + 1);
+    ar.add(&d_scr, (size_t)(radix_scratch_ints(cap) + scan_scratch_ints((long long)t.ncols + 1) + 64));
+    char *block = nullptr;
+    cudaError_t e = pool_alloc((void **)&block, ar.total, dev, st);
+    if (e != cudaSuccess) return e;
+    for (const Arena::Part &x : ar.parts) *x.p = block + x.at;
+    e = cudaMemsetAsync(d_cnt, 0, sizeof(int) * ((size_t)t.ncols + 1), st);
+    if (e == cudaSuccess) {
+        const unsigned gw = grid_for((long long)t.nrows * 32, 256);
+        k_csr_expand<<<gw, 256, 0, st>>>(t.nrows, t.row_ptr, t.col, d_k0, d_v0, d_rows, d_cnt);
+        excl_scan(d_cnt, (long long)t.ncols + 1, d_scr, st);
+        int *sk, *sv;
+        radix_sort_pairs(d_k0, d_v0, d_k1, d_v1, t.nnz, bits_for(t.ncols), d_scr, st, &sk, &sv);
+        k_csc_gather<<<grid_for(t.nnz, 256), 256, 0, st>>>(t.nnz, sv, d_rows, t.val, t.csc_row, t.csc_val);
+        k_widen<<<grid_for((long long)t.ncols + 1, 256), 256, 0, st>>>((long long)t.ncols + 1, d_cnt, t.csc_ptr);
+        e = cudaGetLastError();
+    }
+    pool_free(block, st);
+    return e;
+}
+
 extern "C" eg_status eg_csr2csc_i32(int32_t num_rows, int32_t num_cols, int64_t nnz, const int64_t *row_ptr,
                                    const int32_t *col_idx, const int32_t *val, int64_t *csc_ptr, int32_t *csc_row,
                                    int32_t *csc_val)
@@ -1043,65 +1077,77 @@ extern "C" eg_status eg_csr2csc_i32(int32_t num_rows, int32_t num_cols, int64_t 
         EG_TRY(eg_check_csr(num_rows, num_cols, nnz, row_ptr, col_idx));
         return eg_set_error(EG_ERR_NO_DEVICE, "no CUDA device available");
     }
-    int dev = 0;
+    int dev = 0, sms = 0;
     EG_CUDA(cudaGetDevice(&dev));
+    EG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     Lane *lane = lane_take(dev);
     if (!lane) return eg_set_error(EG_ERR_CUDA, "creation of a stream and its events failed");
     cudaStream_t st = lane->st;
-    const long long cap = std::max<long long>(nnz, 1);
-    long long *d_rp = nullptr, *d_cp64 = nullptr;
-    int *d_col = nullptr, *d_val = nullptr, *d_k0 = nullptr, *d_v0 = nullptr, *d_k1 = nullptr, *d_v1 = nullptr;
-    int *d_rows = nullptr, *d_cnt = nullptr, *d_orow = nullptr, *d_oval = nullptr, *d_scr = nullptr;
-    const long long scr = radix_scratch_ints(cap) + scan_scratch_ints((long long)num_cols + 1) + 64;
-    Arena ar;
+    const size_t cap = (size_t)std::max<long long>(nnz, 1);
+    TransposeParams t;
+    memset(&t, 0, sizeof t);
+    t.nrows = num_rows;
+    t.ncols = num_cols;
+    t.nnz = (int)nnz;
+    t.wait_limit_ns = kWaitLimitNs;
+    long long *d_rp = nullptr;
+    int *d_col = nullptr, *d_val = nullptr;
+    Arena ar; /* inputs with the zeroed control block in one range, that block and the outputs in another */
     ar.add(&d_rp, (size_t)num_rows + 1);
-    ar.add(&d_col, (size_t)cap);
-    ar.add(&d_val, (size_t)cap);
+    ar.add(&d_col, cap);
+    ar.add(&d_val, cap);
+    ar.add(&t.ctrl, 1);
     const size_t inputs = ar.total;
-    ar.add(&d_k0, (size_t)cap);
-    ar.add(&d_v0, (size_t)cap);
-    ar.add(&d_k1, (size_t)cap);
-    ar.add(&d_v1, (size_t)cap);
-    ar.add(&d_rows, (size_t)cap);
-    ar.add(&d_orow, (size_t)cap);
-    ar.add(&d_oval, (size_t)cap);
-    ar.add(&d_cnt, (size_t)num_cols + 2); /* columns' counts; then the check's flag */
-    ar.add(&d_cp64, (size_t)num_cols + 1);
-    ar.add(&d_scr, (size_t)scr);
+    ar.add(&t.csc_ptr, (size_t)num_cols + 1);
+    ar.add(&t.csc_row, cap);
+    ar.add(&t.csc_val, cap);
+    const size_t outputs = ar.total;
+    ar.add(&t.count, (size_t)num_cols + 1);
+    ar.add(&t.totals, (size_t)kTransposeGrid);
+    ar.add(&t.rank, cap);
+    ar.add(&t.rec, cap);
     char *block = nullptr;
     cudaError_t e = pool_alloc((void **)&block, ar.total, dev, st);
     if (e == cudaSuccess) {
         for (const Arena::Part &x : ar.parts) *x.p = block + x.at;
-        const CopyPart parts[3] = {{row_ptr, 0, sizeof(long long) * ((size_t)num_rows + 1)},
+        t.row_ptr = d_rp;
+        t.col = d_col;
+        t.val = d_val;
+        static const TransposeCtrl zero = {};
+        const CopyPart parts[4] = {{row_ptr, 0, sizeof(long long) * ((size_t)num_rows + 1)},
+                                   {&zero, (size_t)((char *)t.ctrl - block), sizeof zero},
                                    {col_idx, (size_t)((char *)d_col - block), sizeof(int) * (size_t)nnz},
                                    {val, (size_t)((char *)d_val - block), sizeof(int) * (size_t)nnz}};
-        e = copy_parts_to_device(block, parts, nnz ? 3 : 1, inputs, dev, st);
+        e = copy_parts_to_device(block, parts, nnz ? 4 : 2, inputs, dev, st);
     }
-    int *d_bad = d_cnt + num_cols + 1, *h_bad = (int *)lane->page;
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_cnt, 0, sizeof(int) * ((size_t)num_cols + 2), st);
-    if (e == cudaSuccess) {
-        k_check_csr<<<grid_for(std::max<long long>(nnz, num_rows), 256), 256, 0, st>>>(num_rows, num_cols, nnz, d_rp, d_col,
-                                                                                    d_bad);
-        const unsigned gw = grid_for((long long)num_rows * 32, 256);
-        k_csr_expand<<<gw, 256, 0, st>>>(num_rows, d_rp, d_col, d_bad, d_k0, d_v0, d_rows, d_cnt);
-        excl_scan(d_cnt, (long long)num_cols + 1, d_scr, st);
-        int *sk, *sv;
-        radix_sort_pairs(d_k0, d_v0, d_k1, d_v1, nnz, bits_for(num_cols), d_scr, st, &sk, &sv);
-        k_csc_gather<<<grid_for(nnz, 256), 256, 0, st>>>(nnz, d_bad, sv, d_rows, d_val, d_orow, d_oval);
-        k_widen<<<grid_for((long long)num_cols + 1, 256), 256, 0, st>>>((long long)num_cols + 1, d_cnt, d_cp64);
-        e = cudaGetLastError();
+    const CopyItem outs[3] = {{csc_ptr, t.csc_ptr, sizeof(long long) * ((size_t)num_cols + 1)},
+                              {csc_row, t.csc_row, sizeof(int) * (size_t)nnz},
+                              {csc_val, t.csc_val, sizeof(int) * (size_t)nnz}};
+    if (e == cudaSuccess) e = launch_transpose(t, transpose_grid(num_rows, num_cols, nnz, sms), st);
+    /* what became of it: with the outputs where those are small */
+    TransposeCtrl got = {};
+    bool out = false;
+    const size_t block_out = outputs - (size_t)((char *)t.ctrl - block);
+    if (e == cudaSuccess && block_out <= kStageBlock) {
+        e = copy_block_to_host(t.ctrl, block_out, dev, st, [&](const char *b) {
+            memcpy(&got, b, sizeof got);
+            out = !got.bad && !got.skewed && !got.abort;
+            for (int i = 0; i < 3 && out; i++)
+                if (outs[i].bytes) memcpy(outs[i].host, b + ((char *)outs[i].dev - (char *)t.ctrl), outs[i].bytes);
+        });
+    } else if (e == cudaSuccess) {
+        e = cudaMemcpyAsync(lane->page, t.ctrl, sizeof got, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (e == cudaSuccess) memcpy(&got, lane->page, sizeof got);
     }
-    const CopyItem outs[3] = {{csc_ptr, d_cp64, sizeof(long long) * ((size_t)num_cols + 1)},
-                              {csc_row, d_orow, sizeof(int) * (size_t)nnz},
-                              {csc_val, d_oval, sizeof(int) * (size_t)nnz}};
-    bool bad = false;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e == cudaSuccess) bad = *h_bad != 0;
-    if (e == cudaSuccess && !bad) e = copy_list(outs, 3, true, dev, st);
+    if (e == cudaSuccess && !out && !got.bad && !got.abort) {
+        if (got.skewed) e = radix_transpose(t, dev, st);
+        if (e == cudaSuccess) e = copy_list(outs, 3, true, dev, st);
+    }
     pool_free(block, st);
     lane_give(lane);
-    if (bad) return eg_check_csr(num_rows, num_cols, nnz, row_ptr, col_idx); /* says what is wrong */
+    if (e == cudaSuccess && got.abort) return eg_set_error(EG_ERR_TIMEOUT, "transpose: a wait of the grid ran out");
+    if (e == cudaSuccess && got.bad) return eg_check_csr(num_rows, num_cols, nnz, row_ptr, col_idx); /* says what is wrong */
     if (e != cudaSuccess) {
         cudaGetLastError();
         return eg_set_error(e == cudaErrorMemoryAllocation ? EG_ERR_OOM : EG_ERR_CUDA, "transpose failed: %s",

@@ -30,7 +30,7 @@ namespace {
 constexpr int kMaxDevices = 64;
 constexpr unsigned long long kPoolKeep = 64ull << 20; /* idle device memory per device */
 constexpr size_t kIdleLanes = 16, kIdleStages = 16;   /* per device; per process  */
-constexpr size_t kHalf = 512 << 10;                   /* a staging buffer has two halves */
+constexpr size_t kHalf = kStageBlock;                   /* a staging buffer has two halves */
 constexpr size_t kMapFrom = 128 << 10;                /* smaller arrays come from memory in use */
 constexpr int kCopyThreads = 8;
 
@@ -373,6 +373,21 @@ cudaError_t copy_parts_to_device(void *dev, const CopyPart *parts, int count, si
     if (e == cudaSuccess) e = cudaEventRecord(s->ev[0], st);
     if (e == cudaSuccess) s->busy[0] = true;
     else cudaStreamSynchronize(st);
+    stage_give(s);
+    return e;
+}
+
+cudaError_t copy_block_to_host(const void *dev, size_t bytes, int device, cudaStream_t st,
+                               const std::function<void(const char *)> &look)
+{
+    Stage *s = stage_take(device);
+    if (!s) return cudaErrorMemoryAllocation;
+    cudaError_t e = s->busy[0] ? cudaEventSynchronize(s->ev[0]) : cudaSuccess;
+    s->busy[0] = false;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(s->p, dev, bytes, cudaMemcpyDeviceToHost, st);
+    const cudaError_t x = cudaStreamSynchronize(st); /* also on an error: no copy may still use the buffer */
+    if (e == cudaSuccess) e = x;
+    if (e == cudaSuccess) look(s->p);
     stage_give(s);
     return e;
 }

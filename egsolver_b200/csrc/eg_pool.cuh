@@ -14,6 +14,8 @@
 
 #include <cuda_runtime.h>
 
+#include <functional>
+
 #include "eg_internal.h"
 
 namespace eg {
@@ -55,6 +57,11 @@ struct CopyPart {
 /* Several host arrays to places in one device block (`total`: its end); small
  * ones together in one copy. */
 cudaError_t copy_parts_to_device(void *dev, const CopyPart *parts, int count, size_t total, int device, cudaStream_t st);
+/* A device block of at most kStageBlock bytes in one copy after what `st`
+ * holds; `look` sees it in the staging buffer. */
+constexpr size_t kStageBlock = 512 << 10;
+cudaError_t copy_block_to_host(const void *dev, size_t bytes, int device, cudaStream_t st,
+                               const std::function<void(const char *)> &look);
 
 }  // namespace eg
 

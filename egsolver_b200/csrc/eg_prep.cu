@@ -503,24 +503,11 @@ void launch_gather_out(int in_bits, int out_bits, int n, const int *iperm, const
 /* Transpose of an input CSR (values kept): the reference's csr2csc.    */
 /* ------------------------------------------------------------------ */
 
-/* *bad is raised when an offset decreases or a column is out of range: the
- * host's loop over 6.3 M columns took 3.4 ms of a 10 ms call, this 0.01 ms.
- * The kernels that index by either return at once then. */
-__global__ void k_check_csr(int nrows, int ncols, long long nnz, const long long *row_ptr, const int *col, int *bad)
-{
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
-    bool wrong = false;
-    for (long long r = t; r < nrows; r += step) wrong |= row_ptr[r + 1] < row_ptr[r];
-    for (long long j = t; j < nnz; j += step) wrong |= (unsigned)col[j] >= (unsigned)ncols;
-    if (wrong) *bad = 1;
-}
-
 /* One warp per row: key = column, value = edge index, the edge's row; also
  * counts columns. */
-__global__ void k_csr_expand(int nrows, const long long *row_ptr, const int *col, const int *bad, int *key, int *val,
+__global__ void k_csr_expand(int nrows, const long long *row_ptr, const int *col, int *key, int *val,
                              int *row_of_edge, int *colcount)
 {
-    if (*bad) return;
     const int lane = threadIdx.x & 31;
     const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -534,10 +521,9 @@ __global__ void k_csr_expand(int nrows, const long long *row_ptr, const int *col
     }
 }
 
-__global__ void k_csc_gather(long long nnz, const int *bad, const int *sorted_edge, const int *row_of_edge,
-                             const int *val, int *csc_row, int *csc_val)
+__global__ void k_csc_gather(long long nnz, const int *sorted_edge, const int *row_of_edge, const int *val,
+                             int *csc_row, int *csc_val)
 {
-    if (*bad) return;
     for (long long l = (long long)blockIdx.x * blockDim.x + threadIdx.x; l < nnz; l += (long long)gridDim.x * blockDim.x) {
         const int j = sorted_edge[l];
         csc_row[l] = row_of_edge[j];

@@ -65,10 +65,9 @@ void launch_count_top(int bits, int n_pad, const void *F, unsigned long long *ou
 /* out[v] = F[iperm[v]] converted between widths, TOP kept as TOP */
 void launch_gather_out(int in_bits, int out_bits, int n, const int *iperm, const void *F, void *out, cudaStream_t st);
 
-__global__ void k_check_csr(int nrows, int ncols, long long nnz, const long long *row_ptr, const int *col, int *bad);
-__global__ void k_csr_expand(int nrows, const long long *row_ptr, const int *col, const int *bad, int *key, int *val,
+__global__ void k_csr_expand(int nrows, const long long *row_ptr, const int *col, int *key, int *val,
                              int *row_of_edge, int *colcount);
-__global__ void k_csc_gather(long long nnz, const int *bad, const int *sorted_edge, const int *row_of_edge,
+__global__ void k_csc_gather(long long nnz, const int *sorted_edge, const int *row_of_edge,
                              const int *val, int *csc_row, int *csc_val);
 __global__ void k_widen(long long len, const int *in, long long *out);
 

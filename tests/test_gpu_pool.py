@@ -62,3 +62,18 @@ def test_threads_share_the_pools():
     for t in threads:
         t.join()
     assert not wrong
+
+
+@pytest.mark.parametrize("rows,cols,nnz,hot", [
+    (1, 1, 1, 0), (5, 3, 2048, 0), (300, 7, 2049, 0),             # one CTA and two
+    (100, 70000, 300, 0), (70000, 100, 300, 0), (1, 50000, 4000, 0),  # few entries, many columns or rows
+    (3000, 4096, 60000, 2048), (3000, 4095, 60000, 20000),        # a column ordered here, one left to the sort
+    (900, 1, 2500, 2500), (200003, 130001, 1500000, 9000), (250000, 300000, 900000, 200000),
+])
+def test_transpose_edges(rows, cols, nnz, hot):
+    rng = np.random.default_rng(nnz)
+    rp, col, val = csr(rng, rows, cols, nnz)
+    if hot:
+        col[rng.choice(nnz, hot, replace=False)] = cols - 1
+    for a, b in zip(eg.csr2csc(rows, cols, rp, col, val), O.csr2csc(rows, cols, rp, col, val)):
+        np.testing.assert_array_equal(a, b)
