@@ -49,9 +49,9 @@
  * successors' values from L2.  Vertices of at most kLightDeg out-edges are
  * sorted by (owner, out-degree) and cut into slices of 32, a warp's lanes; a
  * slice's edges lie column by column, so a thread walks its vertex without
- * bank conflicts, shuffles or much divergence.  A warp's lanes share a vertex
- * of more edges; one of more than kHubEdges is cut into segments dealt to the
- * CTA's warps.  The values that gathers read are numbered the same way (the
+ * bank conflicts, shuffles or much divergence; where a CTA has few, 2, 4 or 8
+ * lanes share each.  A warp's lanes share a vertex of more edges; one of more
+ * than kHubEdges is cut into segments dealt to the CTA's warps.  The values that gathers read are numbered the same way (the
  * CTA's base + slot), so a slice's raises are written as whole sectors.  No
  * transpose is needed.  A game that fits one CTA runs in one, every value in
  * shared memory and __syncthreads for a barrier.
@@ -63,10 +63,10 @@
  * Measured, device time of a whole solve: by frontier and dense rounds that
  * climb to MG / by a first form of this kernel (lanes sharing a vertex in
  * input order, 64-bit values, a barrier with a last arriver) / this one:
- * uniform game of 131,072 vertices 684 ms / 0.41 / 0.28 ms, of 16,381 at a
- * threshold 85 ms / 0.16 / 0.13 ms; power-law game of 2^20 vertices and 8.3 M
- * edges 9.3 s / 15.9 / 4.2 ms, of 6,007 59 ms / 1.25 / 0.35 ms; complete digraph
- * of 2,000 14.2 ms / 0.47 / 0.23 ms; 4-regular game of 1,000 4.1 ms / 0.11 /
+ * uniform game of 131,072 vertices 684 ms / 0.41 / 0.25 ms, of 16,381 at a
+ * threshold 85 ms / 0.16 / 0.09 ms; power-law game of 2^20 vertices and 8.3 M
+ * edges 9.3 s / 15.9 / 4.2 ms, of 6,007 59 ms / 1.25 / 0.30 ms; complete digraph
+ * of 2,000 14.2 ms / 0.47 / 0.15 ms; 4-regular game of 1,000 4.1 ms / 0.11 /
  * 0.05 ms (one CTA).
  *
  * Credits are CT integers with TOP = Lim::top while the solve runs: OMINUS(a,
@@ -80,13 +80,14 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <type_traits>
 
 namespace eg {
 
 constexpr int kBlock = 512;      /* threads of a CTA: registers for eight gathers in flight each */
 constexpr int kWarps = kBlock / 32;
 constexpr int kLightDeg = 16;    /* out-edges up to which a thread may walk a vertex */
-constexpr int kHubEdges = 256;   /* out-edges above which a vertex is cut      */
+constexpr int kHubEdges = 256;   /* out-edges above which a vertex is cut; the longest segment of most */
 constexpr int kMaxTasks = 1040;  /* segments of a CTA's cut vertices           */
 constexpr int kBins = 2 * (kLightDeg + 1);
 constexpr int kVertexBytes = 28; /* credit, potential, its copy (8 B each), id */
@@ -124,10 +125,12 @@ template <> struct Lim<long long> {
  * shared memory; KIND_GLOBAL, the grid with one or both in global memory. */
 enum { KIND_CTA, KIND_STAGED, KIND_GLOBAL };
 
-/* A CTA's vertices: slots 0 .. 32 ns - 1 hold the light ones (slice s = slots
- * 32 s ..), slots 32 ns + h the heavy ones. */
+/* A CTA's vertices: slots 0 .. V ns - 1, V = 32 >> lg, hold the light ones
+ * (slice s = slots V s .., 1 << lg lanes a vertex), slots V ns + h the heavy
+ * ones. */
 struct Range {
     int ns, s0;              /* slices; first slice of player 1              */
+    int lg, light_slots;     /* log2 of a light vertex's lanes; V ns         */
     int nh, nmed;            /* heavy vertices; those not cut (the first)    */
     int base;                /* the grid's number of slot 0                  */
     int own_smem;            /* own values, ids and offsets: shared memory   */
@@ -137,7 +140,8 @@ struct Range {
     const int *soff;         /* slices' first column << 5 | columns          */
     const int2 *E;           /* sliced edges: {successor's number, weight}   */
     const int2 *head;        /* heavy vertices: {first edge in H, edges | owner << 31} */
-    const int2 *H;           /* their edges                                  */
+    const int2 *H, *H2;      /* their edges: those that end by h_smem, the others */
+    int h_smem;
     void *g[3];              /* grid: F, D, K by number                      */
     const long long *rp;     /* the input's row offsets                      */
     int out_bits, round;     /* primal and kill sweeps between two barriers  */
@@ -240,30 +244,31 @@ __device__ __forceinline__ void finish_vertex(const Range &r, const Kind<CT> &k,
     }
 }
 
-/* U edges of each lane, `step` apart: their loads, then the gathers, then the
- * values. */
-template <typename CT, int KIND, int U>
-__device__ __forceinline__ CT walk(const int2 *E, int left, int step, const CT *g, int at_g, int sign, int mul, CT acc)
+/* Up to U columns of a slice, E at a lane's first: their loads, then the
+ * gathers, then the values.  PADS: an edge may be none (-1). */
+template <typename CT, int KIND, int U, bool PADS>
+__device__ __forceinline__ CT walk(const int2 *E, int columns, const CT *g, int at_g, int sign, int mul, CT acc)
 {
     int2 q[U];
     CT y[U];
 #pragma unroll
     for (int j = 0; j < U; j++) {
-        q[j].x = -1;
-        if (j * step < left) q[j] = E[j * step];
+        if (PADS) q[j].x = -1;
+        if (j < columns) q[j] = E[32 * j];
     }
 #pragma unroll
     for (int j = 0; j < U; j++)
-        if (q[j].x >= 0) y[j] = Mem<CT, KIND>::gather(g, at_g, q[j].x);
+        if (PADS ? q[j].x >= 0 : j < columns) y[j] = Mem<CT, KIND>::gather(g, at_g, q[j].x);
 #pragma unroll
     for (int j = 0; j < U; j++)
-        if (q[j].x >= 0) acc = min(acc, edge_value(sign, y[j], mul, q[j].y));
+        if (PADS ? q[j].x >= 0 : j < columns) acc = min(acc, edge_value(sign, y[j], mul, q[j].y));
     return acc;
 }
 
 /* Loads in flight per lane: a few for shared-memory gathers, enough to cover
  * an L2 gather for all but the longest rows. */
 template <int KIND> constexpr int kUnroll = KIND == KIND_CTA ? 2 : 8;
+constexpr int kGroupUnroll = 4; /* where lanes share a vertex, most walk no further */
 
 /* The heavy vertices of one sweep: first the segments of those that are cut,
  * then a warp per vertex of the others (the warps with the fewest slices
@@ -274,11 +279,12 @@ __device__ __forceinline__ void sweep_heavy(const Range &r, const Kind<CT> &kd, 
     using M = Mem<CT, KIND>;
     constexpr int U = kUnroll<KIND>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int slot0 = 32 * r.ns;
+    const int slot0 = r.light_slots;
     const bool hubs = r.nh > r.nmed;
     const CT *g = (const CT *)r.g[kd.mode];
     const int at_g = kd.mode * r.stride;
     int2 hd;
+    const int2 *H;
     int sign;
     CT old;
     auto open = [&](int h) {
@@ -287,13 +293,25 @@ __device__ __forceinline__ void sweep_heavy(const Range &r, const Kind<CT> &kd, 
         hd = r.head[h];
         sign = (hd.y < 0) == (kd.mode == SWEEP_PRIMAL) ? -1 : 1;
         hd.y &= INT32_MAX;
+        H = (hd.x + hd.y <= r.h_smem ? r.H : r.H2) + hd.x;
         return true;
     };
     auto lanes_min = [&](int k0, int k1) {
         CT acc = Lim<CT>::none;
 #pragma unroll 1
-        for (int k = k0 + lane; k < k1; k += 32 * U)
-            acc = walk<CT, KIND, U>(r.H + hd.x + k, k1 - k, 32, g, at_g, sign, sign * kd.mul, acc);
+        for (int k = k0 + lane; k < k1; k += 32 * U) {
+            /* past the end: the last edge again, which changes no min (a look at
+             * each edge instead: complete digraph of 2,000 183 -> 153 us without,
+             * most of it registers that were spilled) */
+            int2 q[U];
+            CT y[U];
+#pragma unroll
+            for (int j = 0; j < U; j++) q[j] = H[min(k + 32 * j, k1 - 1)];
+#pragma unroll
+            for (int j = 0; j < U; j++) y[j] = M::gather(g, at_g, q[j].x);
+#pragma unroll
+            for (int j = 0; j < U; j++) acc = min(acc, edge_value(sign, y[j], sign * kd.mul, q[j].y));
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc = min(acc, (CT)__shfl_xor_sync(0xffffffffu, acc, o));
         return acc;
@@ -329,7 +347,7 @@ __device__ __forceinline__ void sweep_heavy(const Range &r, const Kind<CT> &kd, 
 
 /* One sweep of the CTA's vertices: the light ones here, a slice per warp, a
  * vertex per lane. */
-template <typename CT, int KIND>
+template <typename CT, int KIND, bool GROUP>
 __device__ __forceinline__ void sweep(const Range &r, const Kind<CT> &kd, Hubs &hb, Count &cnt)
 {
     using M = Mem<CT, KIND>;
@@ -337,7 +355,24 @@ __device__ __forceinline__ void sweep(const Range &r, const Kind<CT> &kd, Hubs &
     const int lane = threadIdx.x & 31;
     const CT *g = (const CT *)r.g[kd.mode];
     const int at_g = kd.mode * r.stride;
-    for (int s = threadIdx.x >> 5; s < r.ns; s += kWarps) {
+    if (const int s = threadIdx.x >> 5; GROUP && s < r.ns) { /* no more slices than warps */
+        const int slot = (32 * s + lane) >> r.lg;
+        const int x = M::soff(r, s);
+        const int sign = (s >= r.s0) == (kd.mode == SWEEP_PRIMAL) ? -1 : 1;
+        const CT old = M::own(r, kd.mode, slot);
+        const bool live = old < Lim<CT>::top && old != Lim<CT>::low;
+        const int2 *E = KIND == KIND_GLOBAL ? r.E + 32 * (long long)(x >> 5) + lane
+                                            : (const int2 *)(smem + r.at_E) + 32 * (x >> 5) + lane;
+        CT acc = Lim<CT>::none;
+#pragma unroll 1
+        for (int left = live ? x & 31 : 0; left > 0; left -= kGroupUnroll, E += 32 * kGroupUnroll)
+            acc = walk<CT, KIND, kGroupUnroll, true>(E, left, g, at_g, sign, sign * kd.mul, acc);
+        __syncwarp();
+        for (int o = 1 << r.lg >> 1; o > 0; o >>= 1) acc = min(acc, (CT)__shfl_xor_sync(0xffffffffu, acc, o));
+        if (live && (lane & ((1 << r.lg) - 1)) == 0) finish_vertex<CT, KIND>(r, kd, sign, slot, old, acc, cnt);
+        __syncwarp();
+    }
+    for (int s = threadIdx.x >> 5; !GROUP && s < r.ns; s += kWarps) {
         const int slot = 32 * s + lane;
         const int x = M::soff(r, s);
         const int sign = (s >= r.s0) == (kd.mode == SWEEP_PRIMAL) ? -1 : 1;
@@ -347,8 +382,11 @@ __device__ __forceinline__ void sweep(const Range &r, const Kind<CT> &kd, Hubs &
                                             : (const int2 *)(smem + r.at_E) + 32 * (x >> 5) + lane;
         CT acc = Lim<CT>::none;
 #pragma unroll 1
-        for (int left = 32 * (x & 31); left > 0; left -= 32 * U, E += 32 * U)
-            acc = walk<CT, KIND, U>(E, left, 32, g, at_g, sign, sign * kd.mul, acc);
+        /* full batches apart: 131,072 vertices 262 -> 248 us */
+        for (int left = x & 31; left > 0; left -= U, E += 32 * U) {
+            if (left >= U) acc = walk<CT, KIND, U, false>(E, U, g, at_g, sign, sign * kd.mul, acc);
+            else acc = walk<CT, KIND, U, false>(E, left, g, at_g, sign, sign * kd.mul, acc);
+        }
         finish_vertex<CT, KIND>(r, kd, sign, slot, old, acc, cnt);
     }
     if (r.nh) sweep_heavy<CT, KIND>(r, kd, hb, cnt);
@@ -432,7 +470,7 @@ struct Turn {
 
 /* Everything after the set-up, for one credit width and kind.  Not inlined:
  * each has its registers to itself. */
-template <typename CT, int KIND>
+template <typename CT, int KIND, bool GROUP>
 __device__ __noinline__ void solve(const SweepParams *pp, const Range &rs, Hubs &hb, Turn &turn, SweepState &state,
                                    unsigned it, Count &count)
 {
@@ -440,15 +478,17 @@ __device__ __noinline__ void solve(const SweepParams *pp, const Range &rs, Hubs 
     constexpr bool GRID = KIND != KIND_CTA;
     constexpr CT top = Lim<CT>::top, low = Lim<CT>::low;
     const SweepParams &p = *pp;
-    const Range r = rs;
+    /* in registers where lanes walk long slices; the code without those is
+     * faster with them in shared memory (complete digraph 171 -> 152 us) */
+    std::conditional_t<GROUP, const Range &, const Range> r = rs;
     SweepState st = state;
     Count cnt = count;
     const int tid = threadIdx.x, lane = tid & 31;
-    const int nslots = 32 * r.ns + r.nh;
+    const int nslots = r.light_slots + r.nh;
     const bool watch = p.timeout_ns || p.cancel;
     bool ok = turn.ok != 0, mark = false;
     /* slots without a vertex are never lifted (the others start at 0) */
-    for (int i = tid; i < 32 * r.ns; i += kBlock) {
+    for (int i = tid; i < r.light_slots; i += kBlock) {
         if (M::vid(r, i) < 0) {
             M::set(r, 0, i, top);
             M::set(r, 1, i, low);
@@ -479,7 +519,7 @@ __device__ __noinline__ void solve(const SweepParams *pp, const Range &rs, Hubs 
 #pragma unroll 1
         for (int s = 0; s < ran; s++) {
             if (phase == SWEEP_PRIMAL) cnt.sweeps++;
-            sweep<CT, KIND>(r, kd, hb, cnt);
+            sweep<CT, KIND, GROUP>(r, kd, hb, cnt);
         }
         if (phase == SWEEP_PRIMAL) cnt.changes += cnt.raised;
         if (phase == SWEEP_DUAL) {
@@ -587,7 +627,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
     __shared__ SweepParams ps;
     __shared__ unsigned long long s_sum[4]; /* MG, largest |weight|; then TOPs, lifts, edges, raises */
     __shared__ int s_bin[kBins];            /* light vertices by owner and out-degree, then their next slot */
-    __shared__ int s_cls[4];                /* first slot past the light vertices of player 0; of player 1; columns; light */
+    __shared__ int s_cls[5];                /* first slot past the light vertices of player 0; of player 1; columns; light; lg */
     __shared__ int s_heavy[4];              /* heavy vertices: not cut, cut; their edges; next offset */
     __shared__ int s_scan[kWarps];
     SweepCtrl *c = p.ctrl;
@@ -600,7 +640,11 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
     const int gap = cut[2] - nv0; /* vertex i of the CTA: cut[0] + i, or gap + i from nv0 on */
     const long long e0 = p.rp[cut[0]], e1 = p.rp[cut[2]];
     const int ne = (int)(p.rp[cut[1]] - e0 + p.rp[cut[3]] - e1);
-    const int seg = max(kHubEdges, (ne / 512 + 31) & ~31); /* at most 512 + 512 segments */
+    /* Vertices of more than `cut_from` edges are cut, so that each warp has
+     * one of their segments (power-law games of 6,000 vertices: 269 -> 254 us,
+     * 412 -> 330 us against segments of 256), into at most 512 + 512 of them. */
+    const int cut_from = max(kHubEdges, (ne / 512 + 31) & ~31);
+    const int seg = ne >= 512 * kHubEdges ? cut_from : min(kHubEdges, max(64, (ne / kWarps + 31) & ~31));
     __syncthreads();
     if (tid < kBins) s_bin[tid] = 0;
     if (tid < 4) {
@@ -625,7 +669,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
             const int own1 = p.owner ? p.owner[v] != 0 : v >= p.n0;
             atomicAdd(&s_bin[own1 * (kLightDeg + 1) + deg], 1);
         } else {
-            atomicAdd(&s_heavy[deg > seg], 1);
+            atomicAdd(&s_heavy[deg > cut_from], 1);
             atomicAdd(&s_heavy[2], deg);
         }
     }
@@ -645,18 +689,39 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
                 edges += d > kLightDeg / 2 ? d * x : 0;
             }
         }
-        const bool half = ((few[0] + 31) >> 5) + ((few[1] + 31) >> 5) + s_heavy[0] + many <= kWarps;
+        /* Lanes of a light vertex: as many as leave every slice and every
+         * heavy vertex a warp of its own, and no more than it has out-edges.
+         * A sweep of a few hundred edges is one warp's chain of loads and
+         * instructions, which shared rows shorten (games of 2,000 vertices
+         * 85 -> 60 us, 5,000 112 -> 72, 16,000 118 -> 87; in one CTA, with
+         * gathers from shared memory, 2 us longer). */
+        int all[2], lg = GRID ? 3 : 0, most = 0;
+        for (int o = 0; o < 2; o++) {
+            all[o] = 0;
+            for (int d = 0; d <= kLightDeg; d++) {
+                const int x = s_bin[o * (kLightDeg + 1) + d];
+                all[o] += x;
+                if (x) most = max(most, d);
+            }
+        }
+        while (lg && ((1 << lg >> 1) >= most ||
+                      ((all[0] + (31 >> lg)) >> (5 - lg)) + ((all[1] + (31 >> lg)) >> (5 - lg)) + s_heavy[0] > kWarps))
+            lg--;
+        const bool half = !lg && ((few[0] + 31) >> 5) + ((few[1] + 31) >> 5) + s_heavy[0] + many <= kWarps;
         const int light = half ? kLightDeg / 2 : kLightDeg;
         __syncwarp(3u);
         if (half && tid == 0) {
             s_heavy[0] += many;
             s_heavy[2] += edges;
         }
-        if (tid == 0) s_cls[3] = light;
+        if (tid == 0) {
+            s_cls[3] = light;
+            s_cls[4] = lg;
+        }
         /* the first slot of every (owner, out-degree); player 1's start a slice */
         int total0 = 0;
         for (int d = 0; d <= light; d++) total0 += s_bin[d];
-        int at = tid ? (total0 + 31) & ~31 : 0;
+        int at = tid ? (total0 + (31 >> lg)) & ~(31 >> lg) : 0;
         __syncwarp(3u);
         for (int d = 0; d <= light; d++) {
             const int k = tid * (kLightDeg + 1) + d, x = s_bin[k];
@@ -666,11 +731,11 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
         s_cls[tid] = at;
     }
     __syncthreads();
-    const int light = s_cls[3];
+    const int light = s_cls[3], lg = s_cls[4], V = 32 >> lg;
     const int nmed = s_heavy[0], nh = nmed + s_heavy[1], he = s_heavy[2];
     /* 2. shared memory: own values, ids, slice offsets; then sliced edges;
      * then heavy ones -- what does not fit is in global memory */
-    const int s0 = (s_cls[0] + 31) >> 5, ns = (s_cls[1] + 31) >> 5, nslots = 32 * ns + nh;
+    const int s0 = (s_cls[0] + V - 1) >> (5 - lg), ns = (s_cls[1] + V - 1) >> (5 - lg), nslots = V * ns + nh;
     const int stride = 8 * nslots;
     const int base = GRID ? cut[0] + cut[2] - split + kPadSlots * (int)blockIdx.x : 0;
     long long at = 28LL * nslots + 4LL * ns;
@@ -693,8 +758,9 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
             int W = 0;
             if (s < ns) {
                 const int own1 = s >= s0;
-                const int last = min(32 * s + 31, s_cls[own1] - 1);
+                const int last = min(V * s + V - 1, s_cls[own1] - 1);
                 for (int d = 1; d <= light; d++) W += s_bin[own1 * (kLightDeg + 1) + d] <= last;
+                W = (W + (1 << lg) - 1) >> lg;
             }
             int x = W;
 #pragma unroll
@@ -715,7 +781,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
         }
         if (tid == 0) s_cls[2] = run;
     }
-    for (int i = tid; i < 32 * ns; i += kBlock) vid[i] = -1;
+    for (int i = tid; i < V * ns; i += kBlock) vid[i] = -1;
     if (own_smem)
         for (int i = tid; i < 2 * nslots; i += kBlock) ((long long *)smem)[i] = 0;
     if (GRID) {
@@ -729,16 +795,21 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
     const long long ell = 32LL * s_cls[2]; /* edges with pads */
     const int at_E = (int)at;
     const bool edges_smem = at + 8 * ell <= p.smem_bytes;
-    const bool heavy_smem = at + 8 * (ell + nh + he) <= p.smem_bytes;
+    /* the heavy ones as far as they fit (complete digraph of 2,000, whose parts
+     * are 3% too large: 217 -> 197 us against none) */
+    const bool heavy_smem = at + 8 * (ell + nh) <= p.smem_bytes;
+    const int h_smem = heavy_smem ? (int)min((p.smem_bytes - at) / 8 - ell - nh, (long long)he) : he;
     int2 *E, *rest = nullptr; /* where the sliced edges are, and the heavy heads and edges */
     int2 *out_of_smem = p.E + (e0 + e1 - p.rp[split]) + ((e0 + e1 - p.rp[split]) >> 4) + kPadEdges * (long long)blockIdx.x;
     E = edges_smem ? (int2 *)(smem + at) : out_of_smem;
     rest = heavy_smem ? (int2 *)(smem + at) + ell : edges_smem ? out_of_smem : out_of_smem + ell;
-    int2 *head = rest, *H = rest + nh;
+    int2 *head = rest, *H = rest + nh, *H2 = heavy_smem && edges_smem ? out_of_smem : H;
     if (tid < 2) s_heavy[tid] = 0;
     if (tid == 0) {
         ps = p;
         r.ns = ns;
+        r.lg = lg;
+        r.light_slots = V * ns;
         r.s0 = s0;
         r.nh = nh;
         r.nmed = nmed;
@@ -753,6 +824,8 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
         r.E = E;
         r.head = head;
         r.H = H;
+        r.H2 = H2;
+        r.h_smem = h_smem;
         r.g[0] = p.F;
         r.g[1] = p.D;
         r.g[2] = p.K;
@@ -771,9 +844,9 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
         if (deg <= light) {
             slot = atomicAdd(&s_bin[own1 * (kLightDeg + 1) + deg], 1);
         } else {
-            const int hub = deg > seg;
+            const int hub = deg > cut_from;
             const int h = (hub ? nmed : 0) + atomicAdd(&s_heavy[hub], 1);
-            slot = 32 * ns + h;
+            slot = V * ns + h;
             head[h] = make_int2(atomicAdd(&s_heavy[3], deg), (int)((unsigned)deg | (unsigned)own1 << 31));
             if (hub) {
                 const int nt = (deg + seg - 1) / seg, t0 = atomicAdd(&hb.tasks, nt), k = h - nmed;
@@ -798,7 +871,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
     unsigned wmax = 0u;
     if (turn.ok) {
         for (int s = warp; s < ns; s += kWarps) {
-            const int v = vid[32 * s + lane], b = soff[s] >> 5, W = soff[s] & 31;
+            const int v = vid[(32 * s + lane) >> lg], sub = lane & ((1 << lg) - 1), b = soff[s] >> 5, W = soff[s] & 31;
             long long k0 = 0;
             int deg = 0, lo = INT32_MAX, hi = INT32_MIN;
             if (v >= 0) {
@@ -809,35 +882,59 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
             for (int j0 = 0; j0 < W; j0 += 8) {
                 int2 q[8];
 #pragma unroll
-                for (int j = 0; j < 8; j++)
-                    q[j] = j0 + j < deg ? make_int2(__ldg(p.succ + k0 + j0 + j), __ldg(p.w + k0 + j0 + j)) : make_int2(-1, 0);
+                for (int j = 0; j < 8; j++) {
+                    /* pads: a lane's last edge again, which changes no min and
+                     * spares the walk a look; none where lanes share a vertex,
+                     * whose pads are more */
+                    const int k = lg ? ((j0 + j) << lg) + sub : max(0, min(j0 + j, deg - 1));
+                    q[j] = make_int2(-1, 0);
+                    if (j0 + j < W && k < deg) q[j] = make_int2(__ldg(p.succ + k0 + k), __ldg(p.w + k0 + k));
+                }
 #pragma unroll
                 for (int j = 0; j < 8; j++)
-                    if (j0 + j < deg) q[j].x = GRID ? __ldcg(number + q[j].x) : number[q[j].x];
+                    if (q[j].x >= 0) q[j].x = GRID ? __ldcg(number + q[j].x) : number[q[j].x];
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
-                    if (j0 + j < deg) {
+                    if (j0 + j >= W) continue;
+                    out[32 * (j0 + j)] = q[j];
+                    if (q[j].x >= 0) {
                         lo = min(lo, q[j].y);
                         hi = max(hi, q[j].y);
                     }
-                    if (j0 + j < W) out[32 * (j0 + j)] = q[j];
                 }
             }
+            for (int o = 1 << lg >> 1; o > 0; o >>= 1) {
+                lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+                hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+            }
             if (deg > 0) {
-                if (lo < 0) mg_sum += (unsigned long long)(-(long long)lo);
+                if (lo < 0 && sub == 0) mg_sum += (unsigned long long)(-(long long)lo);
                 wmax = max(wmax, max(lo < 0 ? 0u - (unsigned)lo : (unsigned)lo, hi < 0 ? 0u - (unsigned)hi : (unsigned)hi));
             }
         }
         /* the heavy ones a warp each, the cut ones a warp per segment */
         auto copy = [&](int h, int k0, int k1) {
-            const long long from = p.rp[vid[32 * ns + h]];
+            const long long from = p.rp[vid[V * ns + h]];
             const int2 hd = head[h];
+            int2 *const to = (hd.x + (hd.y & INT32_MAX) <= h_smem ? H : H2) + hd.x;
             int lo = INT32_MAX, hi = INT32_MIN;
-            for (int k = k0 + lane; k < k1; k += 32) {
-                const int x = __ldg(p.succ + from + k), w = __ldg(p.w + from + k);
-                H[hd.x + k] = make_int2(GRID ? __ldcg(number + x) : number[x], w);
-                lo = min(lo, w);
-                hi = max(hi, w);
+#pragma unroll 1
+            for (int k = k0 + lane; k < k1; k += 256) {
+                int2 q[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    q[j] = k + 32 * j < k1 ? make_int2(__ldg(p.succ + from + k + 32 * j), __ldg(p.w + from + k + 32 * j))
+                                           : make_int2(-1, 0);
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (q[j].x >= 0) q[j].x = GRID ? __ldcg(number + q[j].x) : number[q[j].x];
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    if (k + 32 * j >= k1) continue;
+                    to[k + 32 * j] = q[j];
+                    lo = min(lo, q[j].y);
+                    hi = max(hi, q[j].y);
+                }
             }
             lo = __reduce_min_sync(0xffffffffu, lo);
             hi = __reduce_max_sync(0xffffffffu, hi);
@@ -911,16 +1008,18 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
     }
     Count cnt = {0u, 0u, 0ull, 0ull, 0ull};
     __syncthreads();
-    if (!GRID) {
-        if (fits32) solve<int, KIND_CTA>(&ps, r, hb, turn, st, it, cnt);
-        else solve<long long, KIND_CTA>(&ps, r, hb, turn, st, it, cnt);
-    } else if (own_smem && edges_smem) {
-        if (fits32) solve<int, KIND_STAGED>(&ps, r, hb, turn, st, it, cnt);
-        else solve<long long, KIND_STAGED>(&ps, r, hb, turn, st, it, cnt);
-    } else {
-        if (fits32) solve<int, KIND_GLOBAL>(&ps, r, hb, turn, st, it, cnt);
-        else solve<long long, KIND_GLOBAL>(&ps, r, hb, turn, st, it, cnt);
-    }
+    auto run = [&](auto credit, auto kind) {
+        using CT = decltype(credit);
+        if (GRID && (lg || !ns)) solve<CT, decltype(kind)::value, GRID>(&ps, r, hb, turn, st, it, cnt);
+        else solve<CT, decltype(kind)::value, false>(&ps, r, hb, turn, st, it, cnt);
+    };
+    auto run_kind = [&](auto kind) {
+        if (fits32) run(0, kind);
+        else run(0ll, kind);
+    };
+    if (!GRID) run_kind(std::integral_constant<int, KIND_CTA>());
+    else if (own_smem && edges_smem) run_kind(std::integral_constant<int, KIND_STAGED>());
+    else run_kind(std::integral_constant<int, KIND_GLOBAL>());
     unsigned long long sums[4] = {cnt.raised, cnt.lifts, cnt.edges, cnt.changes};
 #pragma unroll
     for (int k = 0; k < 4; k++) {

@@ -128,3 +128,20 @@ def test_hand_over_to_frontier_rounds():
     ref[length - 1::length] = 0
     np.testing.assert_array_equal(f, ref)
     assert st.rounds > 512 and st.num_top == 0
+
+
+# on 37 CTAs 8 lanes share a vertex up to 2,368 vertices, 4 up to 4,736, 2 up
+# to 9,472 (some parts differ by a vertex); complete digraphs whose edges fit
+# 148 CTAs' shared memory, do but for a vertex each, and do not
+@pytest.mark.parametrize("kind,n,deg,ctas", [(4, n, 16, 37) for n in (2000, 2368, 2400, 4736, 4800, 9400, 9700)] +
+                         [(5, 3500, 30, 37), (1, 4000, 4, 37)] + [(3, n, n - 1, 0) for n in (1930, 2000, 2200)])
+def test_lanes_that_share_a_vertex(kind, n, deg, ctas):
+    g = eg.generate(kind, n, deg, 40, 5 + n, param=2 if kind == 4 else 6)
+    f, st = eg.solve(g, grid_ctas=ctas)
+    assert st.grid == (ctas or 148)
+    np.testing.assert_array_equal(f, want(g))
+    if g.num_edges < 50000:
+        rng = np.random.default_rng(n)
+        g = eg.Game(row_ptr=g.row_ptr, succ=g.succ, weight=g.weight * 40000, owner=rng.integers(0, 2, n).astype(np.uint8))
+        f, _ = eg.solve(g, grid_ctas=ctas)
+        np.testing.assert_array_equal(f, want(g))
