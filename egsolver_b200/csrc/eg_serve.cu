@@ -116,7 +116,7 @@ struct Launch {
     int stream;
     int64_t number = 0;
     int units = 0;
-    cudaEvent_t ev = nullptr;
+    Lane *lane = nullptr;       /* its first event: the end; its page: the control block by then */
     std::vector<int64_t> qids;
     void *block = nullptr;      /* device memory of what follows              */
     UnitDesc *dunits = nullptr;
@@ -189,26 +189,41 @@ void drop_resident(eg_server *s, ServedGame &g)
     g.resident = false;
 }
 
-/* Frees resident games nobody uses, oldest first, until `need` bytes fit. */
-bool make_room(eg_server *s, size_t need)
+/* Drops the resident game that nobody uses and that was used longest ago. */
+bool evict_one(eg_server *s)
 {
-    for (;;) {
+    ServedGame *victim = nullptr;
+    for (auto &kv : s->games) {
+        ServedGame &g = *kv.second;
+        if (g.resident && g.active == 0 && (!victim || g.last_use < victim->last_use)) victim = &g;
+    }
+    if (!victim) return false;
+    drop_resident(s, *victim);
+    s->evictions++;
+    return true;
+}
+
+/* Makes room for `need` bytes above the reserve.  *left is what the last look
+ * found, less what was taken since: a look takes 65 us, most of an admission,
+ * and one serves the queries that are admitted together. */
+bool make_room(eg_server *s, std::unique_lock<std::mutex> &lk, size_t need, size_t *left)
+{
+    while (*left < need) {
         size_t free_b = 0, total_b = 0;
-        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+        lk.unlock();
+        const cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
+        lk.lock();
+        if (e != cudaSuccess) {
             cudaGetLastError();
             return false;
         }
         const size_t reserve = (size_t)s->o.hbm_reserve_bytes;
-        if (free_b > reserve && free_b - reserve >= need) return true;
-        ServedGame *victim = nullptr;
-        for (auto &kv : s->games) {
-            ServedGame &g = *kv.second;
-            if (g.resident && g.active == 0 && (!victim || g.last_use < victim->last_use)) victim = &g;
-        }
-        if (!victim) return false;
-        drop_resident(s, *victim);
-        s->evictions++;
+        *left = free_b > reserve ? free_b - reserve : 0;
+        if (*left < need && !evict_one(s)) return false;
+        if (*left < need) *left = 0;
     }
+    *left -= need;
+    return true;
 }
 
 void finish_query(eg_server *s, Query &q, eg_status st, clk::time_point now)
@@ -226,35 +241,89 @@ void finish_query(eg_server *s, Query &q, eg_status st, clk::time_point now)
     s->latencies.push_back(ms_since(q.t_submit, now));
 }
 
-/* Completion of finished micro-batches (lock held). */
-bool reap(eg_server *s)
+/* The control block to the launch's page, then its event. */
+cudaError_t mark_end(Launch &l, cudaStream_t st)
+{
+    const cudaError_t e = cudaMemcpyAsync(l.lane->page, l.dctrl, sizeof(LaunchCtrl), cudaMemcpyDeviceToHost, st);
+    return e == cudaSuccess ? cudaEventRecord(l.lane->ev[0], st) : e;
+}
+
+/* A query's credits, rounds and status to the host. */
+eg_status fetch(eg_server *s, Query &q, int n, cudaStream_t st)
+{
+    const size_t nu = q.units.size();
+    q.result_len = (size_t)n * q.K;
+    q.result.reset(new int64_t[q.result_len]);
+    const size_t bytes = sizeof(long long) * q.result_len;
+    std::vector<char> tail(q.o_end - q.o_rounds); /* rounds and status lie behind one another */
+    cudaError_t e;
+    if (q.o_end <= kStageBlock) { /* all in one copy */
+        e = copy_block_to_host(q.dF, q.o_end, s->o.device, st, [&](const char *b) {
+            memcpy(q.result.get(), b, bytes);
+            memcpy(tail.data(), b + q.o_rounds, tail.size());
+        });
+    } else {
+        e = copy_to_host(q.result.get(), q.dF, bytes, s->o.device, st);
+        if (e == cudaSuccess) e = copy_to_host(tail.data(), q.drounds, tail.size(), s->o.device, st);
+    }
+    if (e != cudaSuccess) return EG_ERR_CUDA;
+    const long long *rr = (const long long *)tail.data();
+    const int *ss = (const int *)(tail.data() + (q.o_status - q.o_rounds));
+    eg_status r = EG_OK;
+    q.rounds = 0;
+    for (size_t u = 0; u < nu; u++) {
+        q.rounds = std::max(q.rounds, rr[u]);
+        if (r == EG_OK && ss[u] != EG_OK) r = (eg_status)ss[u];
+    }
+    return r;
+}
+
+/* Completion of finished micro-batches (lock held; released around the
+ * copies, as around every call to the device: a submit that had to wait for
+ * them took 200 us, and its query then missed the launch of the others).
+ * Admitted queries and their games are erased by nobody else. */
+bool reap(eg_server *s, std::unique_lock<std::mutex> &lk)
 {
     bool any = false;
     for (size_t i = 0; i < s->inflight.size();) {
         Launch &l = s->inflight[i];
-        cudaError_t e = cudaEventQuery(l.ev);
+        cudaStream_t st = s->streams[l.stream];
+        cudaError_t e = cudaEventQuery(l.lane->ev[0]);
         if (e == cudaErrorNotReady) {
             i++;
             continue;
         }
         any = true;
         const clk::time_point now = clk::now();
+        std::vector<std::pair<Query *, ServedGame *>> qs;
+        for (int64_t qid : l.qids) qs.push_back({s->queries[qid].get(), s->games[s->queries[qid]->game].get()});
         UnitCtrl c;
         LaunchCtrl cv;
         memset(&c, 0, sizeof c);
-        const bool have = e == cudaSuccess && copy_to_host(&cv, l.dctrl, sizeof cv, s->o.device, s->streams[l.stream]) == cudaSuccess;
+        const bool have = e == cudaSuccess;
+        if (have) memcpy(&cv, l.lane->page, sizeof cv);
+        lk.unlock();
         if (have && !l.in_tail && tail_entries(l.set, cv) > 0) {
             /* some units went to the tail: its kernels run now */
-            cudaStream_t st = s->streams[l.stream];
             if (launch_tail(s->launchers[(size_t)l.stream], st, l.set, l.dunits, l.tl, l.dscratch, l.dctrl, s->sms,
                             s->o.max_rounds, 0) == EG_OK &&
-                cudaEventRecord(l.ev, st) == cudaSuccess) {
+                mark_end(l, st) == cudaSuccess) {
                 l.in_tail = true;
                 i++;
+                lk.lock();
                 continue;
             }
             e = cudaErrorLaunchFailure;
         }
+        std::vector<eg_status> status;
+        for (auto &x : qs) {
+            status.push_back(e == cudaSuccess ? fetch(s, *x.first, x.second->n, st) : EG_ERR_CUDA);
+            free_query_device(*x.first, st);
+        }
+        if (e != cudaSuccess) cudaStreamSynchronize(st);
+        lane_give(l.lane);
+        pool_free(l.block, st);
+        lk.lock();
         if (have) {
             sum_ctrl(cv, &c);
             if (!s->clock0) s->clock0 = c.t_begin;
@@ -267,50 +336,32 @@ bool reap(eg_server *s)
             sp.end_ms = ((double)c.t_end - (double)s->clock0) * 1e-6;
             s->spans.push_back(sp);
         }
-        for (int64_t qid : l.qids) {
-            Query &q = *s->queries[qid];
-            ServedGame &g = *s->games[q.game];
-            eg_status st = e == cudaSuccess ? EG_OK : EG_ERR_CUDA;
-            if (st == EG_OK) {
-                const size_t nu = q.units.size();
-                /* rounds and status lie behind one another in the block */
-                std::vector<char> tail(q.o_end - q.o_rounds);
-                q.result_len = (size_t)g.n * q.K;
-                q.result.reset(new int64_t[q.result_len]);
-                cudaStream_t qs = s->streams[l.stream];
-                cudaError_t cp = copy_to_host(q.result.get(), q.dF, sizeof(long long) * q.result_len, s->o.device, qs);
-                if (cp == cudaSuccess) cp = copy_to_host(tail.data(), q.drounds, tail.size(), s->o.device, qs);
-                const long long *rr = (const long long *)tail.data();
-                const int *ss = (const int *)(tail.data() + (q.o_status - q.o_rounds));
-                if (cp != cudaSuccess) {
-                    st = EG_ERR_CUDA;
-                } else {
-                    q.rounds = 0;
-                    for (size_t u = 0; u < nu; u++) {
-                        q.rounds = std::max(q.rounds, rr[u]);
-                        if (st == EG_OK && ss[u] != EG_OK) st = (eg_status)ss[u];
-                    }
-                }
-            }
-            s->device_bytes -= (int64_t)q.dbytes;
-            free_query_device(q, s->streams[l.stream]);
-            g.active--;
+        for (size_t k = 0; k < qs.size(); k++) {
+            s->device_bytes -= (int64_t)qs[k].first->dbytes;
+            qs[k].second->active--;
             s->admitted_now--;
-            finish_query(s, q, st, now);
+            finish_query(s, *qs[k].first, status[k], now);
         }
-        cudaEventDestroy(l.ev);
-        pool_free(l.block, s->streams[l.stream]);
         s->inflight.erase(s->inflight.begin() + (long)i);
     }
     if (any) s->cv_done.notify_all();
     return any;
 }
 
-/* Admission in submission order (lock held; releases it around uploads). */
+/* Admission of the queries at hand, in submission order (lock held; released
+ * around calls to the device). */
 bool admit(eg_server *s, std::unique_lock<std::mutex> &lk)
 {
     bool any = false;
-    while (!s->pending.empty() && s->admitted_now < s->o.max_inflight) {
+    size_t left = 0;
+    /* The rest of a burst is submitted meanwhile, so a few more are taken
+     * than are there: 12 queries of 6 thresholds on games of 1000-8000 nodes,
+     * submitted at once, end after 1.03-1.08 ms with 6, 1.23-1.33 with 4,
+     * 1.29-1.44 with 12 (2.4 ms when each admission kept the lock, looked at the
+     * device's memory and copied on its own). */
+    size_t taken = 0;
+    const size_t most = std::max<size_t>(s->pending.size(), 6);
+    for (; !s->pending.empty() && taken < most && s->admitted_now < s->o.max_inflight; taken++) {
         const int64_t qid = s->pending.front();
         Query &q = *s->queries[qid];
         ServedGame &g = *s->games[q.game];
@@ -353,7 +404,7 @@ bool admit(eg_server *s, std::unique_lock<std::mutex> &lk)
         const size_t qbytes = query_bytes(g, q.K, scratch) + units.size() * 16;
         size_t need = qbytes;
         if (!g.resident) need += packed_dev_bytes(g.hp);
-        if (!make_room(s, need)) {
+        if (!make_room(s, lk, need, &left)) {
             if (s->admitted_now == 0 && s->inflight.empty()) { /* can never fit */
                 s->pending.pop_front();
                 finish_query(s, q, EG_ERR_OOM, clk::now());
@@ -399,7 +450,12 @@ bool admit(eg_server *s, std::unique_lock<std::mutex> &lk)
         const size_t o_scr = o_status + ((nu * sizeof(int) + 255) & ~(size_t)255);
         const size_t total = o_scr + scratch;
         char *blk = nullptr;
-        if (pool_alloc((void **)&blk, total, s->o.device, s->upload_stream) != cudaSuccess) break;
+        lk.unlock();
+        const cudaError_t ae = pool_alloc((void **)&blk, total, s->o.device, s->upload_stream);
+        if (ae != cudaSuccess) {
+            lk.lock();
+            break;
+        }
         q.dF = (long long *)blk;
         q.dthr = (int *)(blk + o_thr);
         q.dmg = (long long *)(blk + o_mg);
@@ -435,6 +491,7 @@ bool admit(eg_server *s, std::unique_lock<std::mutex> &lk)
         cudaError_t ce = copy_parts_to_device(q.dthr, parts, 2, o_mg - o_thr + parts[1].bytes, s->o.device, s->upload_stream);
         if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&q.ready, cudaEventDisableTiming);
         if (ce == cudaSuccess) ce = cudaEventRecord(q.ready, s->upload_stream);
+        lk.lock();
         if (ce != cudaSuccess) {
             cudaGetLastError();
             free_query_device(q, s->upload_stream);
@@ -458,15 +515,14 @@ bool admit(eg_server *s, std::unique_lock<std::mutex> &lk)
 }
 
 /* Device side of one micro-batch of the queries l.qids, up to its launch
- * (lock held). */
-eg_status prepare_batch(eg_server *s, Launch &l)
+ * (lock not held). */
+eg_status prepare_batch(eg_server *s, Launch &l, const std::vector<Query *> &qs)
 {
     std::vector<UnitDesc> all;
     std::vector<long long> cost;
-    for (int64_t qid : l.qids) {
-        Query &q = *s->queries[qid];
-        all.insert(all.end(), q.units.begin(), q.units.end());
-        cost.insert(cost.end(), q.cost.begin(), q.cost.end());
+    for (Query *q : qs) {
+        all.insert(all.end(), q->units.begin(), q->units.end());
+        cost.insert(cost.end(), q->cost.begin(), q->cost.end());
     }
     UnitSet &S = l.set;
     group_units(all, cost, std::vector<size_t>(all.size(), 0), &S, nullptr);
@@ -474,7 +530,7 @@ eg_status prepare_batch(eg_server *s, Launch &l)
     l.units = (int)S.units.size();
     s->next_stream = (s->next_stream + 1) % s->o.streams;
     cudaStream_t st = s->streams[l.stream];
-    for (int64_t qid : l.qids) cudaStreamWaitEvent(st, s->queries[qid]->ready, 0);
+    for (Query *q : qs) cudaStreamWaitEvent(st, q->ready, 0);
     const size_t tsb = tail_scratch_bytes(S, s->sms);
     const size_t ub = (sizeof(UnitDesc) * S.units.size() + 255) & ~(size_t)255;
     const size_t cb = (sizeof(LaunchCtrl) + 255) & ~(size_t)255, tb = (tail_bytes(S) + 255) & ~(size_t)255;
@@ -485,27 +541,33 @@ eg_status prepare_batch(eg_server *s, Launch &l)
     l.dctrl = (LaunchCtrl *)(at + ub);
     if (tsb) l.dscratch = at + ub + cb + tb;
     e = copy_to_device(l.dunits, S.units.data(), sizeof(UnitDesc) * S.units.size(), s->o.device, st);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&l.ev, cudaEventDisableTiming);
     if (e != cudaSuccess) return EG_ERR_CUDA;
+    l.lane = lane_take(s->o.device);
+    if (!l.lane) return EG_ERR_CUDA;
     return tail_upload(S, at + ub + cb, st, &l.tl);
 }
 
-/* Launches a prepared micro-batch, or fails its queries (lock held). */
-void start_batch(eg_server *s, Launch &l, eg_status ls)
+/* Launches a prepared micro-batch (lock not held). */
+eg_status start_batch(eg_server *s, Launch &l)
 {
     cudaStream_t st = s->streams[l.stream];
-    cudaError_t e = cudaSuccess;
+    int grid = 0;
+    eg_status ls = launch_units(s->launchers[(size_t)l.stream], st, l.set, l.dunits, l.tl, l.dctrl, s->o.block, s->sms,
+                                s->o.max_rounds, 0, &grid);
+    if (ls == EG_OK && mark_end(l, st) != cudaSuccess) ls = EG_ERR_CUDA;
+    if (ls != EG_OK) cudaStreamSynchronize(st); /* nothing may write the lane's page any more */
+    return ls;
+}
+
+/* A micro-batch under way, or the end of its queries (lock held). */
+void account_batch(eg_server *s, Launch &l, eg_status ls)
+{
     if (ls == EG_OK) {
-        int grid = 0;
-        ls = launch_units(s->launchers[(size_t)l.stream], st, l.set, l.dunits, l.tl, l.dctrl, s->o.block, s->sms,
-                          s->o.max_rounds, 0, &grid);
-        if (ls == EG_OK) e = cudaEventRecord(l.ev, st);
-    }
-    if (e == cudaSuccess && ls == EG_OK) {
         l.number = s->micro_batches++;
         s->inflight.push_back(std::move(l));
         return;
     }
+    cudaStream_t st = s->streams[l.stream];
     cudaGetLastError();
     const clk::time_point now = clk::now();
     for (int64_t qid : l.qids) {
@@ -514,18 +576,18 @@ void start_batch(eg_server *s, Launch &l, eg_status ls)
         free_query_device(q, st);
         s->games[q.game]->active--;
         s->admitted_now--;
-        finish_query(s, q, ls != EG_OK ? ls : EG_ERR_CUDA, now);
+        finish_query(s, q, ls, now);
     }
-    if (l.ev) cudaEventDestroy(l.ev);
+    lane_give(l.lane);
     pool_free(l.block, st);
     s->cv_done.notify_all();
 }
 
-/* Launches the admitted queries (lock held): in two micro-batches where two
+/* Launches the admitted queries (lock held, but not during it): in two micro-batches where two
  * streams are free, the queries dealt heaviest first, so that the first's
  * read-back overlaps the second's run.  Both are prepared before the first
  * is launched: they start a kernel launch apart. */
-bool launch_ready(eg_server *s)
+bool launch_ready(eg_server *s, std::unique_lock<std::mutex> &lk)
 {
     const int free_streams = s->o.streams - (int)s->inflight.size();
     if (s->ready.empty() || free_streams <= 0) return false;
@@ -539,12 +601,18 @@ bool launch_ready(eg_server *s)
     std::stable_sort(ready.begin(), ready.end(), [&](int64_t a, int64_t b) { return cost_of(a) > cost_of(b); });
     const size_t parts = std::min<size_t>({2, (size_t)free_streams, ready.size()});
     std::vector<Launch> ls(parts);
-    std::vector<eg_status> prep(parts, EG_OK);
-    for (size_t k = 0; k < parts; k++) {
-        for (size_t i = k; i < ready.size(); i += parts) ls[k].qids.push_back(ready[i]);
-        prep[k] = prepare_batch(s, ls[k]);
+    std::vector<eg_status> done(parts, EG_OK);
+    std::vector<std::vector<Query *>> qs(parts);
+    for (size_t i = 0; i < ready.size(); i++) {
+        ls[i % parts].qids.push_back(ready[i]);
+        qs[i % parts].push_back(s->queries[ready[i]].get());
     }
-    for (size_t k = 0; k < parts; k++) start_batch(s, ls[k], prep[k]);
+    lk.unlock();
+    for (size_t k = 0; k < parts; k++) done[k] = prepare_batch(s, ls[k], qs[k]);
+    for (size_t k = 0; k < parts; k++)
+        if (done[k] == EG_OK) done[k] = start_batch(s, ls[k]);
+    lk.lock();
+    for (size_t k = 0; k < parts; k++) account_batch(s, ls[k], done[k]);
     return true;
 }
 
@@ -555,9 +623,9 @@ void worker_main(eg_server *s)
     cudaSetDevice(s->o.device);
     std::unique_lock<std::mutex> lk(s->mu);
     for (;;) {
-        bool progress = reap(s);
+        bool progress = reap(s, lk);
         progress |= admit(s, lk);
-        progress |= launch_ready(s);
+        progress |= launch_ready(s, lk);
         if (s->stop && s->pending.empty() && s->ready.empty() && s->inflight.empty()) break;
         if (progress) {
             quiet = 0;

@@ -164,3 +164,52 @@ def test_unknown_game_and_bad_arguments():
         gid = srv.add_game(mixed_games(1)[0])
         with pytest.raises(eg.EGError):
             srv.submit(gid, np.zeros(40, np.int32))  # K > 32
+
+
+@pytest.mark.parametrize("n", [8176, 8180, 9000])
+def test_results_at_the_edge_of_one_copy(n):
+    """A query's block of credits, thresholds, rounds and status: just within
+    the 512 KB that one copy reads, and just past them."""
+    g = eg.generate(1, n, 4, 20, n)
+    p = np.array([-90, -40, -9, -3, 0, 5, 33, 88], np.int32)
+    with eg.Server() as srv:
+        gid = srv.add_game(g)
+        qids = [srv.submit(gid, p + i, 4) for i in range(3)]
+        for i, q in enumerate(qids):
+            srv.wait(q, 120_000)
+            got, _ = srv.result(q)
+            np.testing.assert_array_equal(got, alone(g, p + i, 4))
+
+
+def test_threads_submit_while_queries_run():
+    import threading
+
+    games = mixed_games(6, seed=3)
+    want = {}
+    for i, g in enumerate(games):
+        for r in range(4):
+            p = np.array([-9 + r, 0, 7 * r], np.int32)
+            want[i, r] = (p, alone(g, p, 8))
+    errors = []
+    with eg.Server(streams=3) as srv:
+        gids = [srv.add_game(g) for g in games]
+
+        def client(r):
+            try:
+                for _ in range(3):
+                    qids = [srv.submit(gids[i], want[i, r][0], 8) for i in range(len(games))]
+                    extra = srv.add_game(games[r])
+                    srv.wait(srv.submit(extra, want[r, r][0], 8), 120_000)
+                    for i, q in enumerate(qids):
+                        srv.wait(q, 120_000)
+                        np.testing.assert_array_equal(srv.result(q)[0], want[i, r][1])
+            except Exception as e:  # reported by the main thread
+                errors.append(e)
+
+        ts = [threading.Thread(target=client, args=(r,)) for r in range(4)]
+        for t in ts:
+            t.start()
+        for t in ts:
+            t.join()
+        assert not errors, errors
+        assert srv.stats()["completed"] == 4 * 3 * 7
