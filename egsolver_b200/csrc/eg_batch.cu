@@ -1,6 +1,6 @@
 /*
  * eg_batch.cu -- batched solving of many games at K mean-payoff thresholds
- * in one persistent launch.
+ * in one solve.
  *
  * Work is cut into units: a game at a group of 1, 2, 4 or 8 of its
  * thresholds (weights w * d - p_k).  One CTA solves one unit at a time,

@@ -9,18 +9,19 @@
  *      their queries (device -> host) and release the queries' buffers;
  *   2. admission, in submission order: a query is admitted when fewer than
  *      max_inflight queries are admitted and the free device memory (from
- *      cudaMemGetInfo) minus hbm_reserve_bytes covers its credits and, if
- *      its game is not resident yet, the game's packed layout; idle resident
- *      games are evicted oldest-first when memory is short.  A game stays
- *      resident across all its queries until it is evicted or removed;
+ *      cudaMemGetInfo, less what queries admitted since that look take) minus
+ *      hbm_reserve_bytes covers its credits and, if its game is not resident
+ *      yet, the game's packed layout; idle resident games are evicted
+ *      oldest-first when memory is short.  A game stays resident across all
+ *      its queries until it is evicted or removed;
  *   3. launch: the admitted queries not yet launched go into one or two
  *      micro-batches, i.e. launches of the unit kernels (eg_batch.cu: one CTA
  *      per game x threshold group, credits in shared memory), each on the next
  *      of `streams` streams.  A micro-batch some of whose units went to the
- *      cluster tail gets its tail launched when its units have ended.  Earlier micro-batches keep running; as their CTAs
- *      run out of units and exit, the new launch's CTAs take the freed SMs,
- *      so the work of queries that arrived at different times overlaps on
- *      the device.  Each launch records its first CTA start and last CTA end
+ *      cluster tail gets its tail launched when its units have ended.
+ *      Earlier micro-batches keep running; as their CTAs run out of units and
+ *      exit, the new launch's CTAs take the freed SMs, so the work of queries
+ *      that arrived at different times overlaps on the device.  Each launch records its first CTA start and last CTA end
  *      on the device clock (eg_serve_trace).
  *
  * Routing: games above the batched layout's limit (2^19 vertices), and games
