@@ -8,20 +8,21 @@ floor of a continuous x^-2 power law on [1, 4097) (mean 7.9, m = 8.28M),
 successors uniform without self-loops or duplicates, weights uniform in
 [-1000, 1000], 64-bit credits; seeded (seed 0xE6 + 2), synthetic.
 
-A step is one complete solve from f = 0: transpose and renumbering,
-initial frontier, the persistent lifting kernels (frontier rounds, then
-dense rounds over every vertex) until the least fixed point.
-  value  GTEPS = out-edges scanned by lifts / device time of the solve, with
+A step is one complete solve from f = 0 to the least fixed point, by the
+persistent sweep kernel (credit sweeps, and certificates that give the
+vertices of unbounded credit TOP without the climb to MG).
+  value  GTEPS = out-edges scanned by credit lifts / device time of the solve
+         (the certificates' sweeps are in the time, not in the edges), with
          the game resident in HBM; device time from CUDA events on the
          solver's stream; L2 flushed (256 MB write) before every step
   e2e    the same metric through the one-call public API eg_solve_i64 with
          pinned host buffers: allocation, host->device copy of the CSR, solve,
          device->host copy of the credits, per step (wall clock)
-  roofline   the dominant kernel (k_lift_dense, the dense rounds): its
+  roofline   the dominant kernel (k_sweep): its
          algorithmic bytes per launch / its mean launch time (CUDA events
          around each launch, on the solver's stream), against the measured
-         HBM copy bandwidth; `traffic` is the DRAM bytes per launch scaled
-         from an ncu capture of a round-capped solve (profiles/)
+         HBM copy bandwidth; `traffic` is the DRAM bytes per launch of an ncu
+         capture of the same solve (profiles/)
   cpu_baseline   the reference's own EG_cpu_solver (oracle/_ref, compiled
          unmodified; serial worklist, 1 core) on a bounded sample of the same
          game: its first P worklist pops (reference --eg P)
@@ -33,7 +34,7 @@ single-game solve does not shard); value = edges of all ranks / max time.
 bounded sample of the same workload.
 
 --workload cfg4 (batched): the first --games games of the seeded 4096-game
-stream at K = 8 mean-payoff thresholds in one persistent launch, against
+stream at K = 8 mean-payoff thresholds in one batched solve, against
 one plain solve per (game, threshold) on a seeded sample.  --workload cfg5
 (served): the seeded request stream (n up to --n-max) through the serving
 loop at each --rates arrival rate, against the same arrivals served one at
@@ -718,7 +719,25 @@ def main():
     peak, peak_kind = measured_peak()
     S = credit_bits // 8
     traffic = None
-    if last.dense_rounds > 0 and last.dense_ms > 0:
+    if last.dense_rounds > 0 and last.dense_ms > 0 and last.large_min_deg == 0:
+        # the sweep kernel: it has no degree buckets
+        launches_k = sum(s.dense_launches for s in stats)
+        d_bytes = sum(s.edges * (8 + S) + s.lifts * (8 + S) + s.changes * S for s in stats)
+        d_ms = sum(s.dense_ms for s in stats)
+        per_launch = d_bytes / launches_k
+        achieved = d_bytes / (d_ms / 1e3) / 1e9
+        kernel = "k_sweep (persistent sweep kernel)"
+        tf = ROOT / "profiles" / "k_sweep_traffic.json"
+        if tf.exists():
+            try:
+                d = json.loads(tf.read_text())
+                if d.get("workload") == cfg["workload"] and d.get("n") == game.num_nodes:
+                    traffic = d["dram_bytes_per_launch"]
+            except (ValueError, KeyError):
+                traffic = None
+        extra = {"launches": launches_k, "credit_sweeps_per_launch": sum(s.dense_rounds for s in stats) / launches_k,
+                 "ms_per_launch": d_ms / launches_k}
+    elif last.dense_rounds > 0 and last.dense_ms > 0:
         # the dense-round kernel: mean over its launches in the timed steps
         d_rounds = sum(s.dense_rounds for s in stats)
         d_launch = sum(s.dense_launches for s in stats)

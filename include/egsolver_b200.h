@@ -70,7 +70,12 @@ typedef enum eg_variant {
     EG_VARIANT_SMEM = 4      /* whole game resident in one CTA's shared memory       */
 } eg_variant;
 
-/* Round kinds of the lean grid kernel (eg_opts.direction).  A sparse round
+/* A solve with AUTO, SWITCH and the knobs of rounds (ctas_per_sm, schedule,
+ * the permilles, wide_pairs, profile) at 0 is done by the sweep solver: credit
+ * sweeps cut short by certificates of unbounded credit.  With any of those
+ * set it runs in rounds.  The credits are the same.
+ *
+ * Round kinds of the lean grid kernel (eg_opts.direction).  A sparse round
  * lifts the frontier and pushes predecessors of raised vertices, as the
  * reference's worklist does; a dense round lifts every vertex and pushes
  * nothing.  Both are fair chaotic iterations of the same operator, so the
@@ -109,7 +114,8 @@ typedef struct eg_opts {
     int32_t lanes_per_vertex;    /* with EG_VARIANT_WARP: 2,4,8,16 or 32 lanes per
                                     vertex (reference --shuffling K); 0 means 32       */
     int32_t keep_layout;         /* non-zero: reuse the transpose/renumbering of the
-                                    previous solve of the same resident game           */
+                                    previous solve of the same resident game (rounds;
+                                    the sweep solver has none)                        */
     int32_t grid_ctas;           /* cap on the lifting grid's CTAs (0: every SM, full
                                     occupancy); a smaller grid leaves SMs to other work */
     int32_t task_edges;          /* edges per task of a heavy vertex, 32..256 (0: 256) */
@@ -132,13 +138,13 @@ typedef struct eg_opts {
                                     even when successor and weight fit 32 bits        */
     int32_t dense_depth;         /* chunks in flight per warp in dense rounds: 1 (three
                                     CTAs per SM) or 2 (two CTAs per SM); 0: 2         */
-    int32_t dense_sweeps;        /* sweeps of the edge stream per grid barrier in dense
-                                    rounds: 1 to 4; 0: 4                              */
+    int32_t dense_sweeps;        /* sweeps per grid barrier in dense rounds: 1 to 4
+                                    (0: 4); the sweep solver runs at most 2           */
 } eg_opts;
 
 typedef struct eg_stats {
     int64_t mg;                  /* MG of the game (reference MG_pesi)                */
-    int64_t rounds;              /* synchronous rounds run on the device              */
+    int64_t rounds;              /* rounds of credit lifts run on the device          */
     int64_t lifts;               /* vertices lifted (reference processedNodes)        */
     int64_t edges;               /* sum of out-degrees of lifted vertices             */
     int64_t num_top;             /* vertices whose credit is TOP                       */
@@ -151,16 +157,15 @@ typedef struct eg_stats {
     int64_t changes;             /* lifts that raised a credit                        */
     int64_t pushes;              /* predecessor entries scanned after those raises    */
     int32_t grid, block;         /* launch shape of the lifting kernel                */
-    int32_t dense_rounds;        /* sweeps that lifted every vertex (no frontier); a
-                                    dense round is dense_sweeps sweeps               */
-    int32_t dense_launches;      /* launches of the dense-round kernel                */
+    int32_t dense_rounds;        /* credit sweeps over every vertex (no frontier)     */
+    int32_t dense_launches;      /* launches of the sweep or dense-round kernel       */
     /* with opts.profile, in nanoseconds.  Frontier rounds only: mean time per
      * warp and round in heavy tasks, in word classes, and waiting at the round
      * barrier.  With dense rounds: the slowest slice per dense round (heavy),
      * the mean slice per warp (light), and the mean round-to-round time (wait) */
     double  phase_heavy_ns, phase_light_ns, phase_wait_ns;
-    double  dense_ms;            /* device time of the dense-round kernel's launches  */
-    int64_t dense_changes;       /* credits raised in dense rounds                    */
+    double  dense_ms;            /* device time of those launches                     */
+    int64_t dense_changes;       /* credits raised by them                            */
 } eg_stats;
 
 /* ------------------------------------------------------------------ */
@@ -254,7 +259,7 @@ void eg_dgame_free(eg_dgame *g);
 /* CSR -> CSC transpose (the reference's csr2csc / host_csr2csc)        */
 /* ------------------------------------------------------------------ */
 
-/* Deterministic counting-sort transpose on the device of a host CSR:
+/* Deterministic transpose on the device of a host CSR:
  * csc_ptr (n+1), csc_src (m), csc_val (m) come out array-equal to the
  * reference's host_csr2csc (reference src/host_csr2csc.c:15-46): within
  * each column the entries keep their source order.  Replaces
@@ -264,17 +269,18 @@ eg_status eg_csr2csc_i32(int32_t num_rows, int32_t num_cols, int64_t nnz,
                          int64_t *csc_ptr, int32_t *csc_row, int32_t *csc_val);
 
 /* ------------------------------------------------------------------ */
-/* Batched solving: many games x K thresholds in one persistent launch  */
+/* Batched solving: many games x K thresholds in one solve              */
 /* ------------------------------------------------------------------ */
 
 /* A mean-payoff query "is the mean payoff of v at least p/d?" is the
  * energy game with weights w*d - p (new; the reference solves one energy
  * game per process).  A batch packs many games into one device-resident
- * layout; one persistent launch then solves every (game, threshold) pair.
+ * layout; one solve then settles every (game, threshold) pair.
  * The work is cut into units of one game at a group of 1, 2, 4 or 8
  * thresholds, one CTA per unit with the unit's credits in shared memory,
- * taken from a device queue heaviest first.  When the queue runs dry, the
- * units still running hand their open thresholds to a cluster tail: each
+ * taken from a device queue heaviest first.  When the queue runs dry, units
+ * that certificates did not decide hand their open thresholds to a cluster
+ * tail: each
  * (game, threshold) on a thread-block cluster whose CTAs each hold a
  * replica of its credits. */
 #define EG_BATCH_MAX_K 32
@@ -291,7 +297,8 @@ typedef struct eg_batch_opts {
     int32_t use_graph;           /* non-zero: the solve's launches are captured in a
                                     CUDA graph on the first solve and replayed      */
     int32_t group_max;           /* most thresholds per work unit: 1, 2, 4 or 8
-                                    (0: 8)                                          */
+                                    (0: 8, and fewer for large games while SMs are
+                                    idle)                                           */
     int32_t tail_rows;           /* games of at least this many vertices go straight
                                     to the cluster tail (0: none)                   */
     int32_t park_percent;        /* running units move to the cluster tail once this
