@@ -65,8 +65,8 @@
  * input order, 64-bit values, a barrier with a last arriver) / this one:
  * uniform game of 131,072 vertices 684 ms / 0.41 / 0.25 ms, of 16,381 at a
  * threshold 85 ms / 0.16 / 0.09 ms; power-law game of 2^20 vertices and 8.3 M
- * edges 9.3 s / 15.9 / 4.2 ms, of 6,007 59 ms / 1.25 / 0.30 ms; complete digraph
- * of 2,000 14.2 ms / 0.47 / 0.15 ms; 4-regular game of 1,000 4.1 ms / 0.11 /
+ * edges 9.3 s / 15.9 / 4.0 ms, of 6,007 59 ms / 1.25 / 0.25 ms; complete digraph
+ * of 2,000 14.2 ms / 0.47 / 0.10 ms; 4-regular game of 1,000 4.1 ms / 0.11 /
  * 0.05 ms (one CTA).
  *
  * Credits are CT integers with TOP = Lim::top while the solve runs: OMINUS(a,
@@ -96,9 +96,10 @@ constexpr int kVertexBytes = 28; /* credit, potential, its copy (8 B each), id *
  * kLightDeg edges per owner, and up to 62 slots without a vertex. */
 constexpr int kPadEdges = 4 * 32 * kLightDeg + 64, kPadSlots = 64, kSlackBytes = 8 * kPadEdges + 8192;
 /* Sweeps of the phases; the next dual and primal phases are twice as long.
- * Measured on 131 K vertices / a power-law game of 2^20: first dual phase 6
- * 284 us / 4.5 ms, 8 302 / 4.3; second primal phase 32 against 16, with which
- * many games need a second attempt, 300 us / 4.3 ms against 301 / 5.6. */
+ * Measured, means over 70 games of 64 to 131,072 vertices: first dual phase 6
+ * 75 us, 8 81 us; 4 74 us, but 3-5% slower on 4-regular games and on one of
+ * 16,381 vertices at a threshold.  Second primal phase 32 against 16, with
+ * which many games need a second attempt: 2^20 vertices 4.3 against 5.6 ms. */
 constexpr int kFirstPrimal = 2, kFirstDual = 6, kSecondPrimal = 32, kMaxDual = 32, kMaxPrimal = 1 << 16;
 
 /* flags of a round barrier's word */
@@ -160,12 +161,13 @@ struct Hubs {
  * when it reaches TOP or at the end: until then every primal sweep lifts it. */
 struct Count {
     unsigned raised;
-    unsigned sweeps;          /* primal sweeps begun                         */
+    unsigned sweeps, heavy_sweeps; /* primal sweeps begun, of light and of heavy vertices */
     unsigned long long changes, lifts, edges;
-    __device__ __forceinline__ void settle(const long long *rp, int v)
+    __device__ __forceinline__ void settle(const long long *rp, int v, bool heavy)
     {
-        lifts += sweeps;
-        edges += (unsigned long long)sweeps * (unsigned long long)(rp[v + 1] - rp[v]);
+        const unsigned n = heavy ? heavy_sweeps : sweeps;
+        lifts += n;
+        edges += (unsigned long long)n * (unsigned long long)(rp[v + 1] - rp[v]);
     }
 };
 
@@ -240,7 +242,7 @@ __device__ __forceinline__ void finish_vertex(const Range &r, const Kind<CT> &k,
     M::set(r, k.mode, slot, nv);
     if (k.mode == SWEEP_PRIMAL && nv == top) {
         M::set(r, 1, slot, Lim<CT>::low);
-        cnt.settle(r.rp, M::vid(r, slot));
+        cnt.settle(r.rp, M::vid(r, slot), slot >= r.light_slots);
     }
 }
 
@@ -358,7 +360,7 @@ __device__ __forceinline__ void sweep_heavy(const Range &r, const Kind<CT> &kd, 
 /* One sweep of the CTA's vertices: the light ones here, a slice per warp, a
  * vertex per lane. */
 template <typename CT, int KIND, bool GROUP>
-__device__ __forceinline__ void sweep(const Range &r, const Kind<CT> &kd, Hubs &hb, Count &cnt)
+__device__ __forceinline__ void sweep(const Range &r, const Kind<CT> &kd, Hubs &hb, Count &cnt, bool heavy)
 {
     using M = Mem<CT, KIND>;
     constexpr int U = kUnroll<KIND>;
@@ -399,7 +401,7 @@ __device__ __forceinline__ void sweep(const Range &r, const Kind<CT> &kd, Hubs &
         }
         finish_vertex<CT, KIND>(r, kd, sign, slot, old, acc, cnt);
     }
-    if (r.nh) sweep_heavy<CT, KIND>(r, kd, hb, cnt);
+    if (heavy && r.nh) sweep_heavy<CT, KIND>(r, kd, hb, cnt);
 }
 
 /* The schedule after a round of `ran` sweeps in which `raised` values changed
@@ -515,7 +517,7 @@ __device__ __noinline__ void solve(const SweepParams *pp, const Range &rs, Hubs 
                     M::set(r, 0, i, top);
                     M::set(r, 1, i, low);
                     cnt.raised++;
-                    cnt.settle(r.rp, M::vid(r, i));
+                    cnt.settle(r.rp, M::vid(r, i), i >= r.light_slots);
                 }
             }
             __syncthreads();
@@ -528,8 +530,19 @@ __device__ __noinline__ void solve(const SweepParams *pp, const Range &rs, Hubs 
         const int ran = phase == SWEEP_DUAL ? st.left : phase == SWEEP_KILL ? min(r.round, 2) : min(r.round, st.left);
 #pragma unroll 1
         for (int s = 0; s < ran; s++) {
-            if (phase == SWEEP_PRIMAL) cnt.sweeps++;
-            sweep<CT, KIND, GROUP>(r, kd, hb, cnt);
+            /* The heavy vertices every second time, and in a round's last sweep,
+             * so that a round without a raise has lifted all.  They are most of
+             * the edges of a power-law game, and the parts that hold them the
+             * last at every barrier, but move no faster than what they gather
+             * (power-law games of 2^20 vertices 3.5-5.9 -> 2.5-4.0 ms, of up to
+             * 6,000 211 -> 188 us, complete digraphs 114 -> 77).  In one CTA, with
+             * no barrier to be late at, all every time. */
+            const bool heavy = !GRID || s == ran - 1 || (phase == SWEEP_DUAL && (s & 1));
+            if (phase == SWEEP_PRIMAL) {
+                cnt.sweeps++;
+                cnt.heavy_sweeps += heavy;
+            }
+            sweep<CT, KIND, GROUP>(r, kd, hb, cnt, heavy);
         }
         if (phase == SWEEP_PRIMAL) cnt.changes += cnt.raised;
         if (phase == SWEEP_DUAL) {
@@ -578,7 +591,7 @@ __device__ __noinline__ void solve(const SweepParams *pp, const Range &rs, Hubs 
         if (v < 0) continue;
         const CT f = M::own(r, 0, i);
         if (f == top) cnt.raised++;
-        else cnt.settle(r.rp, v);
+        else cnt.settle(r.rp, v, i >= r.light_slots);
         if (r.out_bits == 32) ((int *)p.out)[v] = f == top ? INT32_MAX : (int)f;
         else ((long long *)p.out)[v] = f == top ? (long long)INT64_MAX : (long long)f;
     }
@@ -1016,7 +1029,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
         r.mg = (long long)mg;
         r.scale = 1ll << nshift;
     }
-    Count cnt = {0u, 0u, 0ull, 0ull, 0ull};
+    Count cnt = {0u, 0u, 0u, 0ull, 0ull, 0ull};
     __syncthreads();
     auto run = [&](auto credit, auto kind) {
         using CT = decltype(credit);
