@@ -169,7 +169,13 @@ class ClockSampler:
         for line in self.proc.stdout:
             self.lines.append(line.strip())
 
-    def stop(self) -> dict:
+    def stop(self, load=None) -> dict:
+        """Ends the sampling.  Timed steps of some milliseconds end before the
+        first sample: `load` (the same step, untimed) then runs on until there
+        is one, two seconds at most."""
+        until = time.perf_counter() + 2.0
+        while load is not None and self.proc is not None and not self.lines and time.perf_counter() < until:
+            load()
         if self.proc is None:
             return {"sm_mhz": None, "sm_max_mhz": None, "reasons": ["nvidia-smi unavailable"]}
         self.proc.terminate()
@@ -409,7 +415,7 @@ def run_batched(args):
         times.append(st.solve_ms)
         stats.append(st)
         progress(f"timed solve {st.solve_ms:.1f} ms, {st.games_failed} game(s) stopped by the time limit")
-    clocks = sampler.stop()
+    clocks = sampler.stop(lambda: b.solve(raise_on_error=False))
     ms = sum(times) / len(times)
     done = G - max(s.games_failed for s in stats)  # games solved to the fixed point in every step
     value = done / (ms / 1e3)
@@ -659,7 +665,7 @@ def main():
         stats.append(st)
     torch.cuda.synchronize()
     t_wall = time.perf_counter() - t_wall
-    clocks = sampler.stop()
+    clocks = sampler.stop(lambda: res.solve(raise_on_error=not capped, **kw))
     if dist:
         dist.barrier()
     dev_ms = sum(s.solve_ms for s in stats)
