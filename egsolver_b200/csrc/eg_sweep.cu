@@ -405,7 +405,9 @@ __device__ __forceinline__ void sweep(const Range &r, const Kind<CT> &kd, Hubs &
 }
 
 /* The schedule after a round of `ran` sweeps in which `raised` values changed
- * (any number but 0 where it is only compared with that). */
+ * (any number but 0 where it is only compared with that).  `stop`: the time
+ * limit or the cancel flag, which ends any phase (a kill phase may be as long
+ * as the game is deep): the credits are lower bounds at all times. */
 __device__ __forceinline__ void advance(const SweepParams &p, SweepState &c, int ran, unsigned long long raised, int stop)
 {
     if (c.phase == SWEEP_PRIMAL) {
@@ -416,14 +418,17 @@ __device__ __forceinline__ void advance(const SweepParams &p, SweepState &c, int
             c.phase = SWEEP_DONE;
             return;
         }
-        c.stop = p.max_rounds >= 0 && c.rounds >= p.max_rounds ? (int)EG_ERR_LOOPCAP : stop;
-        if (c.left > 0) return;
+        if (p.max_rounds >= 0 && c.rounds >= p.max_rounds) stop = (int)EG_ERR_LOOPCAP;
+        c.stop = stop;
+        if (stop || c.left > 0) return;
         if (p.hand_sweeps && c.sweeps >= p.hand_sweeps && (long long)raised < p.hand_raised) {
             c.phase = SWEEP_HANDOVER;
             return;
         }
         c.phase = SWEEP_DUAL;
         c.left = c.dual_len;
+    } else if (stop) {
+        c.stop = stop;
     } else if (c.phase == SWEEP_DUAL) {
         c.dual_len = min(2 * c.dual_len, kMaxDual);
         c.phase = SWEEP_KILL;
@@ -494,6 +499,7 @@ __device__ __noinline__ void solve(const SweepParams *pp, const Range &rs, Hubs 
      * faster with them in shared memory (complete digraph 171 -> 152 us) */
     std::conditional_t<GROUP, const Range &, const Range> r = rs;
     SweepState st = state;
+    const unsigned first = it;
     Count cnt = count;
     const int tid = threadIdx.x, lane = tid & 31;
     const int nslots = r.light_slots + r.nh;
@@ -552,9 +558,9 @@ __device__ __noinline__ void solve(const SweepParams *pp, const Range &rs, Hubs 
         /* the round's raises and the next step of the schedule */
         unsigned long long raised;
         int stop = 0;
-        if (tid == 0 && watch && blockIdx.x == 0 && phase == SWEEP_PRIMAL) {
+        if (tid == 0 && watch && blockIdx.x == 0) {
             if (p.timeout_ns && globaltimer_ns() - p.ctrl->t_start > p.timeout_ns) stop = (int)EG_ERR_TIMEOUT;
-            else if (p.cancel && (st.rounds & 63) == 0 && ld_volatile(p.cancel)) stop = (int)EG_ERR_CANCELLED;
+            else if (p.cancel && ((it - first) & 63) == 0 && ld_volatile(p.cancel)) stop = (int)EG_ERR_CANCELLED;
         }
         if (GRID) {
             const unsigned d = __reduce_add_sync(0xffffffffu, cnt.raised);

@@ -3,6 +3,8 @@ layout changes -- one CTA or the grid, values in shared or global memory,
 edges staged or not, cut vertices -- and the hand-over to frontier rounds."""
 from __future__ import annotations
 
+import threading
+
 import numpy as np
 import pytest
 
@@ -145,3 +147,37 @@ def test_lanes_that_share_a_vertex(kind, n, deg, ctas):
         g = eg.Game(row_ptr=g.row_ptr, succ=g.succ, weight=g.weight * 40000, owner=rng.integers(0, 2, n).astype(np.uint8))
         f, _ = eg.solve(g, grid_ctas=ctas)
         np.testing.assert_array_equal(f, want(g))
+
+
+def chain(n, step=-1):
+    """One path of n vertices, the first half player 0's, into a vertex that
+    stays where it is at weight 0: n - 1 steps of cost, no bound but the path's."""
+    succ = np.minimum(np.arange(1, n + 1), n - 1)
+    weight = np.full(n, step)
+    weight[-1] = 0
+    return eg.Game(row_ptr=np.arange(n + 1), succ=succ, weight=weight, num_nodes0=n // 2)
+
+
+def test_time_limit_of_a_deep_game():
+    """Of 400,000 vertices on a path none is certified, and a kill phase takes
+    them out one after the other: the limit must not wait for its end."""
+    n = 400_000
+    with eg.ResidentGame(chain(n)) as r:
+        status, st = r.solve(raise_on_error=False, timeout_ms=20)
+        assert eg._ffi.STATUS_NAMES[status] == "EG_ERR_TIMEOUT"
+        assert st.solve_ms < 60
+        assert np.all(r.credits() <= np.arange(n)[::-1])
+
+
+def test_cancel_of_a_deep_game():
+    n = 400_000
+    flag = eg.CancelFlag()
+    try:
+        with eg.ResidentGame(chain(n)) as r:
+            threading.Timer(0.02, flag.set).start()
+            status, st = r.solve(raise_on_error=False, cancel=flag)
+            assert eg._ffi.STATUS_NAMES[status] == "EG_ERR_CANCELLED"
+            assert st.solve_ms < 80
+            assert np.all(r.credits() <= np.arange(n)[::-1])
+    finally:
+        flag.free()
