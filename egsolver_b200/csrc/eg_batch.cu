@@ -302,18 +302,22 @@ __device__ __forceinline__ void run_unit(const UnitDesc &u, int uglobal, unsigne
         }
         raised = __reduce_or_sync(0xffffffffu, raised);
         if (lane == 0 && raised) atomicOr(&sh.raise[it], raised);
-        if (tid == 0 && !dual) {
+        if (tid == 0) {
             if (P.timeout_ns && globaltimer_ns() - t0 > P.timeout_ns) atomicOr(&sh.raise[it], 1u << 16);
             /* park: this variant's queue is empty and a share of all phase-1
              * CTAs have nothing left, so the GPU is running the tail; the
              * unit's open thresholds continue on clusters */
-            if (P.tails && (r & 15) == 15 && r >= kParkSweeps && ld_volatile(&P.ctrl->next) >= P.num_units &&
+            if (!dual && P.tails && (r & 15) == 15 && r >= kParkSweeps && ld_volatile(&P.ctrl->next) >= P.num_units &&
                 100 * ld_volatile(P.idle) >= P.park_percent * P.park_total)
                 atomicOr(&sh.raise[it], 1u << 17);
         }
         __syncthreads();
         const unsigned word = sh.raise[it];
         if (tid == 0) sh.raise[it == 0 ? 2 : it - 1] = 0;
+        if (dual && (word & (1u << 16))) {
+            st = EG_ERR_TIMEOUT;
+            break;
+        }
         if (mode == UNIT_DUAL) {
             if (--left == 0 || !(word & full)) mode = UNIT_KILL;
             continue;
@@ -369,13 +373,16 @@ __device__ __forceinline__ void run_unit(const UnitDesc &u, int uglobal, unsigne
         }
     }
     __syncthreads();
-    /* credits out, threshold-major in original vertex ids */
+    /* credits out, threshold-major in original vertex ids; a time limit that
+     * ends an attempt finds potentials in the open thresholds' buffer, of whose
+     * credits only the TOPs (at LOW there) are known */
     unsigned long long top = 0;
     for (int i = tid; i < npad * KG; i += blockDim.x) {
         const int k = i / npad, v = i - k * npad;
         const int o = __ldg(u.orig + v);
         if (o >= 0) {
-            const CT c = F.at(v)[k];
+            CT c = F.at(v)[k];
+            if (mode != UNIT_PRIMAL && (amask >> k & 1u)) c = c == LOWI ? TOPI : (CT)0;
             u.F[(long long)(u.k0 + k) * u.n + o] = c >= TOPI ? (long long)INT64_MAX : (long long)c;
             /* the TOPs of a parked unit's open thresholds are counted by the tail */
             top += c >= TOPI && !(st == kParked && (amask >> k & 1u));

@@ -245,3 +245,23 @@ def test_groups_of_large_games(num, nodes, K):
     assert got[1][0] == num * (K // 8 + (K % 8).bit_count())
     for a, b in zip(got[0][1], got[1][1]):
         np.testing.assert_array_equal(a, b)
+
+
+def chain(n, step=-1):
+    """A path of n vertices into one that stays where it is at weight 0."""
+    weight = np.full(n, step)
+    weight[-1] = 0
+    return eg.Game(row_ptr=np.arange(n + 1), succ=np.minimum(np.arange(1, n + 1), n - 1), weight=weight, num_nodes0=n // 2)
+
+
+def test_time_limit_of_a_deep_game():
+    """No vertex of the path is certified, and a kill phase takes them out one
+    after the other: the limit must not wait for its end, and what the unit
+    holds then are potentials, not credits."""
+    n = 50_000
+    with eg.Batch([chain(n)], thresholds=1, timeout_ms=20, park_percent=1000) as b:
+        b.set_thresholds([0])
+        status, st = b.solve(raise_on_error=False)
+        assert st.games_failed == 1 and st.solve_ms < 60
+        assert eg._ffi.STATUS_NAMES[b.game_result(0)[1]] == "EG_ERR_TIMEOUT"
+        assert np.all(b.credits(0)[0] <= np.arange(n)[::-1])
