@@ -18,6 +18,7 @@ struct SweepState {
     int phase;
     int left;                            /* sweeps left in this phase          */
     int primal_len, dual_len;            /* sweeps of the next phases          */
+    int kills;                           /* rounds of this kill phase          */
     int stop;                            /* 0 running; else an eg_status       */
     long long rounds;                    /* primal rounds completed            */
     long long sweeps;                    /* primal sweeps run                  */

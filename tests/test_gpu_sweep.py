@@ -181,3 +181,17 @@ def test_cancel_of_a_deep_game():
             assert np.all(r.credits() <= np.arange(n)[::-1])
     finally:
         flag.free()
+
+
+# a path of 16,384 on the grid, a shorter one in one CTA
+@pytest.mark.parametrize("n", [16384, 3000])
+def test_dropped_attempts_cost_no_more_than_the_sweeps(n):
+    """Kill sweeps that run to their end on a path take ten times the credit
+    sweeps.  The second game has as many credit sweeps and short kills."""
+    deep, flat = chain(n), chain(n, 0)
+    flat.weight[-2] = -5
+    with eg.ResidentGame(deep) as a, eg.ResidentGame(flat) as b:
+        ms = [min(r.solve()[1].solve_ms for _ in range(3)) for r in (a, b)]
+        np.testing.assert_array_equal(a.credits(), np.arange(n)[::-1])
+        np.testing.assert_array_equal(b.credits(), np.where(np.arange(n) < n - 1, 5, 0))
+    assert ms[0] < 4 * ms[1]
