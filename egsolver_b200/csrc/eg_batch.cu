@@ -127,6 +127,9 @@ enum { UNIT_PRIMAL, UNIT_DUAL, UNIT_KILL };
  * restart once more. */
 constexpr int kUnitFirstPrimal = 2, kUnitSecondPrimal = 32, kUnitFirstDual = 6, kUnitMaxDual = 128;
 constexpr long long kUnitMaxPrimal = 1 << 20;
+/* Kill sweeps that an attempt may take in any case (random games take less
+ * than a hundred). */
+constexpr int kUnitKills = 256;
 /* Units below this many sweeps do not park: all but 1 in 500 of the
  * thresholds of random games at uniform thresholds end within it, and the
  * tail runs no certificates. */
@@ -218,7 +221,10 @@ __device__ __forceinline__ int potential_shift(const UnitDesc &u)
  * exchanged and weights -(2^nshift (w d - p) + 1) (dual sweeps, from 0),
  * then kill sweeps put every vertex out (TOP) whose potential is not one,
  * until none goes.  The vertices left are TOP of the game itself; the others
- * start again from credit 0, for four times as many sweeps, and so on.
+ * start again from credit 0, for four times as many sweeps, and so on.  A
+ * threshold that still loses vertices after as many kill sweeps as there were
+ * primal ones (a path is taken apart one vertex a sweep) has nothing certified
+ * (path of 16,384 vertices, kills to their end: 1,826 ms, of which 423 primal).
  * Nothing of the credits but the TOPs is kept over an attempt: a second
  * buffer would halve the thresholds of a group, and the sweeps run again
  * are at most a third of the last phase.  A vertex at TOP before an attempt
@@ -319,17 +325,22 @@ __device__ __forceinline__ void run_unit(const UnitDesc &u, int uglobal, unsigne
             break;
         }
         if (mode == UNIT_DUAL) {
-            if (--left == 0 || !(word & full)) mode = UNIT_KILL;
+            if (--left == 0 || !(word & full)) {
+                mode = UNIT_KILL;
+                left = 0; /* kill sweeps */
+            }
             continue;
         }
         if (mode == UNIT_KILL) {
-            if (word & full) continue;
+            const unsigned going = word & full;
+            if (going && (++left < kUnitKills || left < min(r, primal_len))) continue;
             /* what is left is certified: TOP; the others start again from 0 */
             for (int i = tid; i < rows * KG; i += blockDim.x) {
                 const int row = i >> LK, k = i & (KG - 1);
                 if (amask >> k & 1u) {
                     CT *x = F.at(row) + k;
-                    *x = row >= npad ? (row == npad ? TOPI : LOWI) : (*x == TOPI ? (CT)0 : TOPI);
+                    const bool open = *x == TOPI || ((going >> k & 1u) && *x != LOWI);
+                    *x = row >= npad ? (row == npad ? TOPI : LOWI) : (open ? (CT)0 : TOPI);
                 }
             }
             mode = UNIT_PRIMAL;

@@ -265,3 +265,31 @@ def test_time_limit_of_a_deep_game():
         assert st.games_failed == 1 and st.solve_ms < 60
         assert eg._ffi.STATUS_NAMES[b.game_result(0)[1]] == "EG_ERR_TIMEOUT"
         assert np.all(b.credits(0)[0] <= np.arange(n)[::-1])
+
+
+def test_dropped_attempts_cost_no_more_than_the_sweeps():
+    """Kill sweeps that run to their end on a path take four times the credit
+    sweeps.  The second game has as many credit sweeps and short kills."""
+    n = 16384
+    deep, flat = chain(n), chain(n, 0)
+    flat.weight[-2] = -5
+    ms = []
+    for g, want in ((deep, np.arange(n)[::-1]), (flat, np.where(np.arange(n) < n - 1, 5, 0))):
+        with eg.Batch([g], thresholds=1, park_percent=1000) as b:
+            b.set_thresholds([0])
+            ms.append(min(b.solve()[1].solve_ms for _ in range(3)))
+            np.testing.assert_array_equal(b.credits(0)[0], want)
+    assert ms[0] < 3 * ms[1]
+
+
+@pytest.mark.parametrize("group_max", [0, 1])
+def test_a_group_in_which_some_thresholds_are_dropped(group_max):
+    """A path at thresholds that leave its steps' cost (an attempt is dropped),
+    take it away, and make every vertex unbounded (certified)."""
+    n = 2000
+    deep, zero, top = np.arange(n)[::-1], np.zeros(n, np.int64), np.full(n, eg.EG_TOP64)
+    p, want = [0, -1, 1, 0, 7, -3, 0], [deep, zero, top, deep, top, zero, deep]
+    with eg.Batch([chain(n)], thresholds=7, group_max=group_max) as b:
+        b.set_thresholds(p)
+        b.solve()
+        np.testing.assert_array_equal(b.credits(0), np.array(want))
