@@ -307,6 +307,19 @@ void pool_free(void *p, cudaStream_t st)
     if (p) cudaFreeAsync(p, st);
 }
 
+size_t pool_idle(int device)
+{
+    cudaMemPool_t pool;
+    unsigned long long held = 0, used = 0;
+    if (pool_of(device, &pool) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return held > used ? (size_t)(held - used) : 0;
+}
+
 Lane *lane_take(int device)
 {
     if (device < 0 || device >= kMaxDevices) return nullptr;

@@ -24,6 +24,9 @@ namespace eg {
  * that has waited for its last use). */
 cudaError_t pool_alloc(void **p, size_t bytes, int device, cudaStream_t st);
 void pool_free(void *p, cudaStream_t st);
+/* Bytes that the device's pool holds and nobody uses: free memory that
+ * cudaMemGetInfo does not count. */
+size_t pool_idle(int device);
 
 /* A stream with timing events and some pinned memory. */
 struct Lane {

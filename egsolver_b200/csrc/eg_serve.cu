@@ -9,11 +9,11 @@
  *      their queries (device -> host) and release the queries' buffers;
  *   2. admission, in submission order: a query is admitted when fewer than
  *      max_inflight queries are admitted and the free device memory (from
- *      cudaMemGetInfo, less what queries admitted since that look take) minus
- *      hbm_reserve_bytes covers its credits and, if its game is not resident
- *      yet, the game's packed layout; idle resident games are evicted
- *      oldest-first when memory is short.  A game stays resident across all
- *      its queries until it is evicted or removed;
+ *      cudaMemGetInfo and what the pool holds idle, less what queries admitted
+ *      since that look take) minus hbm_reserve_bytes covers its credits and,
+ *      if its game is not resident yet, the game's packed layout; idle
+ *      resident games are evicted oldest-first when memory is short.  A game
+ *      stays resident across all its queries until it is evicted or removed;
  *   3. launch: the admitted queries not yet launched go into one or two
  *      micro-batches, i.e. launches of the unit kernels (eg_batch.cu: one CTA
  *      per game x threshold group, credits in shared memory), each on the next
@@ -213,6 +213,7 @@ bool make_room(eg_server *s, std::unique_lock<std::mutex> &lk, size_t need, size
         size_t free_b = 0, total_b = 0;
         lk.unlock();
         const cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
+        free_b += pool_idle(s->o.device);
         lk.lock();
         if (e != cudaSuccess) {
             cudaGetLastError();

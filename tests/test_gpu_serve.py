@@ -213,3 +213,23 @@ def test_threads_submit_while_queries_run():
             t.join()
         assert not errors, errors
         assert srv.stats()["completed"] == 4 * 3 * 7
+
+
+def test_evicted_games_make_room():
+    """Four games of about 30 MB each where the reserve leaves 40 MB, and what
+    the pool keeps comes to 64 MB at most: every query is admitted, after
+    evictions, one game at a time."""
+    torch = pytest.importorskip("torch")
+    games = [eg.generate(1, 30000, 250, 20, 70 + i) for i in range(4)]
+    with eg.Server() as s:  # modules and streams before the look at the free memory
+        gid = s.add_game(games[0])
+        s.wait(s.submit(gid, [900]))
+    with eg.Server(hbm_reserve_bytes=torch.cuda.mem_get_info()[0] - (40 << 20)) as s:
+        gids = [s.add_game(g) for g in games]
+        for turn in range(2):
+            for i, gid in enumerate(gids):
+                q = s.submit(gid, [900])  # above every weight: all TOP, at once
+                s.wait(q)
+                assert np.all(s.result(q)[0] == eg.EG_TOP64)
+        st = s.stats()
+        assert st["failed"] == 0 and 4 <= st["evictions"] <= 7
