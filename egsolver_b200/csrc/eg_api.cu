@@ -113,6 +113,7 @@ struct eg_dgame {
     int *d_counts;
     unsigned long long *d_mg;
     void *d_F, *d_out, *d_conv; /* d_conv: credits in another width */
+    void *d_lent; /* the array of eg_dgame_credits_device, made by its first call */
     uint32_t *d_B;
     Ctrl *d_ctrl;
     /* heavy vertices cut into edge tasks (AUTO layout) */
@@ -272,6 +273,8 @@ extern "C" void eg_dgame_free(eg_dgame *g)
     int prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(g->device);
+    /* waits for whatever still reads it on any stream */
+    if (g->d_lent) cudaFree(g->d_lent);
     if (g->lane) {
         pool_free(g->block, g->st);
         pool_free(g->rounds_block, g->st);
@@ -972,14 +975,31 @@ static eg_status dgame_credits(eg_dgame *g, O *host, int obits)
 extern "C" eg_status eg_dgame_credits_i32(eg_dgame *g, int32_t *credits) { return dgame_credits<int32_t>(g, credits, 32); }
 extern "C" eg_status eg_dgame_credits_i64(eg_dgame *g, int64_t *credits) { return dgame_credits<int64_t>(g, credits, 64); }
 
+/* The caller's work on the pointer is on streams of its own, and may pass it
+ * to a peer or another process: it is not the pool's memory, and its cudaFree
+ * waits for the device. */
 extern "C" eg_status eg_dgame_credits_device(eg_dgame *g, void **dev_ptr, int32_t *credit_bits)
 {
     if (!g || !dev_ptr) return eg_set_error(EG_ERR_INVALID, "NULL argument");
     if (!g->solved) return eg_set_error(EG_ERR_INVALID, "the game has no solved credits");
     EG_CUDA(cudaSetDevice(g->device));
-    if (!g->swept) launch_gather_out(g->solved_bits, g->solved_bits, g->n, g->d_iperm, g->d_F, g->d_out, g->st);
+    if (!g->d_lent) {
+        const size_t bytes = sizeof(int64_t) * (size_t)g->n;
+        const cudaError_t e = cudaMalloc(&g->d_lent, bytes);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            g->d_lent = nullptr;
+            return eg_set_error(EG_ERR_OOM, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+        }
+        g->bytes += bytes;
+    }
+    if (g->swept)
+        EG_CUDA(cudaMemcpyAsync(g->d_lent, g->d_out, (size_t)(g->solved_bits / 8) * (size_t)g->n, cudaMemcpyDeviceToDevice,
+                                g->st));
+    else
+        launch_gather_out(g->solved_bits, g->solved_bits, g->n, g->d_iperm, g->d_F, g->d_lent, g->st);
     EG_CUDA(cudaStreamSynchronize(g->st));
-    *dev_ptr = g->d_out;
+    *dev_ptr = g->d_lent;
     if (credit_bits) *credit_bits = g->solved_bits;
     return EG_OK;
 }

@@ -230,7 +230,9 @@ eg_status eg_dgame_solve(eg_dgame *g, const eg_opts *opts, eg_stats *stats);
 eg_status eg_dgame_credits_i32(eg_dgame *g, int32_t *credits);
 eg_status eg_dgame_credits_i64(eg_dgame *g, int64_t *credits);
 /* Device pointer to the credits of the last solve, in original vertex order
- * (int32 or int64 as solved); valid until the next solve or free. */
+ * (int32 or int64 as solved); valid until the next solve or free.  The array
+ * is the handle's own cudaMalloc, made by the first call; eg_dgame_free waits
+ * for the device before it goes. */
 eg_status eg_dgame_credits_device(eg_dgame *g, void **dev_ptr, int32_t *credit_bits);
 /* Device bytes held by the handle. */
 int64_t eg_dgame_device_bytes(const eg_dgame *g);

@@ -77,3 +77,32 @@ def test_transpose_edges(rows, cols, nnz, hot):
         col[rng.choice(nnz, hot, replace=False)] = cols - 1
     for a, b in zip(eg.csr2csc(rows, cols, rp, col, val), O.csr2csc(rows, cols, rp, col, val)):
         np.testing.assert_array_equal(a, b)
+
+
+def test_a_lent_pointer_is_memory_of_its_own():
+    """The array of credits_device can be mapped by other processes and peers
+    (it is not the pool's), and freeing the game waits for work that another
+    stream still has on it."""
+    torch = pytest.importorskip("torch")
+    from cuda.bindings import driver
+
+    g = eg.generate(4, 3000, 16, 50, 9, param=2)
+    r = eg.ResidentGame(g)
+    for kw in (dict(credit_bits=64), dict(credit_bits=32), dict(credit_bits=64, direction=eg.DIRECTION_DENSE)):
+        bits = kw["credit_bits"]
+        r.solve(**kw)
+        ptr, got_bits = r.credits_device()
+        assert got_bits == bits
+        err, legacy = driver.cuPointerGetAttribute(
+            driver.CUpointer_attribute.CU_POINTER_ATTRIBUTE_IS_LEGACY_CUDA_IPC_CAPABLE, ptr)
+        assert err == driver.CUresult.CUDA_SUCCESS and legacy
+        host = np.zeros(3000, np.int64 if bits == 64 else np.int32)
+        assert driver.cuMemcpyDtoH(host.ctypes.data, ptr, host.nbytes)[0] == driver.CUresult.CUDA_SUCCESS
+        np.testing.assert_array_equal(host, r.credits(bits))
+    side = torch.cuda.Stream()
+    done = torch.cuda.Event()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(40_000_000)
+        done.record()
+    r.free()
+    assert done.query()
