@@ -195,3 +195,41 @@ def test_dropped_attempts_cost_no_more_than_the_sweeps(n):
         np.testing.assert_array_equal(a.credits(), np.arange(n)[::-1])
         np.testing.assert_array_equal(b.credits(), np.where(np.arange(n) < n - 1, 5, 0))
     assert ms[0] < 4 * ms[1]
+
+
+def chains(length, count, tops):
+    """`count` paths of `length` vertices; a cost of 5 before the end of each,
+    which moves back a vertex per sweep, or (the last `tops`) an end whose
+    credit is unbounded, which does too."""
+    n = length * count
+    succ = np.arange(1, n + 1, dtype=np.int32)
+    succ[length - 1::length] = np.arange(length - 1, n, length)
+    weight = np.zeros(n, np.int32)
+    weight[length - 2::length] = -5
+    ref = np.full(n, 5)
+    ref[length - 1::length] = 0
+    if tops:
+        weight[length * (count - tops) + length - 1::length] = -1
+        ref[length * (count - tops):] = eg.EG_TOP64
+    return eg.Game(row_ptr=np.arange(n + 1), succ=succ, weight=weight, num_nodes0=n // 2), ref
+
+
+# long enough that the first look, at the end of the primal phase that passes
+# 2,048 sweeps, finds raises in every path
+@pytest.mark.parametrize("tops,narrow", [(0, False), (3, False), (3, True)])
+def test_frontier_rounds_take_over(tops, narrow):
+    g, ref = chains(16384, 260, tops)
+    f, st = eg.solve(g, narrow=narrow)
+    np.testing.assert_array_equal(f, ref)
+    assert st.kernel_launches > 1 and st.pushes > 0 and 2048 <= st.dense_rounds < 16384
+    assert st.num_top == tops * 16384 and st.credit_bits == (32 if narrow else 64)
+
+
+def test_round_cap_after_the_hand_over():
+    g, ref = chains(16384, 260, 1)
+    with eg.ResidentGame(g) as r:
+        status, st = r.solve(raise_on_error=False, max_rounds=7000)
+        assert eg._ffi.STATUS_NAMES[status] == "EG_ERR_LOOPCAP"
+        assert st.rounds == 7000 and st.pushes > 0
+        part = r.credits()
+        assert np.all(part <= ref) and np.any(part < ref) and np.any(part == 5)
