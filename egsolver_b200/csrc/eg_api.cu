@@ -853,10 +853,12 @@ static eg_status dgame_rounds(eg_dgame *g, const eg_opts *opts, const SweepCtrl 
 
 /* The solve by sweeps with certificates (eg_sweep.cu); a large game whose
  * credits still rise in a few places after kHandSweeps sweeps goes on with
- * frontier and dense rounds.  With `early` (a one-call solve) small results
+ * frontier and dense rounds, or, where their arrays do not fit, is swept to
+ * its end: from 0 again, as the sweep kernel keeps nothing, with the time
+ * `spent_ms` so far (else 0) in the limit and the statistics.  With `early` (a one-call solve) small results
  * come along with the control block, and *early says whether they did: they
  * are in the lane's pinned memory behind it. */
-static eg_status dgame_sweeps(eg_dgame *g, const eg_opts *opts, eg_stats *stats, bool *early)
+static eg_status dgame_sweeps(eg_dgame *g, const eg_opts *opts, eg_stats *stats, bool *early, float spent_ms)
 {
     cudaStream_t st = g->st;
     SweepParams p;
@@ -871,7 +873,7 @@ static eg_status dgame_sweeps(eg_dgame *g, const eg_opts *opts, eg_stats *stats,
     p.out = g->d_out;
     p.ctrl = g->d_sctrl;
     p.max_rounds = opts->max_rounds;
-    p.timeout_ns = opts->timeout_ms > 0 ? (unsigned long long)(opts->timeout_ms * 1e6) : 0ull;
+    p.timeout_ns = opts->timeout_ms > 0 ? (unsigned long long)(std::max(opts->timeout_ms - spent_ms, 1e-6) * 1e6) : 0ull;
     p.wait_limit_ns = kWaitLimitNs;
     if (opts->cancel) {
         void *dp = nullptr;
@@ -881,7 +883,7 @@ static eg_status dgame_sweeps(eg_dgame *g, const eg_opts *opts, eg_stats *stats,
     p.sweeps = opts->dense_sweeps ? opts->dense_sweeps : kMaxDenseSweeps;
     p.bits = opts->credit_bits == 32 ? 32 : 64;
     p.narrow = opts->narrow;
-    if (g->m >= kHandEdges) {
+    if (spent_ms == 0.f && g->m >= kHandEdges) {
         p.hand_sweeps = kHandSweeps;
         p.hand_raised = kSparsePermille * g->n / 1000;
     }
@@ -911,7 +913,14 @@ static eg_status dgame_sweeps(eg_dgame *g, const eg_opts *opts, eg_stats *stats,
     const int stop = c.abort ? (int)EG_ERR_TIMEOUT : c.s.stop;
     if (stop == EG_ERR_OVERFLOW)
         return eg_set_error(EG_ERR_OVERFLOW, "MG = %lld does not fit 32-bit credits", g->mg);
-    if (c.s.phase == SWEEP_HANDOVER && !stop) return dgame_rounds(g, opts, &c, stats);
+    if (c.s.phase == SWEEP_HANDOVER && !stop) {
+        const eg_status s = rounds_alloc(g);
+        if (s == EG_OK) return dgame_rounds(g, opts, &c, stats);
+        if (s != EG_ERR_OOM) return s;
+        float ms = 0.f;
+        EG_CUDA(cudaEventElapsedTime(&ms, g->ev[0], g->ev[3]));
+        return dgame_sweeps(g, opts, stats, early, std::max(ms, 1e-3f));
+    }
     if (early) *early = along;
     g->solved_bits = c.out_bits;
     g->solved = true;
@@ -920,6 +929,8 @@ static eg_status dgame_sweeps(eg_dgame *g, const eg_opts *opts, eg_stats *stats,
         float solve_ms = 0.f, lift_ms = 0.f;
         cudaEventElapsedTime(&solve_ms, g->ev[0], g->ev[3]);
         cudaEventElapsedTime(&lift_ms, g->ev[1], g->ev[3]);
+        solve_ms += spent_ms;
+        lift_ms += spent_ms;
         memset(stats, 0, sizeof *stats);
         stats->mg = g->mg;
         stats->num_top = (int64_t)c.num_top;
@@ -945,7 +956,7 @@ static eg_status dgame_solve(eg_dgame *g, const eg_opts *opts_in, eg_stats *stat
     EG_CUDA(cudaSetDevice(g->device));
     g->launches = 0;
     g->solved = false;
-    return routes_to_sweeps(opts) ? dgame_sweeps(g, opts, stats, early) : dgame_rounds(g, opts, nullptr, stats);
+    return routes_to_sweeps(opts) ? dgame_sweeps(g, opts, stats, early, 0.f) : dgame_rounds(g, opts, nullptr, stats);
 }
 
 extern "C" eg_status eg_dgame_solve(eg_dgame *g, const eg_opts *opts, eg_stats *stats)

@@ -217,8 +217,10 @@ eg_status eg_solve_i64(const eg_game *game, const eg_opts *opts, int64_t *credit
 
 typedef struct eg_dgame eg_dgame;
 
-/* Uploads a host game: allocates device memory for its CSR and all solve
- * state.  The handle keeps them resident until eg_dgame_free. */
+/* Uploads a host game: allocates device memory for its CSR and the state of
+ * solves with these options.  The first solve in rounds allocates theirs too
+ * (EG_ERR_OOM when it does not fit); a solve that only hands over to them is
+ * swept to its end without.  The handle keeps all until eg_dgame_free. */
 eg_status eg_dgame_upload(const eg_game *game, const eg_opts *opts, eg_dgame **out);
 /* Same, from a CSR that is already in device memory (pointers are device
  * pointers; owner may be NULL).  The arrays are copied, not adopted. */

@@ -233,3 +233,22 @@ def test_round_cap_after_the_hand_over():
         assert st.rounds == 7000 and st.pushes > 0
         part = r.credits()
         assert np.all(part <= ref) and np.any(part < ref) and np.any(part == 5)
+
+
+def test_hand_over_without_memory_for_it():
+    """The frontier rounds' arrays do not fit: the sweeps end the solve."""
+    torch = pytest.importorskip("torch")
+    g, ref = chains(8192, 520, 2)
+    with eg.ResidentGame(g) as r:
+        torch.cuda.empty_cache()
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - (300 << 20), dtype=torch.uint8, device="cuda")
+        try:
+            status, st = r.solve(raise_on_error=False)
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+        assert status == 0 and st.pushes == 0 and st.kernel_launches == 2
+        np.testing.assert_array_equal(r.credits(), ref)
+        _, st = r.solve()
+        assert st.pushes > 0
+        np.testing.assert_array_equal(r.credits(), ref)
