@@ -287,9 +287,10 @@ extern "C" void eg_dgame_free(eg_dgame *g)
 
 /* The sweep solver, unless the options ask for a kernel or for kinds of rounds
  * of their own: a variant, a direction or its thresholds, the pair format or
- * launch shape of those kernels, or their phase timers.  It was the faster one
- * at every size measured, 100 to 2^20 vertices (0.5 ms against 0.03 ms, 9.3 s
- * against 12 ms). */
+ * launch shape of those kernels, or their phase timers.  (Not the knobs that
+ * eg_dgame_tune sets: those shape the rounds, and the sweep solver has no use
+ * for them.)  It was the faster one at every size measured, 100 to 2^20
+ * vertices (0.5 ms against 0.03 ms, 9.3 s against 12 ms). */
 static bool routes_to_sweeps(const eg_opts *o)
 {
     return !o || (o->variant == EG_VARIANT_AUTO && o->direction == EG_DIRECTION_SWITCH && o->dense_permille == 0 &&
@@ -869,7 +870,6 @@ static eg_status dgame_sweeps(eg_dgame *g, const eg_opts *opts, eg_stats *stats,
     p.owner = g->d_owner;
     p.n = g->n;
     p.n0 = g->n0;
-    p.m = g->m;
     p.out = g->d_out;
     p.ctrl = g->d_sctrl;
     p.max_rounds = opts->max_rounds;
@@ -880,7 +880,6 @@ static eg_status dgame_sweeps(eg_dgame *g, const eg_opts *opts, eg_stats *stats,
         EG_CUDA(cudaHostGetDevicePointer(&dp, (void *)opts->cancel, 0));
         p.cancel = (const int *)dp;
     }
-    p.sweeps = opts->dense_sweeps ? opts->dense_sweeps : kMaxDenseSweeps;
     p.bits = opts->credit_bits == 32 ? 32 : 64;
     p.narrow = opts->narrow;
     if (spent_ms == 0.f && g->m >= kHandEdges) {

@@ -149,7 +149,7 @@ struct Range {
     int h_smem;
     void *g[3];              /* grid: F, D, K by number                      */
     const long long *rp;     /* the input's row offsets                      */
-    int out_bits, round;     /* primal and kill sweeps between two barriers  */
+    int out_bits;
     long long mg, scale;
 };
 
@@ -511,6 +511,9 @@ __device__ __noinline__ void solve(const SweepParams *pp, const Range &rs, Hubs 
 {
     using M = Mem<CT, KIND>;
     constexpr bool GRID = KIND != KIND_CTA;
+    /* primal and kill sweeps between two barriers (with four, more of them come
+     * after the last raise) */
+    constexpr int kRound = GRID ? 2 : 1;
     constexpr CT top = Lim<CT>::top, low = Lim<CT>::low;
     const SweepParams &p = *pp;
     /* in registers where lanes walk long slices; the code without those is
@@ -551,7 +554,7 @@ __device__ __noinline__ void solve(const SweepParams *pp, const Range &rs, Hubs 
         kd.mul = phase == SWEEP_PRIMAL ? -1 : (int)r.scale;
         kd.cap = phase == SWEEP_PRIMAL ? (CT)r.mg : Lim<CT>::dual_max;
         kd.add = phase == SWEEP_PRIMAL ? (CT)0 : (CT)1;
-        const int ran = phase == SWEEP_DUAL ? st.left : phase == SWEEP_KILL ? min(r.round, 2) : min(r.round, st.left);
+        const int ran = phase == SWEEP_DUAL ? st.left : phase == SWEEP_KILL ? kRound : min(kRound, st.left);
 #pragma unroll 1
         for (int s = 0; s < ran; s++) {
             /* The heavy vertices every second time, and in a round's last sweep,
@@ -876,8 +879,6 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
         r.g[1] = p.D;
         r.g[2] = p.K;
         r.rp = p.rp;
-        /* with four sweeps more of them come after the last raise */
-        r.round = GRID ? min(p.sweeps, 2) : 1;
     }
     int *number = GRID ? (int *)p.K : (int *)(smem + 2 * stride); /* of every vertex, where K is later */
     __syncthreads();

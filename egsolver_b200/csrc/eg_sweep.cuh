@@ -40,7 +40,6 @@ struct SweepParams {
     const int *succ, *w;
     const unsigned char *owner;          /* or null: vertex >= n0 is player 1  */
     int n, n0;
-    long long m;
     void *F, *D, *K;                     /* grid kernel: credits, potentials, their copy (plan.values of 8 B each) */
     int2 *E;                             /* where a CTA's values or edges do not fit its shared memory: */
     int *vid, *soff;                     /* sliced edges, vertices and slice offsets; else null */
@@ -49,7 +48,6 @@ struct SweepParams {
     long long max_rounds;                /* < 0: no cap                        */
     unsigned long long timeout_ns, wait_limit_ns;
     const int *cancel;
-    int sweeps;                          /* most sweeps between two barriers   */
     int bits;                            /* 32, 64: width asked for            */
     int narrow;                          /* 64: may come out in 32 bits        */
     int smem_bytes;                      /* dynamic shared memory              */

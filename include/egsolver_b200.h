@@ -139,7 +139,7 @@ typedef struct eg_opts {
     int32_t dense_depth;         /* chunks in flight per warp in dense rounds: 1 (three
                                     CTAs per SM) or 2 (two CTAs per SM); 0: 2         */
     int32_t dense_sweeps;        /* sweeps per grid barrier in dense rounds: 1 to 4
-                                    (0: 4); the sweep solver runs at most 2           */
+                                    (0: 4)                                            */
 } eg_opts;
 
 typedef struct eg_stats {
@@ -239,8 +239,10 @@ eg_status eg_dgame_credits_device(eg_dgame *g, void **dev_ptr, int32_t *credit_b
 /* Device bytes held by the handle. */
 int64_t eg_dgame_device_bytes(const eg_dgame *g);
 
-/* Autotuner of the AUTO layout (new; the reference picks its kernel from the
- * command line).  Times capped solves (`rounds` rounds each, from f = 0) of
+/* Autotuner of the rounds' AUTO layout (new; the reference picks its kernel
+ * from the command line).  Its knobs are those of the frontier and dense
+ * rounds: a solve that the sweep solver does (see eg_direction) runs the same
+ * with and without them.  Times capped solves (`rounds` rounds each, from f = 0) of
  * the resident game, one knob at a time per degree bucket and round kind:
  * the light/heavy out-degree bound (large_min_deg), the heavy vertices'
  * task size (task_edges), the thread-per-vertex bucket (small_max_deg), the

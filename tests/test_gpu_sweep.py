@@ -252,3 +252,14 @@ def test_hand_over_without_memory_for_it():
         _, st = r.solve()
         assert st.pushes > 0
         np.testing.assert_array_equal(r.credits(), ref)
+
+
+def test_knobs_of_the_rounds_leave_the_sweep_solver_alone():
+    """dense_sweeps is a knob of the dense rounds, and one the tuner sets: the
+    sweep solver runs two sweeps between its barriers whatever it says."""
+    g = eg.generate(4, 9000, 16, 100, 21, param=2)
+    f, st = eg.solve(g)
+    for k in (1, 2, 4):
+        f1, st1 = eg.solve(g, dense_sweeps=k)
+        np.testing.assert_array_equal(f1, f)
+        assert st1.grid == st.grid > 1 and st1.rounds < st1.dense_rounds
