@@ -28,7 +28,9 @@
  * whose credits do not fit one CTA's shared memory while the queue is
  * shallow, are solved by a second thread one threshold at a time on the
  * persistent grid solver, capped at `large_ctas` CTAs so that micro-batches
- * keep SMs to run on.  With a deep queue such games run as units with their
+ * keep SMs to run on: a CTA of it fills an SM, so by default it gets three
+ * quarters of them (on all, a query of 2,000 vertices waited 50 s for the end
+ * of a path of 600,000).  With a deep queue such games run as units with their
  * credits in global memory, for throughput.
  *
  * Every result equals the solve of the same game and threshold alone: a
@@ -726,10 +728,10 @@ extern "C" eg_status eg_serve_create(const eg_serve_opts *opts, eg_server **out)
     if (s->o.streams <= 0) s->o.streams = 4;
     if (s->o.block <= 0) s->o.block = 1024;
     if (s->o.hbm_reserve_bytes <= 0) s->o.hbm_reserve_bytes = 1ll << 30;
-    if (s->o.large_ctas <= 0) s->o.large_ctas = 148;
     if (s->o.max_rounds == 0) s->o.max_rounds = -1;
     cudaSetDevice(s->o.device);
     cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->o.device);
+    if (s->o.large_ctas <= 0) s->o.large_ctas = std::max(1, s->sms - s->sms / 4);
     {
         eg_status ks = unit_kernel_setup(s->o.device);
         if (ks != EG_OK) {

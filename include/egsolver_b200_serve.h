@@ -35,7 +35,8 @@ typedef struct eg_serve_opts {
     int32_t block;               /* threads per CTA of the batched kernel (0 = 1024) */
     int64_t hbm_reserve_bytes;   /* device memory admission leaves free (0 = 1 GiB)  */
     int64_t max_rounds;          /* per query; < 0: no cap                           */
-    int32_t large_ctas;          /* CTAs of the grid solver for large games (0: 148)  */
+    int32_t large_ctas;          /* CTAs, each on an SM of its own, of the grid solver
+                                    for large games (0: three quarters of the SMs)    */
     int32_t reserved[5];
 } eg_serve_opts;
 

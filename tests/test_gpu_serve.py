@@ -2,6 +2,8 @@
 admission by free device memory, the large-game path, statistics."""
 from __future__ import annotations
 
+import time
+
 import numpy as np
 import pytest
 
@@ -233,3 +235,24 @@ def test_evicted_games_make_room():
                 assert np.all(s.result(q)[0] == eg.EG_TOP64)
         st = s.stats()
         assert st["failed"] == 0 and 4 <= st["evictions"] <= 7
+
+
+def test_small_queries_run_beside_the_grid_solver():
+    """A path of 600,000 vertices keeps the grid solver busy for about a
+    second; a query of a small game that comes meanwhile does not wait for it."""
+    n = 600_000
+    weight = np.full(n, -1)
+    weight[-1] = 0
+    deep = eg.Game(row_ptr=np.arange(n + 1), succ=np.minimum(np.arange(1, n + 1), n - 1), weight=weight, num_nodes0=n // 2)
+    small = eg.generate(4, 2000, 16, 100, 3, param=2)
+    with eg.Server() as s:
+        a, b = s.add_game(deep), s.add_game(small)
+        s.wait(s.submit(b, [0, 10]))
+        q = s.submit(a, [0])
+        time.sleep(0.1)
+        q2 = s.submit(b, [0, 10])
+        s.wait(q2)
+        time.sleep(0.1)  # past the end of a solve that the small query waited for
+        assert s.poll(q)[0] == 1  # still running
+        s.wait(q)
+        np.testing.assert_array_equal(s.result(q)[0][0], np.arange(n)[::-1])
