@@ -955,6 +955,9 @@ static eg_status dgame_solve(eg_dgame *g, const eg_opts *opts_in, eg_stats *stat
     EG_CUDA(cudaSetDevice(g->device));
     g->launches = 0;
     g->solved = false;
+    /* keep_layout is about the previous solve, and the sweep solver leaves no
+     * layout: one from before it may be another variant's */
+    if (!opts->keep_layout) g->prepared = false;
     return routes_to_sweeps(opts) ? dgame_sweeps(g, opts, stats, early, 0.f) : dgame_rounds(g, opts, nullptr, stats);
 }
 

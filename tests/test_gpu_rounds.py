@@ -110,3 +110,18 @@ def test_keep_layout(cfg2_2e14, d):
         r.solve()  # the sweep solver in between
         r.solve(keep_layout=True, **d)
         np.testing.assert_array_equal(r.credits(), ref)
+
+
+# large enough for the grid's kernels, whose dense rounds need the AUTO layout
+@pytest.mark.parametrize("variant", [eg.VARIANT_WARP, eg.VARIANT_CTA])
+def test_keep_layout_is_about_the_previous_solve(variant):
+    game = eg.generate(4, 16000, 16, 20, 7, param=2)
+    ref = O.eg_solve(game, bits=64)[0]
+    assert game.num_edges > 1 << 17
+    with eg.ResidentGame(game) as r:
+        r.solve(variant=variant)
+        np.testing.assert_array_equal(r.credits(), ref)
+        r.solve()
+        _, st = r.solve(keep_layout=True, **DENSE)
+        np.testing.assert_array_equal(r.credits(), ref)
+        assert st.dense_rounds > 0 and st.kernel_launches > 1
