@@ -726,7 +726,10 @@ def main():
     S = credit_bits // 8
     traffic = None
     if last.dense_rounds > 0 and last.dense_ms > 0 and last.large_min_deg == 0:
-        # the sweep kernel: it has no degree buckets
+        # the sweep kernel: it has no degree buckets, and counts in 32 bits where
+        # MG + max |weight| < 2^30 and the weights are at most 2^20
+        wmax = int(np.abs(game.weight.astype(np.int64)).max())
+        S = 4 if last.mg + wmax < 1 << 30 and wmax <= 1 << 20 else 8
         launches_k = sum(s.dense_launches for s in stats)
         d_bytes = sum(s.edges * (8 + S) + s.lifts * (8 + S) + s.changes * S for s in stats)
         d_ms = sum(s.dense_ms for s in stats)

@@ -44,17 +44,17 @@ namespace {
 
 constexpr unsigned long long kWaitLimitNs = 5ull * 1000ull * 1000ull * 1000ull; /* 5 s per barrier wait */
 constexpr int kPrepBlock = 256;
-/* AUTO lifts a game with one CTA (frontier in shared memory) up to this
- * many edges; larger games use the persistent grid. */
+/* Rounds in the AUTO layout lift a game with one CTA (frontier in shared
+ * memory) up to this many edges, larger ones on the persistent grid. */
 constexpr long long kSmallGameEdges = 1 << 17;
 /* default round-kind thresholds, raises per thousand vertices */
 constexpr long long kDensePermille = 40;
 constexpr long long kSparsePermille = 15;
 constexpr int kSmallGameMaxPad = 1 << 19;
 /* a sweep solve of a game of at least kHandEdges edges hands over to
- * frontier rounds when, after kHandSweeps sweeps, fewer than kSparsePermille
- * of the vertices rise in a round: a sweep of 2^22 edges takes longer than
- * a frontier round */
+ * frontier rounds when, at the end of a primal phase with kHandSweeps sweeps
+ * or more behind it, fewer than kSparsePermille of the vertices rise in a
+ * round: a sweep of 2^22 edges takes longer than a frontier round */
 constexpr long long kHandEdges = 1 << 22;
 constexpr long long kHandSweeps = 2048;
 constexpr size_t kEarlyAt = 2048; /* credits behind the control block in a lane's pinned memory */

@@ -151,8 +151,8 @@ struct Ctrl {
  * EG_ERR_TIMEOUT and raises abort so the other CTAs stop waiting too.  The
  * last arriver runs `last()` (single thread) before releasing the grid.
  * Returns false when the solve must stop (abort raised). */
-template <class C, class F>
-__device__ __forceinline__ bool grid_barrier(C *c, unsigned long long wait_limit_ns, F last)
+template <class F>
+__device__ __forceinline__ bool grid_barrier(Ctrl *c, unsigned long long wait_limit_ns, F last)
 {
     __shared__ int s_ok;
     __syncthreads();

@@ -59,8 +59,9 @@ void launch_task_reset(int bits, int heavy_begin, int n_pad, const int *toff, Cl
                        cudaStream_t st);
 /* credits: 0 everywhere except TOP at the sentinel topv */
 void launch_init_credits(int bits, int n_alloc, void *F, int topv, cudaStream_t st);
-/* number of TOP credits among the first n_pad, added to *out */
+/* credits in original vertex order back into the renumbered array */
 void launch_resume_credits(int bits, int n, const int *iperm, const void *credits, void *F, cudaStream_t st);
+/* number of TOP credits among the first n_pad, added to *out */
 void launch_count_top(int bits, int n_pad, const void *F, unsigned long long *out, cudaStream_t st);
 /* out[v] = F[iperm[v]] converted between widths, TOP kept as TOP */
 void launch_gather_out(int in_bits, int out_bits, int n, const int *iperm, const void *F, void *out, cudaStream_t st);

@@ -131,9 +131,12 @@ typedef struct eg_opts {
                                     vertices is dense (0: 40)                         */
     int32_t sparse_permille;     /* a dense round with fewer raises per thousand
                                     vertices is followed by sparse ones (0: 15)       */
-    int32_t narrow;              /* non-zero: a 64-bit solve computes in 32 bits when
-                                    MG + max |weight| < 2^31 - 1 (identical credits;
-                                    eg_dgame_credits_device then reports 32)          */
+    int32_t narrow;              /* non-zero: a 64-bit solve keeps its credits in 32
+                                    bits when MG + max |weight| < 2^31 - 1 (identical
+                                    credits; eg_dgame_credits_device then reports 32;
+                                    inside, the sweep solver counts in 32 bits anyway
+                                    where MG + max |weight| < 2^30 and the weights
+                                    are at most 2^20)                                 */
     int32_t wide_pairs;          /* non-zero: dense rounds read 16-byte edge pairs
                                     even when successor and weight fit 32 bits        */
     int32_t dense_depth;         /* chunks in flight per warp in dense rounds: 1 (three
@@ -345,7 +348,9 @@ eg_status eg_batch_solve(eg_batch *b, eg_batch_stats *stats);
 /* Credits of one game, threshold-major: credits[k * n_g + v] (TOP = EG_TOP64). */
 eg_status eg_batch_credits(eg_batch *b, int32_t game, int64_t *credits);
 /* Per-game outcome of the last solve: sweeps (the most of its units) and an
- * eg_status. */
+ * eg_status.  The credits of a game that max_rounds or timeout_ms stopped are
+ * lower bounds.  They need not grow with the limit: a unit that tried for
+ * certificates starts its credits again from 0. */
 eg_status eg_batch_game_result(eg_batch *b, int32_t game, int64_t *rounds, int32_t *status);
 /* Autotuner: times the candidate CTA sizes on the whole batch under a
  * sweep cap and keeps the fastest for later solves (*block receives the CTA
