@@ -554,7 +554,7 @@ __device__ __noinline__ void solve(const SweepParams *pp, const Range &rs, Hubs 
         kd.mul = phase == SWEEP_PRIMAL ? -1 : (int)r.scale;
         kd.cap = phase == SWEEP_PRIMAL ? (CT)r.mg : Lim<CT>::dual_max;
         kd.add = phase == SWEEP_PRIMAL ? (CT)0 : (CT)1;
-        const int ran = phase == SWEEP_DUAL ? st.left : phase == SWEEP_KILL ? kRound : min(kRound, st.left);
+        const int ran = phase == SWEEP_DUAL ? st.left : phase == SWEEP_KILL || !GRID ? kRound : min(kRound, st.left);
 #pragma unroll 1
         for (int s = 0; s < ran; s++) {
             /* The heavy vertices every second time, and in a round's last sweep,

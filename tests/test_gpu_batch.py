@@ -8,6 +8,7 @@ import pytest
 import egsolver_b200 as eg
 from egsolver_b200 import workloads
 from oracle import oracle as O
+from tests.test_gpu_sweep import strip, want
 
 pytestmark = pytest.mark.gpu
 
@@ -293,3 +294,15 @@ def test_a_group_in_which_some_thresholds_are_dropped(group_max):
         b.set_thresholds(p)
         b.solve()
         np.testing.assert_array_equal(b.credits(0), np.array(want))
+
+
+@pytest.mark.parametrize("levels,back", [(400, 0.01), (400, 0.3), (1500, 0.05)])
+def test_deep_games_with_unbounded_parts(levels, back):
+    """Groups whose thresholds are certified after different attempts, or dropped."""
+    g, p = strip(levels, 4, back, levels), [0, 1, -1, 2, -2, 3, -8, 8]
+    with eg.Batch([g], thresholds=8) as b:
+        b.set_thresholds(p)
+        b.solve()
+        got = b.credits(0)
+    for k, x in enumerate(p):
+        np.testing.assert_array_equal(got[k], want(eg.threshold_game(g, x, 1)))

@@ -263,3 +263,34 @@ def test_knobs_of_the_rounds_leave_the_sweep_solver_alone():
         f1, st1 = eg.solve(g, dense_sweeps=k)
         np.testing.assert_array_equal(f1, f)
         assert st1.grid == st.grid > 1 and st1.rounds < st1.dense_rounds
+
+
+def strip(levels, width, back, seed):
+    """Levels of `width` vertices, two edges of cost 1 to 3 from each to the
+    next level, the last level at rest; a share `back` of the vertices has a
+    third edge to some earlier level, which gains or costs a little."""
+    rng = np.random.default_rng(seed)
+    n = levels * width
+    rows = []
+    for v in range(n):
+        lv = v // width
+        if lv == levels - 1:
+            rows.append([(v, 0)])
+            continue
+        e = [((lv + 1) * width + int(rng.integers(width)), -int(rng.integers(1, 4))) for _ in range(2)]
+        if rng.random() < back:
+            e.append((int(rng.integers(v + 1)), int(rng.integers(-3, 40))))
+        rows.append(e)
+    return eg.Game(row_ptr=np.concatenate([[0], np.cumsum([len(e) for e in rows])]),
+                   succ=np.array([s for e in rows for s, _ in e]), weight=np.array([w for e in rows for _, w in e]),
+                   owner=rng.integers(0, 2, n).astype(np.uint8))
+
+
+# one CTA and the grid; attempts that are dropped, then some that certify
+@pytest.mark.parametrize("levels,width", [(500, 4), (2000, 4)])
+@pytest.mark.parametrize("back", [0.01, 0.05, 0.3])
+def test_deep_games_with_unbounded_parts(levels, width, back):
+    g = strip(levels, width, back, levels)
+    f, st = eg.solve(g)
+    assert (st.grid > 1) == (levels > 500)
+    np.testing.assert_array_equal(f, want(g))
