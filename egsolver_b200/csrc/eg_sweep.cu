@@ -440,20 +440,21 @@ __device__ __forceinline__ bool advance(const SweepParams &p, SweepState &c, int
         return false;
     }
     c.stop = stop;
+    /* rounds of a kill phase: `left` counts them down (`rounds` stands still) */
+    const int most = (int)max((long long)kKillRounds, min(c.rounds, 1ll << 28));
     if (c.phase == SWEEP_DUAL) {
         c.dual_len = min(2 * c.dual_len, kMaxDual);
         c.phase = SWEEP_KILL;
-        c.kills = 0;
+        c.left = most;
         return false;
     }
+    if (raised != 0ull && --c.left > 0) return false;
     const bool certified = raised == 0ull;
-    c.kills = min(c.kills + 1, 1 << 28);
-    if (certified || (c.kills >= kKillRounds && c.kills >= c.rounds)) {
-        c.phase = SWEEP_PRIMAL;
-        c.left = c.primal_len;
-        if (c.kills >= kKillRounds) c.left = max(c.left, (certified ? 2 : 4) * c.kills);
-        c.primal_len = min(2 * c.primal_len, kMaxPrimal);
-    }
+    const int kills = most - c.left;
+    c.phase = SWEEP_PRIMAL;
+    c.left = c.primal_len;
+    if (kills >= kKillRounds) c.left = max(c.left, (certified ? 2 : 4) * kills);
+    c.primal_len = min(2 * c.primal_len, kMaxPrimal);
     return certified;
 }
 
@@ -1035,7 +1036,6 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
     st.primal_len = kSecondPrimal;
     st.dual_len = kFirstDual;
     st.stop = out_bits == 32 && mg > (unsigned long long)INT32_MAX ? (int)EG_ERR_OVERFLOW : 0;
-    st.kills = 0;
     st.rounds = st.sweeps = 0;
     __syncthreads();
     if (tid < 4) s_sum[tid] = 0ull;

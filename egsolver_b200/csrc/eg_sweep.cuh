@@ -16,9 +16,8 @@ enum { SWEEP_PRIMAL = 0, SWEEP_DUAL = 1, SWEEP_KILL = 2, SWEEP_DONE = 3, SWEEP_H
  * after every round. */
 struct SweepState {
     int phase;
-    int left;                            /* sweeps left in this phase          */
+    int left;                            /* sweeps, or rounds of a kill phase, left in this one */
     int primal_len, dual_len;            /* sweeps of the next phases          */
-    int kills;                           /* rounds of this kill phase          */
     int stop;                            /* 0 running; else an eg_status       */
     long long rounds;                    /* primal rounds completed            */
     long long sweeps;                    /* primal sweeps run                  */
