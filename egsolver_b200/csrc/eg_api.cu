@@ -910,6 +910,7 @@ static eg_status dgame_sweeps(eg_dgame *g, const eg_opts *opts, eg_stats *stats,
     g->mg = (long long)c.mg;
     g->wmax = (long long)c.wmax;
     const int stop = c.abort ? (int)EG_ERR_TIMEOUT : c.s.stop;
+    if (stop == EG_ERR_INVALID) return eg_set_error(EG_ERR_INVALID, "a vertex has no successor");
     if (stop == EG_ERR_OVERFLOW)
         return eg_set_error(EG_ERR_OVERFLOW, "MG = %lld does not fit 32-bit credits", g->mg);
     if (c.s.phase == SWEEP_HANDOVER && !stop) {

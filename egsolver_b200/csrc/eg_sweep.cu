@@ -680,6 +680,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
     __shared__ int s_cls[5];                /* first slot past the light vertices of player 0; of player 1; columns; light; lg */
     __shared__ int s_heavy[4];              /* heavy vertices: not cut, cut; their edges; next offset */
     __shared__ int s_scan[kWarps];
+    __shared__ int s_sink;                  /* a vertex has no successor: the walks count on one */
     SweepCtrl *c = p.ctrl;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     /* with an owner array the players' vertices are not apart: one part */
@@ -703,6 +704,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
     }
     if (tid == 0) {
         if (blockIdx.x == 0) c->t_start = globaltimer_ns();
+        s_sink = 0;
         hb.tasks = 0;
         hb.seg = seg;
         turn.raised[0] = turn.raised[1] = 0u;
@@ -715,9 +717,10 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
     for (int i = tid; i < nv; i += kBlock) {
         const int v = i < nv0 ? cut[0] + i : gap + i;
         const int deg = (int)(p.rp[v + 1] - p.rp[v]);
+        if (deg <= 0) s_sink = 1;
         if (deg <= kLightDeg) {
             const int own1 = p.owner ? p.owner[v] != 0 : v >= p.n0;
-            atomicAdd(&s_bin[own1 * (kLightDeg + 1) + deg], 1);
+            atomicAdd(&s_bin[own1 * (kLightDeg + 1) + max(deg, 0)], 1);
         } else {
             atomicAdd(&s_heavy[deg > cut_from], 1);
             atomicAdd(&s_heavy[2], deg);
@@ -890,7 +893,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
         const int own1 = p.owner ? p.owner[v] != 0 : v >= p.n0;
         int slot;
         if (deg <= light) {
-            slot = atomicAdd(&s_bin[own1 * (kLightDeg + 1) + deg], 1);
+            slot = atomicAdd(&s_bin[own1 * (kLightDeg + 1) + max(deg, 0)], 1);
         } else {
             const int hub = deg > cut_from;
             const int h = (hub ? nmed : 0) + atomicAdd(&s_heavy[hub], 1);
@@ -1019,7 +1022,8 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
         if (tid == 0 && turn.ok) {
             atomicAdd(&c->mg, s_sum[0]);
             atomicMax(&c->wmax, s_sum[1]);
-            turn.ok = round_barrier(p, c, it, 0ull, &got);
+            turn.ok = round_barrier(p, c, it, (unsigned long long)s_sink, &got);
+            s_sink = got != 0ull;
             s_sum[0] = __ldcg(&c->mg);
             s_sum[1] = __ldcg(&c->wmax);
         }
@@ -1035,7 +1039,9 @@ __global__ void __launch_bounds__(kBlock, 1) k_sweep(const __grid_constant__ Swe
     st.left = kFirstPrimal;
     st.primal_len = kSecondPrimal;
     st.dual_len = kFirstDual;
-    st.stop = out_bits == 32 && mg > (unsigned long long)INT32_MAX ? (int)EG_ERR_OVERFLOW : 0;
+    st.stop = s_sink                                                  ? (int)EG_ERR_INVALID
+              : out_bits == 32 && mg > (unsigned long long)INT32_MAX ? (int)EG_ERR_OVERFLOW
+                                                                      : 0;
     st.rounds = st.sweeps = 0;
     __syncthreads();
     if (tid < 4) s_sum[tid] = 0ull;

@@ -226,7 +226,9 @@ typedef struct eg_dgame eg_dgame;
  * swept to its end without.  The handle keeps all until eg_dgame_free. */
 eg_status eg_dgame_upload(const eg_game *game, const eg_opts *opts, eg_dgame **out);
 /* Same, from a CSR that is already in device memory (pointers are device
- * pointers; owner may be NULL).  The arrays are copied, not adopted. */
+ * pointers; owner may be NULL).  The arrays are copied, not adopted, and not
+ * checked as eg_validate does; the sweep solver refuses a vertex without a
+ * successor (EG_ERR_INVALID). */
 eg_status eg_dgame_from_device(const eg_game *dev_game, const eg_opts *opts, eg_dgame **out);
 /* Solves a resident game from f = 0: transpose, bucket, init, lift.  The
  * credits stay on the device; stats are filled. */

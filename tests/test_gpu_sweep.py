@@ -294,3 +294,25 @@ def test_deep_games_with_unbounded_parts(levels, width, back):
     f, st = eg.solve(g)
     assert (st.grid > 1) == (levels > 500)
     np.testing.assert_array_equal(f, want(g))
+
+
+# one CTA and the grid; the last of a slice, of a player, of the game
+@pytest.mark.parametrize("n,sink", [(100, 0), (100, 63), (3000, 2999), (6000, 31), (20000, 9999), (20000, 19999)])
+def test_device_games_with_a_sink_are_refused(n, sink):
+    """A game that is on the device already has not been through the host's checks."""
+    torch = pytest.importorskip("torch")
+    g = eg.generate(1, n, 4, 9, n + sink)
+    deg = np.full(n, 4)
+    for counts in (np.where(np.arange(n) == sink, 0, deg), deg):
+        rp = np.concatenate([[0], np.cumsum(counts)])
+        dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (rp, g.succ, g.weight)]
+        torch.cuda.synchronize()
+        r = eg.ResidentGame.from_device(n, int(rp[-1]), g.num_nodes0, *(x.data_ptr() for x in dev))
+        if counts is deg:
+            r.solve()
+            np.testing.assert_array_equal(r.credits(), want(g))
+        else:
+            with pytest.raises(eg.EGError) as ei:
+                r.solve()
+            assert ei.value.name == "EG_ERR_INVALID"
+        r.free()
