@@ -262,6 +262,7 @@ def test_time_limit_of_a_deep_game():
     n = 50_000
     with eg.Batch([chain(n)], thresholds=1, timeout_ms=20, park_percent=1000) as b:
         b.set_thresholds([0])
+        b.solve(raise_on_error=False)  # loads the kernel
         status, st = b.solve(raise_on_error=False)
         assert st.games_failed == 1 and st.solve_ms < 60
         assert eg._ffi.STATUS_NAMES[b.game_result(0)[1]] == "EG_ERR_TIMEOUT"
