@@ -358,13 +358,13 @@ bool admit(eg_server *s, std::unique_lock<std::mutex> &lk)
 {
     bool any = false;
     size_t left = 0;
-    /* The rest of a burst is submitted meanwhile, so a few more are taken
-     * than are there, but not so many that the first wait for all.  Medians of
-     * two runs on one box, bursts of 2 / 4 / 12 / 25 / 50 queries of 6 thresholds on
-     * games of 1000-8000 nodes: 0.31 / 0.47 / 1.0 / 1.8 / 3.1-3.8 ms with 6;
-     * 0.31 / 0.5-1.6 / 1.2-2.0 / 1.9-2.6 / 3.3-4.6 with none; 0.3-0.4 /
-     * 0.5-0.7 / 1.2-1.8 / 1.7 / 3.4-4.2 with 16.  (On another box bursts of 12
-     * took 2.3.) */
+    /* The rest of a burst is submitted meanwhile, so a few more are taken than
+     * are there, but not so many that the first wait for all.  Medians of two
+     * runs, bursts of 2 / 4 / 12 / 25 / 50 queries of 6 thresholds on games of
+     * 1000-8000 nodes: 0.31 / 0.47 / 1.0 / 1.8 / 3.1-3.8 ms with 6; 0.31 /
+     * 0.5-1.6 / 1.2-2.0 / 1.9-2.6 / 3.3-4.6 with those that are there; 0.3-0.4
+     * / 0.5-0.7 / 1.2-1.8 / 1.7 / 3.4-4.2 with 16.  (Bursts of 12 took up to
+     * 2.5 on other machines.) */
     size_t taken = 0;
     const size_t most = std::max<size_t>(s->pending.size(), 6);
     for (; !s->pending.empty() && taken < most && s->admitted_now < s->o.max_inflight; taken++) {

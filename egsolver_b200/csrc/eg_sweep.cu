@@ -416,8 +416,8 @@ __device__ __forceinline__ void sweep(const Range &r, const Kind<CT> &kd, Hubs &
  * A kill phase may be as long as the game is deep, and on a path certifies
  * nothing: it is dropped once it has cost as much as the credits so far, and
  * what follows an attempt is at least as long as it was, so that kills stay
- * within about one and a half times the primal rounds (path of 16,384 vertices,
- * kills to their end: 241 ms, of which 24 primal). */
+ * within about one and a half times the primal rounds (path of 16,384 vertices
+ * 52 ms; kills to their end 239 ms, ten times the primal sweeps). */
 __device__ __forceinline__ bool advance(const SweepParams &p, SweepState &c, int ran, unsigned long long raised, int stop)
 {
     if (c.phase == SWEEP_PRIMAL) {
@@ -526,6 +526,7 @@ __device__ __noinline__ void solve(const SweepParams *pp, const Range &rs, Hubs 
     const int tid = threadIdx.x, lane = tid & 31;
     const int nslots = r.light_slots + r.nh;
     const bool watch = p.timeout_ns || p.cancel;
+    const bool watcher = watch && tid == 0 && blockIdx.x == 0;
     bool ok = turn.ok != 0, mark = false;
     /* slots without a vertex are never lifted (the others start at 0) */
     for (int i = tid; i < r.light_slots; i += kBlock) {
@@ -580,7 +581,7 @@ __device__ __noinline__ void solve(const SweepParams *pp, const Range &rs, Hubs 
         /* the round's raises and the next step of the schedule */
         unsigned long long raised;
         int stop = 0;
-        if (tid == 0 && watch && blockIdx.x == 0) {
+        if (watcher) {
             if (p.timeout_ns && globaltimer_ns() - p.ctrl->t_start > p.timeout_ns) stop = (int)EG_ERR_TIMEOUT;
             else if (p.cancel && ((it - first) & 63) == 0 && ld_volatile(p.cancel)) stop = (int)EG_ERR_CANCELLED;
         }
