@@ -459,8 +459,17 @@ bool admit(eg_server *s, std::unique_lock<std::mutex> &lk)
         lk.unlock();
         const cudaError_t ae = pool_alloc((void **)&blk, total, s->o.device, s->upload_stream);
         if (ae != cudaSuccess) {
+            /* less than there seemed to be (what the pool holds may lie in
+             * pieces): without another game, later, or not at all */
             lk.lock();
-            break;
+            left = 0;
+            if (evict_one(s)) continue;
+            if (s->admitted_now > 0 || !s->inflight.empty()) break;
+            s->pending.pop_front();
+            finish_query(s, q, EG_ERR_OOM, clk::now());
+            s->cv_done.notify_all();
+            any = true;
+            continue;
         }
         q.dF = (long long *)blk;
         q.dthr = (int *)(blk + o_thr);
